@@ -139,7 +139,7 @@ __device__ __forceinline__ Foot footprint(uint32_t xr, uint32_t yr, const Worksp
 }
 
 // point_in_tri of a record at pixel (px, py).
-__device__ __forceinline__ bool rec_in_tri(const float4 q[4], int px, int py) {
+__device__ __forceinline__ bool rec_in_tri(const float4 q[3], int px, int py) {
   float fx = (float)px, fy = (float)py;
   float sgn = q[1].w;
   float s = ((q[1].x + q[1].y * fx) + q[1].z * fy) * sgn;
@@ -147,24 +147,20 @@ __device__ __forceinline__ bool rec_in_tri(const float4 q[4], int px, int py) {
   return s > -0.0001f && t > -0.0001f && (s + t) < q[0].w;
 }
 
-// Is the left-column pixel (minx, py) of a record's bbox skipped by the
-// reference walk (py > miny)?
-__device__ __forceinline__ bool walk_skips(uint32_t xr, uint32_t yr, int py, int chunk) {
-  const int minx = xr & 0xFFFF, miny = yr & 0xFFFF;
-  return py > miny && !walk_visits(0, py - miny, (int)(xr >> 16) - minx, (int)(yr >> 16) - miny, (float)miny, chunk);
-}
-
-// walk_skips for the rows [y0, y1) of a record's bbox at once: bit py - ty
-// set where the left-column pixel is skipped.  The same arithmetic as
+// The rows py of [y0, y1) of a record's bbox whose left-column pixel the
+// reference walk skips, as bits py - ty.  The same arithmetic as
 // walk_visits (walk_row_late's 1 / w computed once, (r + 1) * w % chunk
-// stepped row by row).
+// stepped row by row), from the first row that can be late at all
+// (walk_first_late_row): a bbox at least its own height below the top of the
+// surface, which is nearly every record, costs one comparison instead of a
+// division, two modulos and a loop over its rows.
 __device__ __forceinline__ uint32_t walk_skip_rows(uint32_t xr, uint32_t yr, int y0, int y1, int ty, int chunk) {
   const int minx = xr & 0xFFFF, miny = yr & 0xFFFF;
+  const int first = max(y0 - miny, walk_first_late_row(miny));
+  const int last = y1 - miny;  // one past
+  if (first >= last) return 0u;
   const int w = (int)(xr >> 16) - minx, h = (int)(yr >> 16) - miny;
   const float iw = fdiv(1.0f, (float)w), fminy = (float)miny;
-  const int first = max(y0, miny + 1) - miny;  // r of the first row with r > 0
-  const int last = y1 - miny;                  // one past
-  if (first >= last) return 0u;
   auto late = [&](int r) { return floorf(fma_((float)(r * w), iw, fminy)) != fminy + (float)r; };
   const int wm = w % chunk;
   int m = ((first + 1) * w) % chunk;  // (r + 1) * w % chunk
@@ -181,14 +177,6 @@ __device__ __forceinline__ uint32_t walk_skip_rows(uint32_t xr, uint32_t yr, int
     if (m >= chunk) m -= chunk;
   }
   return bits;
-}
-
-// Coverage of a pixel known to lie inside the record's bbox: the reference
-// walk's skipped left-column pixels, then point_in_tri.
-__device__ __forceinline__ bool covers_in_bbox(const float4 q[4], int px, int py, int chunk) {
-  const uint32_t xr = __float_as_uint(q[3].x), yr = __float_as_uint(q[3].y);
-  if (px == (int)(xr & 0xFFFF) && walk_skips(xr, yr, py, chunk)) return false;
-  return rec_in_tri(q, px, py);
 }
 
 // One candidate as a record (and shade record for views); returns its tile footprint.
@@ -227,26 +215,13 @@ __device__ __noinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, 
                        make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), 0.0f, 0.0f)};
   const int x0 = (int)(R.xr & 0xFFFF), x1 = (int)(R.xr >> 16), y0 = (int)(R.yr & 0xFFFF), y1 = (int)(R.yr >> 16);
   uint32_t hits = 0;
-  // covers_in_bbox row by row: the walk rule of each row's left-column pixel
-  // (walk_visits) with 1 / w and (r + 1) * w % chunk computed incrementally
-  const int w = x1 - x0, h = y1 - y0, chunk = S.chunk;
-  const float iw = fdiv(1.0f, (float)w), fminy = (float)y0;
-  auto late = [&](int r) { return floorf(fma_((float)(r * w), iw, fminy)) != fminy + (float)r; };
-  const int wm = w % chunk;
-  int m = (2 * w) % chunk;  // (r + 1) * w % chunk for row r = 1
-  bool late_r = h > 1 ? late(1) : false;
+  // row by row: the walk rule of the row's left-column pixel, then point_in_tri
+  // (walk_skip_rows: 0 at once unless the bbox touches the top of the face;
+  // a bbox of at most 64 pixels has at most 64 rows)
+  const uint64_t skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, S.chunk) |
+                        ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, S.chunk) << 32);
   for (int y = y0; y < y1; y++) {
-    const int r = y - y0;
-    bool skip_left = false;
-    if (r > 0) {
-      const int r1 = r + 1;
-      const bool late_r1 = r1 < h ? late(r1) : false;
-      skip_left = late_r && !(r1 < h && m == 0 && late_r1);
-      late_r = late_r1;
-      m += wm;
-      if (m >= chunk) m -= chunk;
-    }
-    for (int x = skip_left ? x0 + 1 : x0; x < x1; x++)
+    for (int x = x0 + (int)((skip >> (y - y0)) & 1u); x < x1; x++)
       if (rec_in_tri(q, x, y)) {
         atomicMin(S.depth + (size_t)y * S.width + x, depth_at(R.A, R.B, R.C, (float)x, (float)y));
         hits++;
@@ -831,14 +806,25 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // alike.  Pass 0 resolves the minimum depth with shared-memory atomicMin;
 // pass 1 the minimum packed (key << 32 | record) among tests within +-20 of
 // the final depth.  Both are minima, so neither bin order nor thread order
-// changes the result.  When the whole list fits one chunk and each lane has
-// at most kRasterCache covered pixels, pass 1 reuses the covered pixels of
-// pass 0 kept in shared memory.
-constexpr int kRasterCache = 8;
-// Cache slots of an NT-thread view raster: 512-thread CTAs keep none (their
-// static shared memory stays under 48 KB) and re-test in the id pass.
+// changes the result.  Pass 0 keeps its covered pixels in a list per warp
+// (kHitCap, compacted in place when it fills: an entry 20 or more behind the
+// pixel's depth so far never passes), and pass 1 runs over those lists; only a
+// tile whose lists overflow all the same tests its records again.
+//
+// Measured (launch alone, before -> now; bound by instruction issue, 72 %
+// active, and by the barriers between chunks): 1080p terrain 114 -> 81 us, 9
+// ragged views of a 500k-triangle scene 689 -> 431 us (tiles of several chunks
+// no longer stage and test everything twice; the walk rule costs a comparison
+// per record), 2560x1440 under 1,000 screen-covering triangles 22.4 -> 0.43 ms
+// (the depth cull at staging).
+constexpr int kHitCap = 256;  // entries of a warp's list: about 100 are used in a tile of 1.2 layers
+// 512-thread CTAs keep no lists (their static shared memory stays under 48 KB)
+// and re-test in the id pass.
 template <int NT>
-__host__ __device__ constexpr int raster_cache_slots() { return NT <= 256 ? kRasterCache : 0; }
+__host__ __device__ constexpr int raster_hits() { return NT <= 256 ? kHitCap * (NT / 32) : 0; }
+// A list entry's second word: pixel | record << 8, so records below 2^24
+// (passes with room for more re-test tiles of several chunks).
+constexpr uint32_t kHitRecords = 1u << 24;
 constexpr uint32_t kSlotBits = 9;  // staged slots of a one-chunk tile: below 512
 
 // Exclusive block scan with a single barrier: each warp scans its lanes,
@@ -885,23 +871,49 @@ __device__ __forceinline__ uint32_t pack_rgba(float r, float g, float b, float a
   return quant8(r) | (quant8(g) << 8) | (quant8(b) << 16) | (quant8(a) << 24);
 }
 
+// Drops the entries of a warp's list that are 20 or more behind their pixel's
+// depth so far (the final depth is at most that, and kernel2's window ends 20
+// behind it).  Every lane of the warp calls it; returns the new length.
+__device__ __noinline__ uint32_t compact_hits(uint2* hits, uint32_t n, const uint32_t* sdepth) {
+  const int lane = threadIdx.x & 31;
+  uint32_t kept = 0;
+  for (uint32_t g0 = 0; g0 < n; g0 += 32) {
+    const uint32_t g = g0 + lane;
+    uint2 e = make_uint2(0, 0);
+    bool keep = false;
+    if (g < n) {
+      e = hits[g];
+      const uint32_t fd = sdepth[swz32((int)(e.y & 0xFF))];
+      keep = fd > kDepthClear - kBufError || e.x < fd + kBufError;
+    }
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, keep);  // (every lane has read its entry)
+    if (keep) hits[kept + (uint32_t)__popc(b & ((1u << lane) - 1u))] = e;
+    kept += (uint32_t)__popc(b);
+    __syncwarp();
+  }
+  return kept;
+}
+
 // Shared memory of one tile's raster (NT threads; ID: views).
 template <int NT, bool ID>
 struct RasterSmem {
-  float4 srec[4][NT];  // the staged records' four float4, one array each (conflict-free stores)
+  float4 srec[3][NT];  // the staged records' first three float4, one array each (conflict-free stores)
   uint32_t sidx[NT];
   uint32_t soff[NT + 1];
   uint32_t sgeo[NT];  // lx0 | ly0 << 4 | bw << 8 | ceil(65536 / pairs per row) << 13
-  uint16_t sskip[NT];  // bit ly: the walk skips the record's left-column pixel in tile row ly
+  // bit ly: the walk skips the record's left-column pixel in tile row ly (0
+  // when that column lies left of the tile)
+  uint16_t sskip[NT];
   // the covered pixels of pass 0 kept for the id pass: depth, and pixel |
-  // staged record << 8; slot k of thread t at k * NT + t
-  uint32_t scd[ID && raster_cache_slots<NT>() ? raster_cache_slots<NT>() * NT : 1];
-  uint32_t scm[ID && raster_cache_slots<NT>() ? raster_cache_slots<NT>() * NT : 1];
+  // record << 8 (the staged slot in one-chunk tiles, else the pass's record);
+  // warp w's list at w * kHitCap
+  uint2 hits[ID && raster_hits<NT>() ? raster_hits<NT>() : 1];
   uint32_t sdepth[kTilePixels];
   unsigned long long sid[kTilePixels];
   uint32_t swarp[NT / 32];
   uint32_t sscan;
   uint32_t ssamples;
+  uint32_t szcap;  // every coverable pixel of the tile ends at this depth or nearer
   Surface S;
   uint32_t s;  // the tile's surface
   uint32_t lists[4];
@@ -918,7 +930,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   constexpr bool with_id = ID;
   constexpr int NW = NT / 32;
   constexpr uint32_t kCountShift = 18;  // scan word: pixels (< 2^18) | records << 18
-  float4 (&srec)[4][NT] = sm.srec;
+  float4 (&srec)[3][NT] = sm.srec;
   uint32_t* sidx = sm.sidx;
   uint32_t* soff = sm.soff;
   uint32_t* sgeo = sm.sgeo;
@@ -952,6 +964,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
     lists[2] = ftot + ws.coarse_off[ct];
     lists[3] = ws.coarse_count[ct];
     ssamples = 0;
+    sm.szcap = kDepthClear;
   }
   if (with_id) {
     for (int p = tid; p < kTilePixels; p += NT) {
@@ -1019,17 +1032,39 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   // minimum of (key << 32 | record), with half the shared-memory traffic.
   const bool packed = with_id && resident && ws.pack_keys;
   uint32_t* sid32 = reinterpret_cast<uint32_t*>(sid);
-  // the covered tests of pass 0 (resident tiles), up to kRasterCache per
-  // thread, kept in sm.scd / sm.scm; nh counts them
+  // the warp's list of covered pixels and its length
+  uint2* hits = sm.hits + warp * (with_id && raster_hits<NT>() ? kHitCap : 0);
   uint32_t nh = 0;
+  bool listing = with_id && raster_hits<NT>() > 0 && (resident || ws.rec_cap <= kHitRecords);
   uint32_t wsamples = 0;  // covered tests of pass 0 seen by this warp
   bool cached = false;
   for (int pass = 0; pass < passes; pass++) {
     for (uint32_t c0 = 0; c0 < ntotal; c0 += NT) {
       const uint32_t m = min((uint32_t)NT, ntotal - c0);
+      if (cached) {
+        // pass 1 from the lists of pass 0
+        if (c0 == 0) {
+          for (uint32_t g = lane; g < nh; g += 32) {
+            const uint2 e = hits[g];
+            const int p = (int)(e.y & 0xFF);
+            const uint32_t lo = e.y >> 8;
+            const uint32_t d = e.x, fd = sdepth[swz32(p)];
+            if (d > fd - kBufError && d < fd + kBufError) {
+              if (!resident)
+                atomicMin(&sid[swz64(p)], ((unsigned long long)__ldg(&ws.rec[lo].key) << 32) | lo);
+              else if (packed)
+                atomicMin(sid32 + swz32(p), (__float_as_uint(srec[2][lo].w) << kSlotBits) | lo);
+              else
+                atomicMin(&sid[swz64(p)], ((unsigned long long)__float_as_uint(srec[2][lo].w) << 32) | sidx[lo]);
+            }
+          }
+        }
+        break;
+      }
       if (!(resident && pass == 1)) {
         if (pass != 0 || c0 != 0) __syncthreads();  // the previous chunk's readers are done
         uint32_t area = 0, r = 0, geo = 0, skip = 0;
+        int bx0 = 0, bx1 = 0, by0 = 0, by1 = 0;
         float4 q0, q1, q2, q3;
         if ((uint32_t)tid < m) {
           const uint32_t e = c0 + tid;
@@ -1040,8 +1075,8 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           q2 = __ldg(src + 2);
           q3 = __ldg(src + 3);
           const uint32_t xr = __float_as_uint(q3.x), yr = __float_as_uint(q3.y);
-          const int bx0 = max((int)(xr & 0xFFFF), tx0), bx1 = min((int)(xr >> 16), tx0 + kTile);
-          const int by0 = max((int)(yr & 0xFFFF), ty0), by1 = min((int)(yr >> 16), ty0 + kTile);
+          bx0 = max((int)(xr & 0xFFFF), tx0), bx1 = min((int)(xr >> 16), tx0 + kTile);
+          by0 = max((int)(yr & 0xFFFF), ty0), by1 = min((int)(yr >> 16), ty0 + kTile);
           if (bx1 > bx0 && by1 > by0) {
             // the tests are horizontal pixel pairs: ceil(bw / 2) per row
             const uint32_t bw = (uint32_t)(bx1 - bx0), pw = (bw + 1) >> 1;
@@ -1051,6 +1086,35 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             if ((int)(xr & 0xFFFF) >= tx0) skip = walk_skip_rows(xr, yr, by0, by1, ty0, chunk);
           }
         }
+        // Depth cull.  A record that covers every coverable pixel of the tile
+        // bounds their final depths by its own farthest depth here; a record
+        // whose nearest depth lies 20 or more behind such a bound changes
+        // neither the depths nor (outside kernel2's window) the ids, so when
+        // it covers its whole box its pixels are only counted.  The bound
+        // comes from the chunks before this one and the warp's own records.
+        // (Coverable: a bbox ends at the surface's last column and row, which
+        // stay clear.)
+        const bool whole = area && bx0 == tx0 && by0 == ty0 && bx1 == min(tx0 + kTile, S.width - 1) &&
+                           by1 == min(ty0 + kTile, S.height - 1) && !skip;
+        uint32_t zcap = __shfl_sync(0xFFFFFFFFu, sm.szcap, 0);
+        if (__any_sync(0xFFFFFFFFu, whole) || zcap != kDepthClear) {
+          bool full = false;
+          uint32_t dlo = 0, dhi = kDepthClear;
+          if (area)
+            full = box_bounds(q0.x, q0.y, q0.z, EdgeTest{q1.x, q1.y, q1.z, q2.x, q2.y, q2.z, q1.w, q0.w}, bx0, by0,
+                              bx1 - 1, by1 - 1, &dlo, &dhi);
+          const uint32_t bound = __reduce_min_sync(0xFFFFFFFFu, full && whole ? dhi : kDepthClear);
+          if (bound < zcap) {
+            zcap = bound;
+            if (lane == 0) atomicMin(&sm.szcap, bound);
+          }
+          uint32_t hidden = 0;
+          if (full && zcap < kDepthClear - kBufError && dlo >= zcap + kBufError) {
+            hidden = (uint32_t)((bx1 - bx0) * (by1 - by0)) - (uint32_t)__popc(skip);
+            area = 0;
+          }
+          if (pass == 0) wsamples += __reduce_add_sync(0xFFFFFFFFu, hidden);
+        }
         const uint32_t word = area ? (area | (1u << kCountShift)) : 0u;
         uint32_t tot = 0;
         const uint32_t off = block_excl_scan1<NT>(word, swarp, &tot);
@@ -1059,7 +1123,6 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           srec[0][slot] = q0;
           srec[1][slot] = q1;
           srec[2][slot] = q2;
-          srec[3][slot] = q3;
           sidx[slot] = r;
           sgeo[slot] = geo;
           sskip[slot] = (uint16_t)skip;
@@ -1073,27 +1136,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       }
       const uint32_t nstaged = sscan >> kCountShift;
       const uint32_t total = soff[nstaged];
-      if (resident && pass == 1 && cached) {
-        // pass 1 from the tests pass 0 kept
-        for (uint32_t g = 0; g < nh; g++) {
-          const uint32_t cm = sm.scm[g * NT + tid];
-          const int p = (int)(cm & 0xFF);
-          const uint32_t lo = (cm >> 8) & 0x3FF;
-          const uint32_t d = sm.scd[g * NT + tid], fd = sdepth[swz32(p)];
-          if (d > fd - kBufError && d < fd + kBufError) {
-            const uint32_t key = __float_as_uint(srec[2][lo].w);
-            if (packed)
-              atomicMin(sid32 + swz32(p), (key << kSlotBits) | lo);
-            else
-              atomicMin(&sid[swz64(p)], ((unsigned long long)key << 32) | sidx[lo]);
-          }
-        }
-        continue;
-      }
       // this warp's contiguous range of the test list, in windows of 32
       const uint32_t per = ((total + NW * 32 - 1) / (NW * 32)) * 32;
       const uint32_t start = min(total, (uint32_t)warp * per), end = min(total, start + per);
-      const bool keep = resident && pass == 0 && with_id && raster_cache_slots<NT>() > 0;
       if (start < end) {
         // first record: the last staged record with soff <= start (warp-uniform)
         int rec = 0, hi = (int)nstaged - 1;
@@ -1110,7 +1155,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           const uint32_t upto = lane == 31 ? starts : starts & ((2u << lane) - 1u);
           const uint32_t lo = (uint32_t)rec + __popc(upto);
           const uint32_t t = base + lane;
-          uint32_t nhit = 0;
+          bool h0 = false, h1 = false;
+          int x = 0, y = 0, p = 0;
+          float4 q[3];
           if (t < end) {
             // test t of the record: the pixel pair (lx, ly), (lx + 1, ly)
             const uint32_t geo = sgeo[lo];
@@ -1118,40 +1165,41 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             const uint32_t bw = (geo >> 8) & 0x1F, pw = (bw + 1) >> 1;
             const uint32_t ry = (local * (geo >> 13)) >> 16, rp = local - ry * pw;
             const int lx = (int)(geo & 0xF) + 2 * (int)rp, ly = (int)((geo >> 4) & 0xF) + (int)ry;
-            const float4 q[4] = {srec[0][lo], srec[1][lo], srec[2][lo], srec[3][lo]};
-            const int x = tx0 + lx, y = ty0 + ly;
-            // covers_in_bbox, the walk rule from the staged mask (only the
-            // first pixel of a pair can be the bbox's left column)
-            const bool h0 = !(x == (int)(__float_as_uint(q[3].x) & 0xFFFF) && ((sskip[lo] >> ly) & 1)) &&
-                            rec_in_tri(q, x, y);
-            const bool h1 = 2 * rp + 1 < bw && rec_in_tri(q, x + 1, y);
-            auto resolve = [&](int px, int plx) {
-              const uint32_t d = depth_at(q[0].x, q[0].y, q[0].z, (float)px, (float)y);
-              const int p = ly * kTile + plx;
-              if (pass == 0) {
-                atomicMin(&sdepth[swz32(p)], d);
-                if (keep) {
-                  if (nh < (uint32_t)raster_cache_slots<NT>()) {
-                    sm.scd[nh * NT + tid] = d;
-                    sm.scm[nh * NT + tid] = (uint32_t)p | (lo << 8);
-                  }
-                  nh++;
-                }
-              } else {
-                const uint32_t fd = sdepth[swz32(p)];
-                if (d > fd - kBufError && d < fd + kBufError) {
-                  if (packed)
-                    atomicMin(sid32 + swz32(p), (__float_as_uint(q[2].w) << kSlotBits) | lo);
-                  else
-                    atomicMin(&sid[swz64(p)], ((unsigned long long)__float_as_uint(q[2].w) << 32) | sidx[lo]);
-                }
-              }
-            };
-            if (h0) resolve(x, lx);
-            if (h1) resolve(x + 1, lx + 1);
-            nhit = (uint32_t)h0 + (uint32_t)h1;
+            q[0] = srec[0][lo], q[1] = srec[1][lo], q[2] = srec[2][lo];
+            x = tx0 + lx, y = ty0 + ly, p = ly * kTile + lx;
+            // the walk rule from the staged mask (only a row's first pixel
+            // can be the bbox's left column), then point_in_tri
+            h0 = !(rp == 0 && ((sskip[lo] >> ly) & 1)) && rec_in_tri(q, x, y);
+            h1 = 2 * rp + 1 < bw && rec_in_tri(q, x + 1, y);
           }
-          if (pass == 0) wsamples += __reduce_add_sync(0xFFFFFFFFu, nhit);
+          const unsigned b0 = __ballot_sync(0xFFFFFFFFu, h0), b1 = __ballot_sync(0xFFFFFFFFu, h1);
+          const uint32_t n0 = (uint32_t)__popc(b0), n1 = (uint32_t)__popc(b1);
+          if (pass == 0) {
+            wsamples += n0 + n1;
+            if (listing && nh + n0 + n1 > (uint32_t)kHitCap) {  // warp-uniform
+              nh = compact_hits(hits, nh, sdepth);
+              listing = nh + n0 + n1 <= (uint32_t)kHitCap;
+            }
+          }
+          auto resolve = [&](int px, int pp, uint32_t slot) {
+            const uint32_t d = depth_at(q[0].x, q[0].y, q[0].z, (float)px, (float)y);
+            if (pass == 0) {
+              atomicMin(&sdepth[swz32(pp)], d);
+              if (listing) hits[slot] = make_uint2(d, (uint32_t)pp | ((resident ? lo : sidx[lo]) << 8));
+            } else {
+              const uint32_t fd = sdepth[swz32(pp)];
+              if (d > fd - kBufError && d < fd + kBufError) {
+                if (packed)
+                  atomicMin(sid32 + swz32(pp), (__float_as_uint(q[2].w) << kSlotBits) | lo);
+                else
+                  atomicMin(&sid[swz64(pp)], ((unsigned long long)__float_as_uint(q[2].w) << 32) | sidx[lo]);
+              }
+            }
+          };
+          const unsigned below = (1u << lane) - 1u;
+          if (h0) resolve(x, p, nh + (uint32_t)__popc(b0 & below));
+          if (h1) resolve(x + 1, p + 1, nh + n0 + (uint32_t)__popc(b1 & below));
+          if (pass == 0 && listing) nh += n0 + n1;
           // the record of test base + 32: lane 31's, or the next one if it starts there
           rec = (int)((uint32_t)rec + __popc(starts));
           if ((uint32_t)rec + 1 < nstaged && soff[rec + 1] == base + 32) rec++;
@@ -1159,14 +1207,11 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       }
     }
     if (pass == 0 && lane == 0 && wsamples) atomicAdd(&ssamples, wsamples);
-    // a resident tile's id pass reads pass 0's kept tests when every thread's
-    // fit (block-uniform)
-    if (resident && with_id && pass == 0) {
-      const bool over = __syncthreads_or(nh > (uint32_t)raster_cache_slots<NT>()) != 0;
-      cached = raster_cache_slots<NT>() > 0 && !over;
-    } else {
+    // the id pass reads pass 0's lists when every warp's held (block-uniform)
+    if (with_id && pass == 0)
+      cached = __syncthreads_and(listing) != 0;
+    else
       __syncthreads();
-    }
   }
   if (tid == 0 && ssamples) atomicAdd(&ws.ctr->samples, (unsigned long long)ssamples);
   for (int lp = tid; lp < kTilePixels; lp += NT) {

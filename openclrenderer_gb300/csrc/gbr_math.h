@@ -96,17 +96,27 @@ GBR_HD float min3f(float a, float b, float c) { return fmin_(fmin_(a, b), c); }
 GBR_HD float max3f(float a, float b, float c) { return fmax_(fmax_(a, b), c); }
 
 // float -> uint32 conversion: truncate, saturate, NaN -> 0.
+// (The device conversion instructions do exactly that: cvt.rzi clamps to the
+// destination's range and turns NaN into 0.)
 GBR_HD uint32_t f2u_sat(float q) {
+#if defined(__CUDA_ARCH__)
+  return __float2uint_rz(q);
+#else
   if (!(q > 0.0f)) return 0u;
   if (q >= 4294967296.0f) return 0xFFFFFFFFu;
   return (uint32_t)q;
+#endif
 }
 // float -> int32 conversion (convert_int): truncate, saturate, NaN -> 0.
 GBR_HD int32_t f2i_sat(float q) {
+#if defined(__CUDA_ARCH__)
+  return __float2int_rz(q);
+#else
   if (q != q) return 0;
   if (q >= 2147483648.0f) return 2147483647;
   if (q <= -2147483648.0f) return (-2147483647 - 1);
   return (int32_t)q;
+#endif
 }
 
 // ---- pinned vector helpers (component order as OpenCL evaluates) ----------
@@ -342,7 +352,41 @@ GBR_HD bool edge_inside(const EdgeTest& e, float px, float py) {
 // Quantised depth of a covered pixel (cl2.cl:5113-5115).
 GBR_HD uint32_t depth_at(float A, float B, float C, float px, float py) {
   float f = fma_(A, px, fma_(B, py, C));
+#if defined(__CUDA_ARCH__)
+  // 2^32 / f as 2^32 * (1 / f): scaling by a power of two is exact, so both
+  // round 1 / f once, except where 1 / f is subnormal (both then truncate to
+  // 0) or overflows (both saturate).  A reciprocal is the cheaper of the two.
+  return f2u_sat(__frcp_rn(f) * kMulInt);
+#else
   return f2u_sat(fdiv(kMulInt, f));
+#endif
+}
+
+// The depths (depth_at) of a record over the pixels [x0, x1] x [y0, y1] lie in
+// [*dlo, *dhi]; returns whether edge_inside holds at every one of them.  Each
+// step of edge_inside's s and t and of the depth plane is a rounded operation
+// monotone in x and in y, so their extrema over the box are the values at its
+// corners, rounding included; s + t is bounded by the rounded sum of the two
+// maxima.  A plane that is not positive over the whole box gives the bounds 0
+// and UINT_MAX (the depth wraps there), and a NaN fails every comparison.
+GBR_HD bool box_bounds(float A, float B, float C, const EdgeTest& e, int x0, int y0, int x1, int y1, uint32_t* dlo,
+                       uint32_t* dhi) {
+  const float fx0 = (float)x0, fx1 = (float)x1, fy0 = (float)y0, fy1 = (float)y1;
+  const bool sx = e.sa * e.sign >= 0.0f, sy = e.sb * e.sign >= 0.0f;
+  const float smax = ((e.s0 + e.sa * (sx ? fx1 : fx0)) + e.sb * (sy ? fy1 : fy0)) * e.sign;
+  const float smin = ((e.s0 + e.sa * (sx ? fx0 : fx1)) + e.sb * (sy ? fy0 : fy1)) * e.sign;
+  const bool tx = e.ta * e.sign >= 0.0f, ty = e.tb * e.sign >= 0.0f;
+  const float tmax = ((e.t0 + e.ta * (tx ? fx1 : fx0)) + e.tb * (ty ? fy1 : fy0)) * e.sign;
+  const float tmin = ((e.t0 + e.ta * (tx ? fx0 : fx1)) + e.tb * (ty ? fy0 : fy1)) * e.sign;
+  const bool ax = A >= 0.0f, ay = B >= 0.0f;
+  const float fmin = fma_(A, ax ? fx0 : fx1, fma_(B, ay ? fy0 : fy1, C));
+  *dlo = 0;
+  *dhi = kDepthClear;
+  if (fmin > 0.0f) {
+    *dlo = depth_at(A, B, C, ax ? fx1 : fx0, ay ? fy1 : fy0);
+    *dhi = depth_at(A, B, C, ax ? fx0 : fx1, ay ? fy0 : fy1);
+  }
+  return smin > -0.0001f && tmin > -0.0001f && (smax + tmax) < e.bound;
 }
 
 // ---- the fragment walk ------------------------------------------------------
@@ -368,6 +412,15 @@ GBR_HD bool walk_visits(int j, int r, int w, int h, float miny, int chunk) {
   int r1 = r + 1;
   return r1 < h && ((r1 * w) % chunk) == 0 && walk_row_late(w, miny, r1);
 }
+
+// The first row that walk_row_late can find late: row r of a bbox with top
+// row miny is never late while r <= miny.  RN(1 / w) is below 1 / w by at
+// most a relative 2^-24, so the walk's position lies below miny + r by at most
+// r * 2^-24, which fmaf rounds away unless it exceeds half the spacing of the
+// floats just below v = miny + r: 2^(k-24) for v in (2^k, 2^(k+1)), 2^(k-25)
+// for v = 2^k.  Either needs r > v / 2, that is r > miny.  (Row 0 is never
+// late.)
+GBR_HD int walk_first_late_row(int miny) { return miny + 1; }
 
 // Largest resolution for which walk_visits is proven exact.
 constexpr int kMaxWalkWidth = 3840;

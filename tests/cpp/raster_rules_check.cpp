@@ -1,0 +1,61 @@
+// Checks the tile rasteriser's shortcuts (gbr_math.h) against what they stand
+// for: walk_first_late_row against walk_row_late over every width <= W, top
+// row < H and row (a row before it must not be late), and box_bounds against
+// depth_at and edge_inside at every pixel of random triangles' boxes.
+// Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+
+#include "gbr_math.h"
+
+using namespace gbr;
+
+int main(int argc, char** argv) {
+  if (argc < 4) return 2;
+  const int W = atoi(argv[1]), H = atoi(argv[2]), n = atoi(argv[3]);
+  long early = 0, late = 0;
+#pragma omp parallel for schedule(dynamic, 8) reduction(+ : early, late)
+  for (int w = 1; w <= W; w++)
+    for (int miny = 0; miny < H; miny++) {
+      const float iw = 1.0f / (float)w, fm = (float)miny;  // walk_row_late's arithmetic, 1 / w hoisted
+      for (int r = 0; r <= H - miny; r++) {
+        const bool l = floorf(fmaf((float)(r * w), iw, fm)) != fm + (float)r;
+        early += l && r < walk_first_late_row(miny);
+        late += l;
+      }
+    }
+  std::mt19937 rng(5);
+  auto uni = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(rng); };
+  long bad = 0, full = 0, bounded = 0;
+  for (int i = 0; i < n; i++) {
+    // vertices from sub-pixel to far off screen, near, far and mixed depths, some degenerate
+    const float span = powf(10.0f, uni(-0.5f, 5.0f));
+    float x[3], y[3], z[3];
+    const float z0 = powf(10.0f, uni(1.31f, 5.54f));
+    for (int k = 0; k < 3; k++) {
+      x[k] = roundf(uni(-span, span) + 800.0f);
+      y[k] = roundf(uni(-span, span) + 500.0f);
+      z[k] = (rng() & 3) ? z0 : powf(10.0f, uni(1.31f, 5.54f));
+    }
+    if (!(rng() & 15)) x[2] = x[1], y[2] = y[1];
+    const f3 xv = mk3(x[0], x[1], x[2]), yv = mk3(y[0], y[1], y[2]);
+    const f3 dv = mk3(rcp(fdiv(z[0], kDepthFar)), rcp(fdiv(z[1], kDepthFar)), rcp(fdiv(z[2], kDepthFar)));
+    float A, B, C;
+    plane_const(dv, xv, yv, rconstant(xv, yv), &A, &B, &C);
+    const EdgeTest e = make_edge(x[0], y[0], x[1], y[1], x[2], y[2]);
+    const int x0 = (int)(rng() % 1600), y0 = (int)(rng() % 1000), x1 = x0 + (int)(rng() % 16), y1 = y0 + (int)(rng() % 16);
+    uint32_t lo, hi;
+    const bool f = box_bounds(A, B, C, e, x0, y0, x1, y1, &lo, &hi);
+    full += f;
+    bounded += lo != 0;
+    for (int py = y0; py <= y1; py++)
+      for (int px = x0; px <= x1; px++) {
+        const uint32_t d = depth_at(A, B, C, (float)px, (float)py);
+        if (d < lo || d > hi || (f && !edge_inside(e, (float)px, (float)py))) bad++;
+      }
+  }
+  printf("early=%ld late=%ld boxes=%d full=%ld bounded=%ld bad=%ld\n", early, late, n, full, bounded, bad);
+  return early == 0 && late > 0 && bad == 0 && full > 0 && bounded > 0 ? 0 : 1;
+}

@@ -1,0 +1,74 @@
+"""Tiles the rasteriser treats specially: records that cover whole tiles and hide others, more
+records than one chunk stages, more covered pixels than the id pass keeps, ragged edges."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from openclrenderer_gb300 import structs as S  # noqa: E402
+from openclrenderer_gb300.pipeline import GpuScene  # noqa: E402
+from oracle import oracle as O  # noqa: E402
+from tests.scene_util import screen_tri, tri_scene  # noqa: E402
+
+TWO_SIDED = [S.make_descriptor(tid=0, feature_flag=S.FLAG_TWO_SIDED)]
+
+
+def layers(w, h, n_big, n_small, gap, seed):
+    """n_big tilted screen-covering triangles `gap` apart in depth (0: all coplanar), and small ones between them."""
+    rng = np.random.default_rng(seed)
+    tl = []
+    for i in rng.permutation(n_big):
+        z = 500.0 + gap * i + rng.uniform(0, 2.0, 3) * (gap > 0)
+        tl.append(screen_tri([-w, 3 * w, -w], [-h, -h, 3 * h], z, w, h))
+    for _ in range(n_small):
+        c, r = rng.uniform(0, 1, 2) * (w, h), rng.uniform(0.5, 20.0)
+        a = rng.uniform(0, 2 * np.pi, 3)
+        tl.append(screen_tri(c[0] + r * np.cos(a), c[1] + r * np.sin(a), rng.uniform(400, 500 + gap * n_big + 100), w, h))
+    return tri_scene(tl, w, h, descs=np.stack(TWO_SIDED))
+
+
+@pytest.mark.parametrize("w,h", [(2, 2), (16, 16), (17, 33), (130, 47), (129, 64)])
+@pytest.mark.parametrize("n_big,n_small,gap", [(1, 0, 1.0), (3, 40, 50.0), (150, 300, 5.0), (300, 0, 0.0), (600, 500, 0.01)])
+def test_layers(w, h, n_big, n_small, gap):
+    sc = layers(w, h, n_big, n_small, gap, seed=w + n_big)
+    gs = GpuScene(sc)
+    ref = O.render(sc, O.build_textures(sc.tex_sizes, sc.tex_pixels), sc.cameras[0], sc.views[0])
+    for threads in (128, 256, 512):
+        gs.set_tuning(S.PASS_VIEW, raster_threads=threads)
+        got = gs.render(sc.cameras[0], sc.views[0]).numpy()
+        assert np.array_equal(got["depth"], ref["depth"])
+        assert np.array_equal(got["id"], ref["id"])
+        assert np.abs(got["rgba"].astype(int) - ref["rgba"].astype(int)).max() <= 1
+    gs.close()
+
+
+def test_samples_count_hidden_records():
+    """view_samples counts every covered (record, pixel) pair, hidden ones too: the sum over the records alone."""
+    sc = layers(75, 50, 40, 60, 30.0, seed=9)
+    gs = GpuScene(sc)
+    gs.render(sc.cameras[0], sc.views[0])
+    total, alone = gs.stats()["view_samples"], 0
+    for t in range(len(sc.tris)):
+        gs.set_triangles(sc.tris[t:t + 1])
+        alone += int((gs.render(sc.cameras[0], sc.views[0]).numpy()["depth"] != 0xFFFFFFFF).sum())
+    assert total == alone
+    gs.close()
+
+
+def test_hidden_cube_face_records():
+    """Cubemap tiles with walls behind one another."""
+    tl = []
+    for z in (300.0, 420.0, 360.0, 300.5, 900.0):
+        tl.append([(-2000, -2000, z), (6000, -2000, z), (-2000, 6000, z)])
+        tl.append([(z, -2000, -2000), (z, 6000, -2000), (z, -2000, 6000)])
+    sc = tri_scene(tl, 64, 48, descs=np.stack(TWO_SIDED),
+                   lights=np.stack([S.make_light((0, 0, 0), radius=5000.0, shadow=1)]))
+    gs = GpuScene(sc)
+    gs.shadow_pass()
+    dyn, _ = O.shadow(sc)
+    assert np.array_equal(gs.cubemaps()[:len(dyn)], dyn)
+    gs.close()
