@@ -353,7 +353,7 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
     CU(mark(5, st));
   } else if (view && sh.shade) {
     CU(mark(6, st));
-    CU(launch_shade(sd, wm.views.p, sh.nitems, wm.surf.p, sh.nfine, ws, st, sh.features));
+    CU(launch_shade(sd, wm.views.p, sh.nitems, wm.surf.p, sh.nfine, ws, st, sh.features, 0, sh.one_view, sh.one_surf));
     CU(mark(5, st));
   }
   CU(cudaMemcpyAsync(host_ctr, ws.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
@@ -977,6 +977,10 @@ static gbr_status render_views(gbr_scene* s, uint32_t n, const gbr_camera* cams,
   sh.ncoarse = cb;
   sh.npix = npix;
   sh.nobjects = s->ndescs;
+  if (n == 1) {
+    sh.one_view = vp.data();
+    sh.one_surf = surfs.data();
+  }
   sh.shade = false;
   for (uint32_t i = 0; i < n; i++) {
     if (outs[i].rgba || outs[i].normals) sh.shade = true;

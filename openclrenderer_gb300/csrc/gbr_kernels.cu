@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "gbr_internal.h"
+#include "gbr_shade_math.h"
 
 namespace gbr {
 namespace {
@@ -867,8 +868,11 @@ __device__ __forceinline__ int swz32(int p) {
 __device__ __forceinline__ int swz64(int p) { return p ^ ((p >> 4) & 15); }
 
 // kernel3's RGBA8 output word
+// (quant8 of each channel: saturation is the clamp, NaN included, and the
+// truncation to a byte is the low byte of an addition of 2^23 rounded toward zero)
 __device__ __forceinline__ uint32_t pack_rgba(float r, float g, float b, float a) {
-  return quant8(r) | (quant8(g) << 8) | (quant8(b) << 16) | (quant8(a) << 24);
+  auto q = [](float v) { return __float_as_uint(__fadd_rz(__saturatef(v) * 255.0f + 0.5f, 8388608.0f)); };
+  return __byte_perm(__byte_perm(q(r), q(g), 0x0040), __byte_perm(q(b), q(a), 0x0040), 0x5410);
 }
 
 // Drops the entries of a warp's list that are 20 or more behind their pixel's
@@ -1249,13 +1253,9 @@ struct ShadeCtx {
   const Surface* S;
 };
 
-// (float)d / 2^32 * 350000: the division by 2^32 only shifts the exponent
-// (no rounding, no underflow for d >= 1), so it is a multiplication by 2^-32.
-constexpr float kInvMulInt = 2.3283064365386963e-10f;
-__device__ __forceinline__ float depth_to_dist(uint32_t d) { return ((float)d * kInvMulInt) * kDepthFar; }
-
-// Exact byte -> float without a conversion instruction: 2^23 + b, minus 2^23.
-__device__ __forceinline__ float u8f(uint32_t b) { return __uint_as_float(0x4B000000u | b) - 8388608.0f; }
+// Byte -> float: one conversion that selects its byte (kernel3 0.6 % fewer
+// instructions than 2^23 + b, minus 2^23; the conversion pipe is a third busy).
+__device__ __forceinline__ float u8f(uint32_t b) { return (float)(uint8_t)b; }
 
 // read_tex_array_all_precalculated (cl2.cl:823-851) in one atlas slot of the
 // texture level table: (ox, oy) is the slot origin in its page, tnum * width
@@ -1291,37 +1291,65 @@ __device__ __forceinline__ int texel_coord(float pos, int plus, int w) {
   return min(max(p, 0), w - 1);
 }
 
-// COLOUR: the result only scales the colour (the texel colour), so the blend
-// may contract; the normal map's fetch, which feeds the exact normal, keeps
-// the plain products.
-template <bool COLOUR>
-__device__ f4 bilinear_pre(const TexSlot& ts, float mx, float my) {
-  float posx = floorf(mx), posy = floorf(my);
+// The four texels of a bilinear footprint and its weights.
+struct Footprint {
+  int x0, x1, y0, y1;
+  float ux, uy;
+};
+__device__ __forceinline__ Footprint footprint_at(const TexSlot& ts, float mx, float my) {
+  Footprint f;
+  const float posx = floorf(mx), posy = floorf(my);
   const int w = (int)ts.width, ox = (int)ts.ox, oy = (int)ts.oy;
-  const int x0 = ox + texel_coord(posx, 0, w), x1 = ox + texel_coord(posx, 1, w);
-  const int y0 = oy + texel_coord(posy, 0, w), y1 = oy + texel_coord(posy, 1, w);
-  f4 c0 = texel(ts, x0, y0);
-  f4 c1 = texel(ts, x1, y0);
-  f4 c2 = texel(ts, x0, y1);
-  f4 c3 = texel(ts, x1, y1);
-  float ux = mx - posx, uy = my - posy;
-  float bx = 1.0f - ux, by = 1.0f - uy;
+  f.x0 = ox + texel_coord(posx, 0, w), f.x1 = ox + texel_coord(posx, 1, w);
+  f.y0 = oy + texel_coord(posy, 0, w), f.y1 = oy + texel_coord(posy, 1, w);
+  f.ux = mx - posx, f.uy = my - posy;
+  return f;
+}
+
+// The bilinear fetch of the normal map and the reflection map, which feed
+// decisions: plain products.
+__device__ f4 bilinear_exact(const TexSlot& ts, float mx, float my) {
+  const Footprint f = footprint_at(ts, mx, my);
+  const f4 c0 = texel(ts, f.x0, f.y0), c1 = texel(ts, f.x1, f.y0), c2 = texel(ts, f.x0, f.y1),
+           c3 = texel(ts, f.x1, f.y1);
+  const float ux = f.ux, uy = f.uy, bx = 1.0f - ux, by = 1.0f - uy;
   f4 r;
-  if (COLOUR) {
-    r.x = fma_(fma_(c2.x, bx, c3.x * ux), uy, fma_(c0.x, bx, c1.x * ux) * by);
-    r.y = fma_(fma_(c2.y, bx, c3.y * ux), uy, fma_(c0.y, bx, c1.y * ux) * by);
-    r.z = fma_(fma_(c2.z, bx, c3.z * ux), uy, fma_(c0.z, bx, c1.z * ux) * by);
-    r.w = fma_(fma_(c2.w, bx, c3.w * ux), uy, fma_(c0.w, bx, c1.w * ux) * by);
-  } else {
-    r.x = fma_(c0.x, bx, c1.x * ux) * by + fma_(c2.x, bx, c3.x * ux) * uy;
-    r.y = fma_(c0.y, bx, c1.y * ux) * by + fma_(c2.y, bx, c3.y * ux) * uy;
-    r.z = fma_(c0.z, bx, c1.z * ux) * by + fma_(c2.z, bx, c3.z * ux) * uy;
-    r.w = fma_(c0.w, bx, c1.w * ux) * by + fma_(c2.w, bx, c3.w * ux) * uy;
-  }
+  r.x = fma_(c0.x, bx, c1.x * ux) * by + fma_(c2.x, bx, c3.x * ux) * uy;
+  r.y = fma_(c0.y, bx, c1.y * ux) * by + fma_(c2.y, bx, c3.y * ux) * uy;
+  r.z = fma_(c0.z, bx, c1.z * ux) * by + fma_(c2.z, bx, c3.z * ux) * uy;
+  r.w = fma_(c0.w, bx, c1.w * ux) * by + fma_(c2.w, bx, c3.w * ux) * uy;
   return r;
 }
 
-// texture_filter_diff (cl2.cl:1511-1573); COLOUR as for bilinear_pre.  The
+// The bilinear fetch of a texel colour, which only scales the colour: the
+// blend is contracted, and two channels go through one packed instruction.
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+struct Texel2 {
+  float2 rg, ba;
+};
+__device__ __forceinline__ Texel2 texel2(const TexSlot& ts, int ix, int iy) {
+  const uint32_t t = __ldg(reinterpret_cast<const uint32_t*>(ts.page) + ((size_t)iy * kTexPage + ix));
+  Texel2 r;
+  r.rg = make_float2(u8f(t & 0xFF), u8f((t >> 8) & 0xFF));
+  r.ba = make_float2(u8f((t >> 16) & 0xFF), u8f(t >> 24));
+  return r;
+}
+__device__ __forceinline__ Texel2 bilinear_colour(const TexSlot& ts, float mx, float my) {
+  const Footprint f = footprint_at(ts, mx, my);
+  const Texel2 c0 = texel2(ts, f.x0, f.y0), c1 = texel2(ts, f.x1, f.y0), c2 = texel2(ts, f.x0, f.y1),
+               c3 = texel2(ts, f.x1, f.y1);
+  const float2 u = dup2(f.ux), v = dup2(f.uy), bx = dup2(1.0f - f.ux), by = dup2(1.0f - f.uy);
+  auto blend = [&](float2 a0, float2 a1, float2 a2, float2 a3) {
+    return __ffma2_rn(__ffma2_rn(a2, bx, __fmul2_rn(a3, u)), v, __fmul2_rn(__ffma2_rn(a0, bx, __fmul2_rn(a1, u)), by));
+  };
+  Texel2 r;
+  r.rg = blend(c0.rg, c1.rg, c2.rg, c3.rg);
+  r.ba = blend(c0.ba, c1.ba, c2.ba, c3.ba);
+  return r;
+}
+
+// texture_filter_diff (cl2.cl:1511-1573); COLOUR: bilinear_colour's blend, in
+// packed channels (1080p kernel3 1 % fewer instructions).  The
 // two mip levels come from the texture level table: level mip_lower (the
 // texture itself at 0) and level min(mip_lower, 3) + 1, the slots the
 // reference's tid_lower / tid_higher name.
@@ -1337,37 +1365,24 @@ __device__ f4 texture_filter_diff(const SceneDev& sc, f2 vt, f2 vtdiff, int tid2
   float fmd = wif - mip_lower;
   const int lo = (int)mip_lower, hi = min(lo, kMipLevels - 1) + 1;
   const TexSlot sl = level_slot(sc, __ldg(lv + lo)), sh = level_slot(sc, __ldg(lv + hi));
-  f4 c1 = bilinear_pre<COLOUR>(sl, vtm.x * sl.width, vtm.y * sl.width);
-  f4 c2 = bilinear_pre<COLOUR>(sh, vtm.x * sh.width, vtm.y * sh.width);
   const float i255 = 1.0f / 255.0f;
   f4 r;
   if (COLOUR) {
-    r.x = fma_(c2.x - c1.x, fmd, c1.x) * i255;
-    r.y = fma_(c2.y - c1.y, fmd, c1.y) * i255;
-    r.z = fma_(c2.z - c1.z, fmd, c1.z) * i255;
-    r.w = fma_(c2.w - c1.w, fmd, c1.w) * i255;
+    const Texel2 c1 = bilinear_colour(sl, vtm.x * sl.width, vtm.y * sl.width);
+    const Texel2 c2 = bilinear_colour(sh, vtm.x * sh.width, vtm.y * sh.width);
+    const float2 f = dup2(fmd), k = dup2(i255), neg = dup2(-1.0f);  // fma(c1, -1, c2) = c2 - c1
+    const float2 rg = __fmul2_rn(__ffma2_rn(__ffma2_rn(c1.rg, neg, c2.rg), f, c1.rg), k);
+    const float2 ba = __fmul2_rn(__ffma2_rn(__ffma2_rn(c1.ba, neg, c2.ba), f, c1.ba), k);
+    r.x = rg.x; r.y = rg.y; r.z = ba.x; r.w = ba.y;
   } else {
+    const f4 c1 = bilinear_exact(sl, vtm.x * sl.width, vtm.y * sl.width);
+    const f4 c2 = bilinear_exact(sh, vtm.x * sh.width, vtm.y * sh.width);
     r.x = (c1.x + (c2.x - c1.x) * fmd) * i255;
     r.y = (c1.y + (c2.y - c1.y) * fmd) * i255;
     r.z = (c1.z + (c2.z - c1.z) * fmd) * i255;
     r.w = (c1.w + (c2.w - c1.w) * fmd) * i255;
   }
   return r;
-}
-
-// depth_to_dist(d) compared with a threshold t: (float)d * 2^-32 is exact and
-// a scaling by a power of two commutes with rounding (every value here is a
-// normal float), so depth_to_dist(d) = RN((float)d * 350000) * 2^-32, and
-// depth_to_dist(d) > t exactly when RN((float)d * 350000) > t * 2^32.
-constexpr float kTwo32 = 4294967296.0f;
-__device__ __forceinline__ float depth_scaled(uint32_t d) { return (float)d * kDepthFar; }
-
-// How many of the thresholds t0 < t1 < t2 < t3 < t4 lie below d2, i.e.
-// (d2 > t0) + ... + (d2 > t4): the thresholds dep + z (z = -2..2, dep <=
-// 350000) are strictly increasing in float, so the predicates are monotone and
-// three comparisons find the count.
-__device__ __forceinline__ int ssao_count(float d2, float t0, float t1, float t2, float t3, float t4) {
-  return d2 > t2 ? (d2 > t4 ? 5 : (d2 > t3 ? 4 : 3)) : (d2 > t1 ? 2 : (d2 > t0 ? 1 : 0));
 }
 
 // A tap coordinate of generate_ssao: clamped to [1, n - 2] as the reference
@@ -1377,45 +1392,72 @@ __device__ __forceinline__ int ssao_coord(float v, int n) {
   return max((int)clampf_(v, 1.0f, (float)n - 2.0f), 0);
 }
 
-// generate_ssao (cl2.cl:2194-2260).  The 25 taps share 5 rows and 5
-// columns, whose offsets round(k * world_rad), k = -2..2, are the same five
-// values: round is odd-symmetric (half away from zero) and 1 * r, 2 * r and
-// -r, -2 * r are exact, so two roundings give all of them.  The depth
-// thresholds dep + z are computed once, and the count (at most 125, exact in
-// float) is kept in an integer.  Far from the camera (world_rad < 0.25) every
-// offset rounds to 0 and all 25 taps read the same pixel; when that holds for
-// the whole warp, the pixel is read once and its count taken 25 times.
-// seed2 = rand_xorshift(wang_hash(x + W*H*y)), the pixel's first random
-// number, which kernel3's normal jitter also draws.
-// depth is read with plain (coherent) loads: in the fused pass other blocks
-// wrote it during the same launch.
-__device__ float generate_ssao(int x, int y, uint32_t seed2, const uint32_t* depth, int W, int H, float fov) {
-  float foffset = (float)seed2 * kInvMulInt;
-  float dep = depth_to_dist(__ldca(depth + (size_t)y * W + x));
-  float rad = kSsaoRad + foffset * 0.5f;  // foffset / 2, exact
-  float world_rad = fdiv(rad * fov, dep);
+// The 25 taps' counts with the thresholds as the reference adds them up: the
+// few pixels for which ssao_tap is not exact (within 2 units below a power of
+// two, or nearer than 8).
+__device__ __noinline__ int ssao_taps_any(int x, int y, float dep, float world_rad, const uint32_t* depth, int W,
+                                          int H) {
   // the thresholds dep + z, z = -2..2, scaled by 2^32 (depth_scaled)
   const float t0 = (dep + -2.0f) * kTwo32, t1 = (dep + -1.0f) * kTwo32, t2 = dep * kTwo32,
               t3 = (dep + 1.0f) * kTwo32, t4 = (dep + 2.0f) * kTwo32;
   int acc = 0;
-  if (__all_sync(__activemask(), world_rad < 0.25f)) {
-    const float d2 = depth_scaled(__ldca(depth + (size_t)ssao_coord((float)y, H) * W + ssao_coord((float)x, W)));
-    acc = 25 * ssao_count(d2, t0, t1, t2, t3, t4);
+  const float r1 = roundf(world_rad), r2 = roundf(2.0f * world_rad), r0 = roundf(0.0f * world_rad);
+  for (int yy = -2; yy <= 2; yy++) {
+    const float oy = yy == 0 ? r0 : copysignf(yy == 2 || yy == -2 ? r2 : r1, (float)yy);
+    const uint32_t* row = depth + (size_t)ssao_coord((float)y + oy, H) * W;
+    for (int xx = -2; xx <= 2; xx++) {
+      const float ox = xx == 0 ? r0 : copysignf(xx == 2 || xx == -2 ? r2 : r1, (float)xx);
+      acc += ssao_count(depth_scaled(__ldca(row + ssao_coord((float)x + ox, W))), t0, t1, t2, t3, t4);
+    }
+  }
+  return acc;
+}
+
+// ssao_coord(v + off) for an integer offset: max(v + off, 1), then min with
+// n - 2 and max with 0, an instruction each.
+__device__ __forceinline__ int ssao_coord_int(int v, int off, int n) {
+  return __vimin_s32_relu(__viaddmax_s32(v, off, 1), n - 2);
+}
+
+// generate_ssao (cl2.cl:2194-2260) for a pixel of depth d.  The 25 taps share
+// 5 rows and 5 columns, whose offsets round(k * world_rad), k = -2..2, are the
+// same five values: round is odd-symmetric (half away from zero) and 1 * r,
+// 2 * r and -r, -2 * r are exact, so two roundings give all of them; they and
+// the coordinates are small integers.  The count (at most 125, exact in float)
+// is kept in an integer.  Far from the camera (world_rad < 0.25) every offset
+// rounds to 0 and all 25 taps read the same pixel; when that holds for the
+// whole warp, the pixel is read once and its count taken 25 times.
+// seed2 = rand_xorshift(wang_hash(x + W*H*y)), the pixel's first random
+// number, which kernel3's normal jitter also draws.
+// depth is read with plain (coherent) loads: in the fused pass other blocks
+// wrote it during the same launch.
+__device__ float generate_ssao(int x, int y, uint32_t seed2, uint32_t d, const uint32_t* depth, int W, int H,
+                               float fov) {
+  float foffset = (float)seed2 * kInvMulInt;
+  const float dep = depth_to_dist(d);
+  float rad = kSsaoRad + foffset * 0.5f;  // foffset / 2, exact
+  float world_rad = fdiv(rad * fov, dep);
+  int acc = 0;
+  const float c8 = (2.0f - dep) * 0.125f;
+  if (!ssao_exact(dep)) {
+    acc = ssao_taps_any(x, y, dep, world_rad, depth, W, H);
+  } else if (__all_sync(__activemask(), world_rad < 0.25f)) {
+    acc = 25 * (int)(ssao_tap(__ldca(depth + (size_t)ssao_coord_int(y, 0, H) * W + ssao_coord_int(x, 0, W)), c8) -
+                     kSsaoTapZero);
   } else {
-    const float r1 = roundf(world_rad), r2 = roundf(2.0f * world_rad), r0 = roundf(0.0f * world_rad);
-    const float off[5] = {-r2, -r1, r0, r1, r2};
+    const int i1 = min((int)roundf(world_rad), 8192), i2 = min((int)roundf(2.0f * world_rad), 8192);  // views: < 4096
+    const int off[5] = {-i2, -i1, 0, i1, i2};
     int wx[5];
 #pragma unroll
-    for (int k = 0; k < 5; k++) wx[k] = ssao_coord((float)x + off[k], W);
+    for (int k = 0; k < 5; k++) wx[k] = ssao_coord_int(x, off[k], W);
+    uint32_t sum = 0;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-      const uint32_t* row = depth + (size_t)ssao_coord((float)y + off[k], H) * W;
+      const uint32_t* row = depth + (size_t)ssao_coord_int(y, off[k], H) * W;
 #pragma unroll
-      for (int xx = 0; xx < 5; xx++) {
-        const float d2 = depth_scaled(__ldca(row + wx[xx]));
-        acc += ssao_count(d2, t0, t1, t2, t3, t4);
-      }
+      for (int xx = 0; xx < 5; xx++) sum += ssao_tap(__ldca(row + wx[xx]), c8);
     }
+    acc = (int)(sum - 25u * kSsaoTapZero);
   }
   // the occlusion scales the colour only: approximate divisions
   const float facc = (float)acc * (1.0f / 125.0f);
@@ -1481,10 +1523,29 @@ __device__ __forceinline__ f4 vertex_col(uint32_t c) {
 
 // Colour-only arithmetic of the light loop: every use below feeds the colour
 // continuously (no comparison, rounding or index depends on it), so the
-// approximate division is covered by the 1/255 colour tolerance.
-__device__ __forceinline__ float crcp(float b) { return __fdividef(1.0f, b); }
+// approximate division is covered by the 1/255 colour tolerance.  The
+// hardware's approximations, taken as single instructions: __fdividef,
+// rsqrtf and __expf compute the same values but wrap them in three or four
+// more for subnormal operands and results, which here are either exact zeros
+// or far below a colour level.  (1080p kernel3 3,350 -> 3,060 instructions
+// per pixel, 223 -> 210 us.)
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float crcp(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return r;
+}
 __device__ __forceinline__ f3 cnormalize(f3 a) {
-  float r = rsqrtf(dot3(a, a));
+  float r = rsqrt_ftz(dot3(a, a));
   return mk3(a.x * r, a.y * r, a.z * r);
 }
 // Colour-path dot product with contraction.
@@ -1498,10 +1559,12 @@ __device__ __forceinline__ float c_rational_acos(float x) {
 }
 
 
-// Colour-only square root (approximate; exact IEEE result for 0, negative,
-// infinite and NaN inputs).
+// Colour-only square root: 0 for 0, NaN for a negative input.  (An infinite
+// input gives NaN as well; gamma_inv's sum of infinities of both signs is NaN
+// either way.)
 __device__ __forceinline__ float csqrt(float x) {
-  return (x > 0.0f && x < 3.0e38f) ? x * rsqrtf(x) : fsqrt(x);
+  const float s = x * rsqrt_ftz(x);
+  return x == 0.0f ? 0.0f : s;
 }
 // gamma_inv (cl2.cl:5778-5782) on the colour path.
 __device__ __forceinline__ float c_gamma_inv(float c) {
@@ -1551,7 +1614,7 @@ __device__ __forceinline__ void stage_light(const gbr_light* L, bool linear, flo
   const float bw = L->shadow ? brightness : brightness * (1.0f / (1.0f - kLightCutoff));
   dst[0] = make_float4(L->pos[0], L->pos[1], L->pos[2], cut2);
   dst[1] = make_float4(c.x, c.y, c.z, bw);
-  dst[2] = make_float4(radius, crcp(radius), L->diffuse,
+  dst[2] = make_float4(radius, __fdividef(1.0f, radius), L->diffuse,
                        __uint_as_float((L->shadow ? 1u : 0u) | (L->is_static ? 2u : 0u)));
 }
 
@@ -1745,7 +1808,7 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
   const bool two = (ff & kFlagTwoSided) > 0;
   const bool recv_dyn = !((ff & kFlagNoDynShadows) > 0);
   if ((obits >> 31) && two) normal = neg3(normal);  // back-facing (cl2.cl:491-494)
-  const float ssao = generate_ssao(x, y, seed2, S.depth, W, H, fov);
+  const float ssao = generate_ssao(x, y, seed2, d, S.depth, W, H, fov);
   normal = fast_normalize3(normal);
   const f3 lnormal = cnormalize(add3(normal, mk3(rseed.x * 0.01f, rseed.y * 0.01f, rseed.z * 0.01f)));
   const float ambient = V.use_linear ? gamma_fwd(kAmbient) : kAmbient;
@@ -1774,7 +1837,7 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
     const float4 LB = lights[kLightQuads * i + 1], LC = lights[kLightQuads * i + 2];
     const uint32_t lflags = __float_as_uint(LC.w);
     const f3 lcol = mk3(LB.x, LB.y, LB.z);
-    const float rinv = rsqrtf(d2);
+    const float rinv = rsqrt_ftz(d2);
     if (lflags & 1u) {  // a shadow light: its distance in IEEE arithmetic
       const float d2s = dot3(ptl, ptl);
       float occlusion = 1.0f;
@@ -1807,7 +1870,7 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
       const float omv = 1.0f - vdh, omv2 = omv * omv;
       const float fresnel = fma_(0.6f, (omv2 * omv2) * omv, 0.4f);
       const float alpha = c_rational_acos(ndh);
-      const float microfacet = 0.8346f * __expf((alpha * alpha) * nr2);
+      const float microfacet = 0.8346f * ex2_ftz(((alpha * alpha) * nr2) * 1.4426950408889634f);
       const float sv = (2.0f * ndh) * crcp(vdh);
       const float geometric = min3f(1.0f, sv * ndv, sv * ndl);
       const float spec = ((fresnel * microfacet) * geometric) * r_pndv;
@@ -1831,14 +1894,14 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
     // (ptl) through dot products: |v + l|^2 = 2 + 2 v.l, n.H = (n.v + n.l) /
     // |v + l|, v.H = (1 + v.l) / |v + l|
     const float nl = cdot3(normal, ptl), vl = cdot3(l2p, ptl);
-    const float rh = rsqrtf(fma_(2.0f, vl, 2.0f));
+    const float rh = rsqrt_ftz(fma_(2.0f, vl, 2.0f));
     const float vdh = fmax_(0.0f, (1.0f + vl) * rh);
     const float ndh = fmax_(0.0f, (ndv_raw + nl) * rh);
     const float ndl = fmax_(0.0f, nl);
     const float omv = 1.0f - vdh, omv2 = omv * omv;
     const float fresnel = fma_(0.6f, (omv2 * omv2) * omv, 0.4f);
     const float alpha = c_rational_acos(ndh);
-    const float microfacet = 0.8346f * __expf((alpha * alpha) * nr2);
+    const float microfacet = 0.8346f * ex2_ftz(((alpha * alpha) * nr2) * 1.4426950408889634f);
     const float sv = (2.0f * ndh) * crcp(vdh);
     const float geometric = min3f(1.0f, sv * ndv, sv * ndl);
     const float spec = ((fresnel * microfacet) * geometric) * r_pndv;
@@ -1936,6 +1999,15 @@ __device__ __forceinline__ void shade_tile(const SceneDev& sc, const ViewParams*
   }
 }
 
+// 1080p terrain: 2,760 instructions per pixel (3,350 before the
+// approximations as single instructions, the SSAO counts without compares,
+// packed texel blends and the view in the constant bank), 187 us (223); 64
+// sphere views 2.18 ms (2.62).  It is bound by instruction issue (77 %
+// active).  The lights' shared memory is sized by the scene: with room for
+// kMaxLights the L1 lost 3 points of its hit rate (1.4 % of the batch's time).
+// Tiles of 128 or 64 pixels per block were slower (203 / 212 us): their
+// blocks share less in the L1 and start more often.
+//
 // A pass whose setup or binning overflowed its scratch leaves the depth and
 // record map unwritten (the raster returns at once); shading returns too, and
 // the host re-runs the pass with grown scratch.
@@ -1944,15 +2016,22 @@ __device__ __forceinline__ void shade_tile(const SceneDev& sc, const ViewParams*
 // once; tiles (null for one view): each tile's surface (Workspace).  Each
 // thread reads its pixel; empty pixels get the clear colour, covered ones are
 // compacted in pixel order into the first threads, which shade them.
-template <bool FEAT>
-__global__ void __launch_bounds__(256, 4) k_shade(SceneDev sc, const ViewParams* __restrict__ views,
-                                               const Surface* __restrict__ surfs, uint32_t nviews,
-                                               const ShadeRec* __restrict__ srec, const Counters* __restrict__ ctr,
+// ONE: a pass of one view whose parameters come with the launch (one_view,
+// one_surf: constant-bank operands instead of loads that hold registers);
+// otherwise they are read from views / surfs.
+template <bool FEAT, bool ONE>
+__global__ void __launch_bounds__(kTilePixels, 4) k_shade(SceneDev sc,
+                                               const __grid_constant__ ViewParams one_view,
+                                               const __grid_constant__ Surface one_surf,
+                                               const ViewParams* __restrict__ views,
+                                               const Surface* __restrict__ surfs, const ShadeRec* __restrict__ srec,
+                                               const Counters* __restrict__ ctr,
                                                uint32_t rec_cap, uint32_t tile0,
                                                const uint8_t* __restrict__ tile_empty,
                                                const uint2* __restrict__ tiles) {
   constexpr int NW = kTilePixels / 32;
-  __shared__ ShadeSmem sm;
+  extern __shared__ float4 s_lights[];  // kLightQuads per light of the scene
+  __shared__ float s_colx[kTile + 1], s_rowy[kTile + 1];
   __shared__ uint32_t s_warp[NW];
   __shared__ uint32_t s_px[kTilePixels], s_d[kTilePixels], s_r[kTilePixels];
   if (ctr->overflow) return;
@@ -1961,9 +2040,9 @@ __global__ void __launch_bounds__(256, 4) k_shade(SceneDev sc, const ViewParams*
   // every thread reads the tile's flag and surface (the same words): the
   // return is block-uniform and needs no barrier
   if (tile_empty && tile_empty[tile]) return;
-  const uint32_t sid = tiles ? tiles[tile].x : 0u;  // null: one view
-  const Surface& S = surfs[sid];
-  const ViewParams& V = views[sid];
+  const uint32_t sid = !ONE && tiles ? tiles[tile].x : 0u;  // null: one view
+  const Surface& S = ONE ? one_surf : surfs[sid];
+  const ViewParams& V = ONE ? one_view : views[sid];
   const uint32_t lt = tile - S.tile_base;
   const int x0 = (lt % S.tiles_x) * kTile, y0 = (lt / S.tiles_x) * kTile;
   // the thread's own pixel: empty pixels are written at once; covered ones
@@ -1983,13 +2062,13 @@ __global__ void __launch_bounds__(256, 4) k_shade(SceneDev sc, const ViewParams*
   if (inside && !cov) shade_clear<FEAT>(V, p, d);
   const bool linear = V.use_linear != 0;
   for (uint32_t i = threadIdx.x; i < sc.nlights; i += kTilePixels)
-    stage_light(sc.lights + i, linear, sm.lights + kLightQuads * i);
+    stage_light(sc.lights + i, linear, s_lights + kLightQuads * i);
   if (threadIdx.x < 2 * (kTile + 1)) {
     const int i = threadIdx.x % (kTile + 1);
     if (threadIdx.x <= kTile)
-      sm.colx[i] = fdiv((float)(x0 + i) - (float)S.width / 2.0f, V.fov);
+      s_colx[i] = fdiv((float)(x0 + i) - (float)S.width / 2.0f, V.fov);
     else
-      sm.rowy[i] = fdiv((float)(y0 + i) - (float)S.height / 2.0f, V.fov);
+      s_rowy[i] = fdiv((float)(y0 + i) - (float)S.height / 2.0f, V.fov);
   }
   __syncthreads();
   uint32_t base = 0, total = 0;
@@ -2008,8 +2087,8 @@ __global__ void __launch_bounds__(256, 4) k_shade(SceneDev sc, const ViewParams*
   __syncthreads();
   if (threadIdx.x < total) {
     const uint32_t q = s_px[threadIdx.x];
-    shade_covered<FEAT>(sc, V, S, srec, sm.lights, x0 + (int)(q & (kTile - 1)), y0 + (int)(q / kTile),
-                        s_d[threadIdx.x], s_r[threadIdx.x], sm.colx, sm.rowy);
+    shade_covered<FEAT>(sc, V, S, srec, s_lights, x0 + (int)(q & (kTile - 1)), y0 + (int)(q / kTile),
+                        s_d[threadIdx.x], s_r[threadIdx.x], s_colx, s_rowy);
   }
 }
 
@@ -2349,15 +2428,19 @@ cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t n
 }
 
 cudaError_t launch_shade(const SceneDev& sc, const ViewParams* d_views, uint32_t nviews, const Surface* d_surf,
-                         uint32_t ntiles, const Workspace& ws, cudaStream_t st, bool features, uint32_t tile0) {
+                         uint32_t ntiles, const Workspace& ws, cudaStream_t st, bool features, uint32_t tile0,
+                         const ViewParams* one_view, const Surface* one_surf) {
   if (!ntiles) return cudaSuccess;
   if (!sc.objq || !sc.texlv || !ws.srec || (nviews > 1 && !ws.tiles)) return cudaErrorInvalidValue;
+  const bool one = nviews == 1 && one_view && one_surf;
+  auto go = [&](auto kernel) {
+    kernel<<<ntiles, kTilePixels, sizeof(float4) * kLightQuads * sc.nlights, st>>>(sc, one ? *one_view : ViewParams{}, one ? *one_surf : Surface{}, d_views, d_surf,
+                                   ws.srec, ws.ctr, ws.rec_cap, tile0, ws.tile_empty, ws.tiles);
+  };
   if (features)
-    k_shade<true><<<ntiles, 256, 0, st>>>(sc, d_views, d_surf, nviews, ws.srec, ws.ctr, ws.rec_cap, tile0,
-                                          ws.tile_empty, ws.tiles);
+    one ? go(k_shade<true, true>) : go(k_shade<true, false>);
   else
-    k_shade<false><<<ntiles, 256, 0, st>>>(sc, d_views, d_surf, nviews, ws.srec, ws.ctr, ws.rec_cap, tile0,
-                                           ws.tile_empty, ws.tiles);
+    one ? go(k_shade<false, true>) : go(k_shade<false, false>);
   return cudaGetLastError();
 }
 

@@ -126,6 +126,9 @@ struct PassShape {
   uint32_t nseg = 0;                // views: segments of the fused raster -> shade pass (GBR_RS_FUSED)
   uint32_t ngroups = 0;             // views: pipelined groups (GBR_RS_PIPELINED), 0 or >= 2
   uint32_t group_tile[kRsGroups + 1] = {};  // first tile of each group; [ngroups] = all tiles
+  // the view of an uncaptured pass of one view, in host memory until the pass is queued
+  const ViewParams* one_view = nullptr;
+  const Surface* one_surf = nullptr;
 };
 
 // The fused pass's work order over view surfaces (k_raster_shade): each

@@ -1,0 +1,52 @@
+// gbr_shade_math.h — scalar pieces of kernel3 and the post passes that stand
+// for longer expressions of the reference, shared with their host checks.
+#pragma once
+
+#include "gbr_math.h"
+
+namespace gbr {
+
+// (float)d / 2^32 * 350000: the division by 2^32 only shifts the exponent
+// (no rounding, no underflow for d >= 1), so it is a multiplication by 2^-32.
+constexpr float kInvMulInt = 2.3283064365386963e-10f;
+GBR_HD float depth_to_dist(uint32_t d) { return ((float)d * kInvMulInt) * kDepthFar; }
+
+// depth_to_dist(d) compared with a threshold t: (float)d * 2^-32 is exact and
+// a scaling by a power of two commutes with rounding (every value here is a
+// normal float), so depth_to_dist(d) = RN((float)d * 350000) * 2^-32, and
+// depth_to_dist(d) > t exactly when RN((float)d * 350000) > t * 2^32.
+constexpr float kTwo32 = 4294967296.0f;
+GBR_HD float depth_scaled(uint32_t d) { return (float)d * kDepthFar; }
+
+// How many of the thresholds t0 < t1 < t2 < t3 < t4 lie below d2, i.e.
+// (d2 > t0) + ... + (d2 > t4): the thresholds dep + z (z = -2..2, dep <=
+// 350000) are strictly increasing in float, so the predicates are monotone and
+// three comparisons find the count.
+GBR_HD int ssao_count(float d2, float t0, float t1, float t2, float t3, float t4) {
+  return d2 > t2 ? (d2 > t4 ? 5 : (d2 > t3 ? 4 : 3)) : (d2 > t1 ? 2 : (d2 > t0 ? 1 : 0));
+}
+
+// ssao_count of one tap for a pixel at distance dep (ssao_exact), given c8 =
+// (2 - dep) / 8: how many of dep + k, k = -2..2, lie below the tap's distance
+// v.  That is ceil(v - dep + 2) clamped to 0..5, and u = (v - dep + 2) / 8 is
+// one fused operation, exact wherever it falls inside (0, 1) (v and dep are
+// then within a factor of two and share their grid): clamped by saturation,
+// multiplied back and rounded up to an integer by the addition of 1.5 * 2^23.
+// Returns that float's bits, kSsaoTapZero + count: six instructions and no
+// compare or select per tap.
+constexpr uint32_t kSsaoTapZero = 0x4B400000u;
+GBR_HD uint32_t ssao_tap(uint32_t d, float c8) {
+  const float u = fma_(depth_scaled(d), kInvMulInt * 0.125f, c8);
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(fminf(__fmaf_ru(__saturatef(u), 8.0f, 12582912.0f), 12582917.0f));
+#else
+  return kSsaoTapZero + (uint32_t)fminf(ceilf(clampf_(u, 0.0f, 1.0f) * 8.0f), 5.0f);
+#endif
+}
+// Are the thresholds dep + k exact?  Below dep always (dep >= 8); above it
+// unless dep + k crosses into a binade that cannot hold it.
+GBR_HD bool ssao_exact(float dep) {
+  return dep >= 8.0f && (dep + 1.0f) - dep == 1.0f && (dep + 2.0f) - dep == 2.0f;
+}
+
+}  // namespace gbr

@@ -1,14 +1,15 @@
 // Checks the tile rasteriser's shortcuts (gbr_math.h) against what they stand
 // for: walk_first_late_row against walk_row_late over every width <= W, top
 // row < H and row (a row before it must not be late), and box_bounds against
-// depth_at and edge_inside at every pixel of random triangles' boxes.
+// depth_at and edge_inside at every pixel of random triangles' boxes; and
+// ssao_tap against ssao_count wherever ssao_exact holds.
 // Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <random>
 
-#include "gbr_math.h"
+#include "gbr_shade_math.h"
 
 using namespace gbr;
 
@@ -56,6 +57,34 @@ int main(int argc, char** argv) {
         if (d < lo || d > hi || (f && !edge_inside(e, (float)px, (float)py))) bad++;
       }
   }
+  long taps = 0, inexact = 0, wrong = 0;
+  for (int i = 0; i < n; i++) {
+    // distances over the whole range, every other one within 3 units of a power of two
+    float dep = powf(2.0f, uni(-1.0f, 18.42f));
+    if (i & 1) dep = exp2f((float)(3 + rng() % 16)) + uni(-3.0f, 3.0f);
+    const uint32_t d0 = f2u_sat(dep / kDepthFar * kMulInt);
+    dep = depth_to_dist(d0);
+    if (!ssao_exact(dep)) {
+      inexact++;
+      continue;
+    }
+    const float t[5] = {(dep + -2.0f) * kTwo32, (dep + -1.0f) * kTwo32, dep * kTwo32, (dep + 1.0f) * kTwo32,
+                        (dep + 2.0f) * kTwo32};
+    for (int k = 0; k < 40; k++) {
+      uint32_t d = rng();
+      if (k < 36) {  // at and around every threshold
+        const float at = t[k % 5] / kDepthFar;
+        d = f2u_sat(at) + (uint32_t)((int)(rng() % 5) - 2) * ((k & 8) ? 1u : 300u);
+      }
+      if (k == 36) d = 0;
+      if (k == 37) d = kDepthClear;
+      taps++;
+      wrong += ssao_tap(d, (2.0f - dep) * 0.125f) - kSsaoTapZero !=
+               (uint32_t)ssao_count(depth_scaled(d), t[0], t[1], t[2], t[3], t[4]);
+    }
+  }
+  printf("taps=%ld inexact=%ld wrong=%ld\n", taps, inexact, wrong);
+  bad += wrong;
   printf("early=%ld late=%ld boxes=%d full=%ld bounded=%ld bad=%ld\n", early, late, n, full, bounded, bad);
-  return early == 0 && late > 0 && bad == 0 && full > 0 && bounded > 0 ? 0 : 1;
+  return early == 0 && late > 0 && bad == 0 && taps > 0 && inexact > 0 && full > 0 && bounded > 0 ? 0 : 1;
 }
