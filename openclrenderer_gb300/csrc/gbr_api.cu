@@ -363,13 +363,13 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
 bool absorb_counters(gbr_scene* s, const Counters& c, WorkMem& w, float headroom, bool view) {
   if (!c.overflow) {
     if (view) {
-      s->stats.view_records = c.nrec;
-      s->stats.view_bin_entries = (uint64_t)c.fine_total + c.coarse_total;
+      s->stats.view_records = c.vis;
+      s->stats.view_bin_entries = c.bins;
       s->stats.fragments_ref = c.frag_ref;
       s->stats.view_samples = c.samples;
     } else {
-      s->stats.shadow_records = c.nrec;
-      s->stats.shadow_bin_entries = (uint64_t)c.fine_total + c.coarse_total;
+      s->stats.shadow_records = c.vis;
+      s->stats.shadow_bin_entries = c.bins;
       s->stats.shadow_samples = c.samples;
     }
     return true;
@@ -377,8 +377,8 @@ bool absorb_counters(gbr_scene* s, const Counters& c, WorkMem& w, float headroom
   s->stats.retries++;
   const double h = std::min(std::max((double)headroom, 1.05), 4.0);
   if (c.overflow & 1u)
-    w.rec_target = (uint32_t)std::min<double>((double)c.nrec * h + 1024.0, (double)0xFFFFFFF0u);
-  uint64_t need_bins = (uint64_t)c.fine_total + c.coarse_total;
+    w.rec_target = (uint32_t)std::min<double>((double)c.vis * h + 1024.0, (double)0xFFFFFFF0u);
+  uint64_t need_bins = c.bins;
   if (c.overflow & 1u) need_bins = std::max<uint64_t>(need_bins, (uint64_t)w.rec_target * 4);
   w.bin_target = (uint32_t)std::min<double>((double)need_bins * h + 4096.0, (double)0xFFFFFFF0u);
   return false;

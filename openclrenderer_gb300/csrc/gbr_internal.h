@@ -42,7 +42,7 @@ struct __align__(16) RasterRec {
   uint32_t xr;           // minx | maxx << 16
   uint32_t yr;           // miny | maxy << 16
   uint32_t surface;
-  uint32_t pad;
+  uint32_t tight;        // the box is tight_box's: one column and row less than bbox4
 };
 
 // Per visible clipped triangle of a view: kernel3's per-triangle constants,
@@ -111,9 +111,12 @@ struct ShadowJob {
 
 struct Counters {
   unsigned long long frag_ref;  // sum of ceil(area / chunk): the reference's work items
-  uint32_t nrec;                // records requested
+  uint32_t nrec;                // records stored (or asked for, after an overflow)
   uint32_t overflow;            // bit 0 records, bit 1 bins, bit 2 a bounded wait gave up (fused pass)
   uint32_t fine_total, coarse_total;
+  uint32_t ncoarse;             // records in coarse bins: their list runs down from the end of the bins
+  uint32_t vis;                 // visible triangles: the records, and those that cover no pixel
+  unsigned long long bins;      // tiles of the visible triangles' bbox4
   unsigned long long samples;   // covered pixel-samples (point_in_tri passes) of the depth pass
 };
 
@@ -122,7 +125,7 @@ struct SceneDev {
   uint32_t ntris;
   // world-space vertex positions, rot_quat(v * scale, q) + world_pos (the
   // first half of full_rotate_quat, cl2.cl:700-710); w of vertex 0 holds the
-  // object id.  3 per triangle.
+  // object id, w of vertex 1 the object's feature flags.  3 per triangle.
   const float4* world;
   // per object, kObjQuads float4: fast_normalize4(world_rot_quat), the
   // normalised inverse back_rot_quat applies (cl2.cl:350-370), and the

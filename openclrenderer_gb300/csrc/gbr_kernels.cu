@@ -21,28 +21,6 @@ __device__ __forceinline__ f4 ld4(const float* p) {
   return r;
 }
 
-// Warp-aggregated allocation of n slots from *counter; every lane of the
-// warp must call it (n may be 0).  Returns this lane's first slot.
-__device__ __forceinline__ uint32_t warp_alloc(uint32_t* counter, uint32_t n) {
-  const unsigned full = 0xFFFFFFFFu;
-  int lane = threadIdx.x & 31;
-  uint32_t incl = n;
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t v = __shfl_up_sync(full, incl, o);
-    if (lane >= o) incl += v;
-  }
-  uint32_t total = __shfl_sync(full, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(full, base, 31);
-  return base + incl - n;
-}
-
-__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-  return v;
-}
-
 // Warp-aggregated "atomicAdd(&counter[key], 1)": lanes with the same key
 // share one atomic.  Every lane of the warp must call it; inactive lanes pass
 // active = false.  Returns this lane's old value + its rank within its key.
@@ -61,11 +39,14 @@ __device__ __forceinline__ uint32_t agg_inc(uint32_t* counter, uint32_t key, boo
   return res;
 }
 
-// A visible clipped triangle before it becomes a record.
+// A visible clipped triangle before it becomes a record.  (The second
+// triangle of a split at the near clip, which is rare, is made after the first
+// one is done with, so that only one is held at a time.)
 struct Cand {
   f3 p[3];
-  float rc;
-  float mm[4];
+  float mm[4];  // bbox4, or the smaller box of tight_box
+  float area;   // of bbox4
+  int box;      // tight_box
   uint32_t key;
 };
 
@@ -81,18 +62,21 @@ __device__ __forceinline__ bool cull_candidate(Cand& c, bool two_sided, float w,
   if (!valid || cond) return false;
   f3 xpv = mk3(roundf(p[0].x), roundf(p[1].x), roundf(p[2].x));
   f3 ypv = mk3(roundf(p[0].y), roundf(p[1].y), roundf(p[2].y));
-  c.rc = rconstant(xpv, ypv);
   bbox4(p[0], p[1], p[2], w, h, c.mm);
-  return (c.mm[1] - c.mm[0]) * (c.mm[3] - c.mm[2]) > 0.0f;
+  c.area = (c.mm[1] - c.mm[0]) * (c.mm[3] - c.mm[2]);
+  c.box = tight_box(xpv, ypv, w, h, c.mm);
+  return c.area > 0.0f;
 }
 
-__device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, RasterRec& R) {
+// rc: rconstant of the rounded vertices, which kernel3's plane reads too
+__device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, RasterRec& R, float* rc) {
   const f3* p = c.p;
   f3 xpv = mk3(roundf(p[0].x), roundf(p[1].x), roundf(p[2].x));
   f3 ypv = mk3(roundf(p[0].y), roundf(p[1].y), roundf(p[2].y));
   f3 depths = mk3(rcp(fdiv(p[0].z, kDepthFar)), rcp(fdiv(p[1].z, kDepthFar)),
                   rcp(fdiv(p[2].z, kDepthFar)));
-  plane_const(depths, xpv, ypv, c.rc, &R.A, &R.B, &R.C);
+  *rc = rconstant(xpv, ypv);
+  plane_const(depths, xpv, ypv, *rc, &R.A, &R.B, &R.C);
   EdgeTest e = make_edge(xpv.x, ypv.x, xpv.y, ypv.y, xpv.z, ypv.z);
   R.s0 = e.s0; R.sa = e.sa; R.sb = e.sb; R.sign = e.sign;
   R.t0 = e.t0; R.ta = e.ta; R.tb = e.tb; R.bound = e.bound;
@@ -100,7 +84,7 @@ __device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, Raster
   R.xr = (uint32_t)c.mm[0] | ((uint32_t)c.mm[1] << 16);
   R.yr = (uint32_t)c.mm[2] | ((uint32_t)c.mm[3] << 16);
   R.surface = surface;
-  R.pad = 0;
+  R.tight = c.box == kBoxTight ? 1u : 0u;
 }
 
 __device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& R) {
@@ -108,35 +92,115 @@ __device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& R) {
   d[0] = make_float4(R.A, R.B, R.C, R.bound);
   d[1] = make_float4(R.s0, R.sa, R.sb, R.sign);
   d[2] = make_float4(R.t0, R.ta, R.tb, __uint_as_float(R.key));
-  d[3] = make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), __uint_as_float(R.surface), 0.0f);
+  d[3] = make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), __uint_as_float(R.surface),
+                     __uint_as_float(R.tight));
 }
 
-// Tile footprint of a bbox [minx,maxx) x [miny,maxy).
+// Tile footprint of a record: inclusive fine tiles, or coarse tiles when its
+// bbox4 touches more than ws.fine_max fine tiles (tiles of kTile <<
+// ws.coarse_shift pixels).  A tight box counts and places only the tiles it
+// touches itself; *ref is the number of tiles of the bbox4, what a scratch
+// limit is measured against.
 struct Foot {
-  int tx0, tx1, ty0, ty1;  // inclusive fine tiles
+  int tx0, tx1, ty0, ty1;
   bool coarse;
 };
 __device__ __forceinline__ int foot_count(const Foot& f) { return (f.tx1 - f.tx0 + 1) * (f.ty1 - f.ty0 + 1); }
-// Global tile index (fine or coarse counter array) of the k-th tile of a footprint.
-__device__ __forceinline__ uint32_t foot_tile(const Foot& f, int k, const Surface& S) {
-  const int w = f.tx1 - f.tx0 + 1;
-  const int ty = f.ty0 + k / w, tx = f.tx0 + k % w;
-  return f.coarse ? S.ctile_base + ty * S.ctiles_x + tx : S.tile_base + ty * S.tiles_x + tx;
-}
-// Records touching more than ws.fine_max fine tiles go to the coarse bins
-// (tiles of kTile << ws.coarse_shift pixels).
-__device__ __forceinline__ Foot footprint(uint32_t xr, uint32_t yr, const Workspace& ws) {
+__device__ __forceinline__ Foot footprint(uint32_t xr, uint32_t yr, uint32_t tight, const Workspace& ws, int* ref) {
+  const int minx = xr & 0xFFFF, maxx = xr >> 16, miny = yr & 0xFFFF, maxy = yr >> 16;
+  int bx0 = (minx - (int)tight) >> 4, by0 = max(miny - (int)tight, 0) >> 4;  // tight: minx >= 1
   Foot f;
-  int minx = xr & 0xFFFF, maxx = xr >> 16, miny = yr & 0xFFFF, maxy = yr >> 16;
-  f.tx0 = minx / kTile; f.tx1 = (maxx - 1) / kTile;
-  f.ty0 = miny / kTile; f.ty1 = (maxy - 1) / kTile;
-  f.coarse = (f.tx1 - f.tx0 + 1) * (f.ty1 - f.ty0 + 1) > ws.fine_max;
-  if (f.coarse) {
-    const int sh = ws.coarse_shift;
-    f.tx0 >>= sh; f.tx1 >>= sh;
-    f.ty0 >>= sh; f.ty1 >>= sh;
-  }
+  f.tx0 = minx >> 4; f.tx1 = (maxx - 1) >> 4;
+  f.ty0 = miny >> 4; f.ty1 = (maxy - 1) >> 4;
+  f.coarse = (f.tx1 - bx0 + 1) * (f.ty1 - by0 + 1) > ws.fine_max;
+  const int sh = f.coarse ? ws.coarse_shift : 0;
+  f.tx0 >>= sh; f.tx1 >>= sh; bx0 >>= sh;
+  f.ty0 >>= sh; f.ty1 >>= sh; by0 >>= sh;
+  *ref = (f.tx1 - bx0 + 1) * (f.ty1 - by0 + 1);
   return f;
+}
+static_assert(kTile == 16, "footprint shifts by 4");
+// The tiles of a footprint one after another, as indices into the fine or
+// coarse counters.
+struct FootWalk {
+  int tx, ty;
+  __device__ __forceinline__ FootWalk(const Foot& f) : tx(f.tx0), ty(f.ty0) {}
+  __device__ __forceinline__ uint32_t fine(const Surface& S) const { return S.tile_base + ty * S.tiles_x + tx; }
+  __device__ __forceinline__ void next(const Foot& f) {
+    if (++tx > f.tx1) {
+      tx = f.tx0;
+      ty++;
+    }
+  }
+};
+// Calls go(record, fine tile) for every (record, fine tile) pair of a warp's
+// lanes, each with a record r and `mine' tiles (0: none).  Footprints of up to
+// kLockstep tiles go lane by lane in lockstep, so that neighbouring triangles,
+// which usually share tiles, can share an atomic (agg: go_agg(tile, on) for all
+// lanes); larger ones are laid end to end and dealt out to the lanes, 32 pairs
+// at a time (a lane walking its own 16 tiles is a chain of 16 atomics).
+constexpr int kLockstep = 4;
+template <class GoAgg, class Go>
+__device__ __forceinline__ void each_fine_tile(const Foot& f, int mine, const Surface* S, uint32_t r, GoAgg go_agg,
+                                               Go go) {
+  constexpr unsigned full = 0xFFFFFFFFu;
+  const bool big = mine > kLockstep;
+  const int most = (int)__reduce_max_sync(full, big ? 0u : (uint32_t)mine);
+  FootWalk walk(f);
+  for (int it = 0; it < most; it++) {
+    const bool on = !big && it < mine;
+    go_agg(on ? walk.fine(*S) : 0u, on);
+    walk.next(f);
+  }
+  if (!__any_sync(full, big)) return;
+  const int lane = threadIdx.x & 31;
+  int start = big ? mine : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(full, start, o);
+    if (lane >= o) start += v;
+  }
+  const int total = __shfl_sync(full, start, 31);
+  start -= big ? mine : 0;  // exclusive
+  const int w = f.tx1 - f.tx0 + 1, row = big ? S->tiles_x : 0;
+  const uint32_t base = big ? S->tile_base + f.ty0 * row + f.tx0 : 0u;
+#pragma unroll 2
+  for (int t0 = 0; t0 < total; t0 += 32) {
+    const int t = t0 + lane;
+    int src = 0;  // the last lane whose pairs start at or before t
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(full, start, src + o) <= t) src += o;
+    const int k = t - __shfl_sync(full, start, src), sw = __shfl_sync(full, w, src), srow = __shfl_sync(full, row, src);
+    const uint32_t sbase = __shfl_sync(full, base, src), sr = __shfl_sync(full, r, src);
+    if (t < total) {
+      const int ky = k / sw;
+      go(sr, sbase + (uint32_t)(ky * srow + (k - ky * sw)));
+    }
+  }
+}
+// Calls go(lane's record index, coarse tile) for every (record, coarse tile)
+// pair of the lanes that have a coarse footprint: the warp takes one record
+// after another, its lanes the tiles.  (A lane looping over its own record's
+// tiles, 240 at 2560x1440, made the setup and the fill wait for the few warps
+// of large records.)  Every lane of the warp calls it.
+template <class Go>
+__device__ __forceinline__ void each_coarse_tile(const Foot& f, bool coarse, const Surface* S, uint32_t r, Go go) {
+  for (unsigned todo = __ballot_sync(0xFFFFFFFFu, coarse); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const int tx0 = __shfl_sync(0xFFFFFFFFu, f.tx0, src), w = __shfl_sync(0xFFFFFFFFu, f.tx1, src) - tx0 + 1;
+    const int ty0 = __shfl_sync(0xFFFFFFFFu, f.ty0, src), h = __shfl_sync(0xFFFFFFFFu, f.ty1, src) - ty0 + 1;
+    const uint32_t row = (uint32_t)__shfl_sync(0xFFFFFFFFu, coarse ? S->ctiles_x : 0, src);
+    const uint32_t base = __shfl_sync(0xFFFFFFFFu, coarse ? S->ctile_base : 0u, src) + ty0 * row + tx0;
+    const uint32_t rr = __shfl_sync(0xFFFFFFFFu, r, src);
+    // k / w as a product: exact while k * w < 2^20 (w <= 60, h <= 34: 64-pixel tiles of 3840x2160)
+    const uint32_t inv = ((1u << 20) + (uint32_t)w - 1u) / (uint32_t)w;
+#pragma unroll 1
+    for (int k = threadIdx.x & 31; k < w * h; k += 32) {
+      const uint32_t ky = ((uint32_t)k * inv) >> 20;
+      go(rr, base + ky * row + ((uint32_t)k - ky * (uint32_t)w));
+    }
+  }
 }
 
 // point_in_tri of a record at pixel (px, py).
@@ -180,20 +244,19 @@ __device__ __forceinline__ uint32_t walk_skip_rows(uint32_t xr, uint32_t yr, int
   return bits;
 }
 
-// One candidate as a record (and shade record for views); returns its tile footprint.
-__device__ __forceinline__ int write_rec(const Cand& c, uint32_t r, uint32_t surface, const Workspace& ws, bool view,
-                                         Foot* foot) {
+// One candidate as a record (and shade record for views).
+__device__ __forceinline__ void write_rec(const Cand& c, uint32_t r, uint32_t surface, const Workspace& ws,
+                                          bool view) {
   RasterRec R;
-  make_rec(c, surface, R);
+  float rc;
+  make_rec(c, surface, R, &rc);
   store_rec(ws.rec + r, R);
   if (view) {  // what prep_shade needs (the fill turns it into the shade constants)
     uint32_t tri = c.key >> 1;
-    ws.srec[r].a = make_float4(c.p[0].x, c.p[0].y, c.p[0].z, c.rc);
+    ws.srec[r].a = make_float4(c.p[0].x, c.p[0].y, c.p[0].z, rc);
     ws.srec[r].e0 = make_float4(c.p[1].x, c.p[1].y, c.p[1].z, __uint_as_float(tri));
     ws.srec[r].e1 = make_float4(c.p[2].x, c.p[2].y, c.p[2].z, 0.0f);
   }
-  *foot = footprint(R.xr, R.yr, ws);
-  return foot_count(*foot);
 }
 
 // Depth-only passes (cube faces): a candidate whose bbox has at most this
@@ -202,15 +265,12 @@ __device__ __forceinline__ int write_rec(const Cand& c, uint32_t r, uint32_t sur
 // and a minimum does not depend on order -- instead of becoming a record.
 constexpr float kDirectArea = 64.0f;
 
-__device__ __forceinline__ bool direct_cand(const Cand& c) {
-  return (c.mm[1] - c.mm[0]) * (c.mm[3] - c.mm[2]) <= kDirectArea;
-}
-
 // kernel1 of one small candidate into its surface's depth; returns the
 // covered pixel count.
-__device__ __noinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, const Surface& S) {
+__device__ __forceinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, const Surface& S) {
   RasterRec R;
-  make_rec(c, surface, R);
+  float rc;
+  make_rec(c, surface, R, &rc);
   const float4 q[4] = {make_float4(R.A, R.B, R.C, R.bound), make_float4(R.s0, R.sa, R.sb, R.sign),
                        make_float4(R.t0, R.ta, R.tb, __uint_as_float(R.key)),
                        make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), 0.0f, 0.0f)};
@@ -219,8 +279,10 @@ __device__ __noinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, 
   // row by row: the walk rule of the row's left-column pixel, then point_in_tri
   // (walk_skip_rows: 0 at once unless the bbox touches the top of the face;
   // a bbox of at most 64 pixels has at most 64 rows)
-  const uint64_t skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, S.chunk) |
-                        ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, S.chunk) << 32);
+  uint64_t skip = 0;
+  if (!R.tight)
+    skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, S.chunk) |
+           ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, S.chunk) << 32);
   for (int y = y0; y < y1; y++) {
     for (int x = x0 + (int)((skip >> (y - y0)) & 1u); x < x1; x++)
       if (rec_in_tri(q, x, y)) {
@@ -231,58 +293,92 @@ __device__ __noinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, 
   return hits;
 }
 
-// Append this lane's candidates (n = 0, 1 or 2: c0, then c1) as records and
-// count their bins (depth-only passes rasterise small ones directly).  Every
-// lane of the warp must call it.  Returns this lane's reference fragment count
-// (sum of ceil(area / chunk)).
-__device__ unsigned long long emit(const Cand& c0, const Cand& c1, int n, uint32_t surface, const Surface* surfs,
-                                   const Workspace& ws, bool view) {
-  const bool d0 = !view && n > 0 && direct_cand(c0), d1 = !view && n > 1 && direct_cand(c1);
-  const uint32_t nr = (uint32_t)(n > 0 && !d0) + (uint32_t)(n > 1 && !d1);
-  const uint32_t base = warp_alloc(&ws.ctr->nrec, nr);
-  unsigned long long frags = 0;
-  const Surface& S = surfs[surface];
-  Foot f0{0, 0, 0, 0, false}, f1{0, 0, 0, 0, false};
-  int n0 = 0, n1 = 0;
-  uint32_t slot = base, hits = 0;
-  if (n > 0) {
-    frags += (unsigned long long)ceilf(fdiv((c0.mm[1] - c0.mm[0]) * (c0.mm[3] - c0.mm[2]), (float)S.chunk));
-    if (d0) hits += direct_raster(c0, surface, S);
-    else if (slot < ws.rec_cap) n0 = write_rec(c0, slot++, surface, ws, view, &f0);
-    else atomicOr(&ws.ctr->overflow, 1u);
+// What the setup threads of a block add up before it reaches the pass's
+// counters: one global atomic per counter and block instead of one per warp.
+struct SetupSums {
+  unsigned long long frags;
+  uint32_t bins, vis, samples, warps;
+  __device__ __forceinline__ void clear() {
+    frags = 0;
+    bins = vis = samples = warps = 0;
   }
-  if (n > 1) {
-    frags += (unsigned long long)ceilf(fdiv((c1.mm[1] - c1.mm[0]) * (c1.mm[3] - c1.mm[2]), (float)S.chunk));
-    if (d1) hits += direct_raster(c1, surface, S);
-    else if (slot < ws.rec_cap) n1 = write_rec(c1, slot++, surface, ws, view, &f1);
-    else atomicOr(&ws.ctr->overflow, 1u);
-  }
-  if (!view) {
-    hits = __reduce_add_sync(0xFFFFFFFFu, hits);
-    if ((threadIdx.x & 31) == 0 && hits) atomicAdd(&ws.ctr->samples, (unsigned long long)hits);
-  }
-  // tile counts, aggregated across the warp (neighbouring triangles usually
-  // share tiles): iterate over this lane's (record, tile) pairs in lockstep
-  const int total = n0 + n1;
-  int maxt = total;
-  for (int o = 16; o > 0; o >>= 1) maxt = max(maxt, __shfl_xor_sync(0xFFFFFFFFu, maxt, o));
-  for (int it = 0; it < maxt; it++) {
-    const bool act = it < total;
-    const bool second = it >= n0;
-    const Foot& f = second ? f1 : f0;
-    const int k = second ? it - n0 : it;
-    const bool coarse = act && f.coarse;
-    const uint32_t tile = act ? foot_tile(f, k, S) : 0u;
-    // fine and coarse counters live in different arrays: aggregate them separately
-    agg_inc(ws.fine_count, tile, act && !coarse);
-    agg_inc(ws.coarse_count, tile, act && coarse);
-  }
-  return frags;
+};
+struct SetupCounts {
+  uint32_t frags = 0, bins = 0, vis = 0, samples = 0;  // of this lane
+};
+// Adds the lanes' counts to the block's.  (A lane's fragments of up to 12
+// triangles: below 2^18.)
+__device__ __forceinline__ void setup_add(SetupSums* b, const SetupCounts& c) {
+  const uint32_t frags = __reduce_add_sync(0xFFFFFFFFu, c.frags), bins = __reduce_add_sync(0xFFFFFFFFu, c.bins);
+  const uint32_t vis = __reduce_add_sync(0xFFFFFFFFu, c.vis), samples = __reduce_add_sync(0xFFFFFFFFu, c.samples);
+  if ((threadIdx.x & 31) != 0) return;
+  if (frags) atomicAdd(&b->frags, (unsigned long long)frags);
+  if (bins) atomicAdd(&b->bins, bins);
+  if (vis) atomicAdd(&b->vis, vis);
+  if (samples) atomicAdd(&b->samples, samples);
+}
+// Every warp of the block calls it once, when it is done; the last one writes
+// the block's sums.
+__device__ __forceinline__ void setup_done(SetupSums* b, const Workspace& ws) {
+  if ((threadIdx.x & 31) != 0) return;
+  __threadfence_block();
+  if (atomicAdd(&b->warps, 1u) + 1u != blockDim.x / 32) return;
+  __threadfence_block();
+  volatile SetupSums* v = b;
+  if (v->frags) atomicAdd(&ws.ctr->frag_ref, (unsigned long long)v->frags);
+  if (v->bins) atomicAdd(&ws.ctr->bins, (unsigned long long)v->bins);
+  if (v->vis) atomicAdd(&ws.ctr->vis, (uint32_t)v->vis);
+  if (v->samples) atomicAdd(&ws.ctr->samples, (unsigned long long)v->samples);
 }
 
-__device__ __forceinline__ void add_frags(const Workspace& ws, unsigned long long frags) {
-  frags = warp_sum_u64(frags);
-  if ((threadIdx.x & 31) == 0 && frags) atomicAdd(&ws.ctr->frag_ref, frags);
+// Append this lane's candidate (act: it has one) as a record and count its
+// bins (depth-only passes rasterise small ones directly).  A candidate without
+// a pixel (kBoxEmpty) is counted as visible, but not stored.  Every lane of
+// the warp must call it.
+template <bool VIEW>
+__device__ __forceinline__ void emit(const Cand& c, bool act, uint32_t surface, const Surface& S, const Workspace& ws,
+                                     SetupCounts& cnt) {
+  constexpr unsigned full = 0xFFFFFFFFu;
+  const bool direct = !VIEW && act && c.area <= kDirectArea, rec = act && !direct;
+  if (act) {  // ceil(area / chunk)
+    const float chunk = (float)S.chunk;
+    cnt.frags += c.area <= chunk ? 1u : (uint32_t)ceilf(fdiv(c.area, chunk));
+  }
+  if (direct && c.box != kBoxEmpty) cnt.samples += direct_raster(c, surface, S);
+  if (!__any_sync(full, rec)) return;
+  const bool store = rec && c.box != kBoxEmpty;
+  Foot f{0, -1, 0, -1, false};
+  if (rec) {
+    int ref;
+    f = footprint((uint32_t)c.mm[0] | ((uint32_t)c.mm[1] << 16), (uint32_t)c.mm[2] | ((uint32_t)c.mm[3] << 16),
+                  c.box != kBoxAny ? 1u : 0u, ws, &ref);
+    cnt.vis++;
+    cnt.bins += (uint32_t)ref;
+  }
+  const unsigned who = __ballot_sync(full, store);
+  const int lane = threadIdx.x & 31;
+  uint32_t slot = 0;
+  if (lane == 0 && who) slot = atomicAdd(&ws.ctr->nrec, (uint32_t)__popc(who));
+  slot = __shfl_sync(full, slot, 0) + (uint32_t)__popc(who & ((1u << lane) - 1u));
+  const bool stored = store && slot < ws.rec_cap;
+  if (stored)
+    write_rec(c, slot, surface, ws, VIEW);
+  else if (store)
+    atomicOr(&ws.ctr->overflow, 1u);
+  // tile counts
+  each_fine_tile(f, stored && !f.coarse ? foot_count(f) : 0, &S, slot,
+                 [&](uint32_t tile, bool on) { agg_inc(ws.fine_count, tile, on); },
+                 [&](uint32_t, uint32_t tile) { atomicAdd(&ws.fine_count[tile], 1u); });
+  const bool coarse = stored && f.coarse;
+  each_coarse_tile(f, coarse, &S, slot, [&](uint32_t, uint32_t tile) { atomicAdd(&ws.coarse_count[tile], 1u); });
+  // the list of coarse records, from the end of the bins down (k_fill)
+  const unsigned listed = __ballot_sync(full, coarse);
+  if (listed) {
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&ws.ctr->ncoarse, (uint32_t)__popc(listed));
+    at = __shfl_sync(full, at, 0) + (uint32_t)__popc(listed & ((1u << lane) - 1u));
+    if (coarse && at < ws.bin_cap) ws.bins[ws.bin_cap - 1 - at] = slot;
+  }
 }
 
 __device__ __forceinline__ void load_tri_pos(const gbr_triangle* T, f3 v[3], uint32_t* o_id) {
@@ -317,11 +413,12 @@ __global__ void __launch_bounds__(256) k_world(SceneDev sc, float4* __restrict__
     const f4 qn = fast_normalize4(ld4(G->world_rot_quat));
     const f3 wp = ld3(G->world_pos);
     const float scale = __ldg(&G->scale);
+    const int flags = __ldg(&G->feature_flag);
     float4* out = world + (size_t)tri * 3;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       f3 r = add3(rot_quat_n(mul3s(v[k], scale), qn), wp);
-      out[k] = make_float4(r.x, r.y, r.z, k == 0 ? __uint_as_float(o_id) : 0.0f);
+      out[k] = make_float4(r.x, r.y, r.z, k == 0 ? __uint_as_float(o_id) : k == 1 ? __int_as_float(flags) : 0.0f);
       const float d = fast_length3(sub3(r, wp));
       rmax = d == d ? fmax_(rmax, d) : __int_as_float(0x7F800000);  // a NaN vertex disables the cull
     }
@@ -424,9 +521,10 @@ __global__ void __launch_bounds__(256) k_texture_levels(const uint32_t* __restri
   texlv[i] = make_float4((float)(col * w), (float)(row * w), (float)w, __uint_as_float(page));
 }
 
-// World-space vertices of a triangle: from the scene's cache when there is
-// one, else computed here with the same arithmetic as k_world.
-__device__ __forceinline__ void load_world(const SceneDev& sc, uint32_t tri, f3 w[3], uint32_t* o_id) {
+// World-space vertices of a triangle, its object and the object's feature
+// flags: from the scene's cache when there is one, else computed here with the
+// same arithmetic as k_world.
+__device__ __forceinline__ void load_world(const SceneDev& sc, uint32_t tri, f3 w[3], uint32_t* o_id, int* flags) {
   if (!sc.world) {
     f3 v[3];
     load_tri_pos(sc.tris + tri, v, o_id);
@@ -434,6 +532,7 @@ __device__ __forceinline__ void load_world(const SceneDev& sc, uint32_t tri, f3 
     const f4 qn = fast_normalize4(ld4(G->world_rot_quat));
     const f3 wp = ld3(G->world_pos);
     const float scale = __ldg(&G->scale);
+    *flags = __ldg(&G->feature_flag);
 #pragma unroll
     for (int k = 0; k < 3; k++) w[k] = add3(rot_quat_n(mul3s(v[k], scale), qn), wp);
     return;
@@ -444,85 +543,116 @@ __device__ __forceinline__ void load_world(const SceneDev& sc, uint32_t tri, f3 
   w[1] = mk3(b.x, b.y, b.z);
   w[2] = mk3(c.x, c.y, c.z);
   *o_id = __float_as_uint(a.w);
+  *flags = __float_as_int(b.w);
 }
 
 // The camera half of full_rotate_quat (cl2.cl:700-729): world -> camera
-// space, near/far clip, projection.
+// space, near/far clip, projection of clip output k (0 or 1).  Returns the
+// number of clip outputs; o is only written for k below it.
 __device__ __forceinline__ int transform_clip(const f3 w[3], f3 cpos, f3 c, f3 s, float fov, float width,
-                                              float height, f3 o0[3], f3 o1[3]) {
+                                              float height, int k, f3 o[3]) {
   f3 t0[3], t1[3];
   const int n = clip_tri_reg(rot_cs(w[0], cpos, c, s), rot_cs(w[1], cpos, c, s), rot_cs(w[2], cpos, c, s), t0, t1);
-  if (n > 0) {
+  if (k < n) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) o0[k] = depth_project1(t0[k], width, height, fov);
-  }
-  if (n > 1) {  // only a triangle with one vertex behind the near plane splits
-#pragma unroll
-    for (int k = 0; k < 3; k++) o1[k] = depth_project1(t1[k], width, height, fov);
+    for (int j = 0; j < 3; j++) o[j] = depth_project1(k ? t1[j] : t0[j], width, height, fov);
   }
   return n;
 }
 
-// prearrange's handling of one (triangle, surface): up to two clip outputs,
-// culled, as candidates c0 (first survivor) and c1.
-__device__ __forceinline__ int make_cands(const f3 w[3], f3 cpos, f3 c, f3 s, float fov, float width, float height,
-                                          bool two, uint32_t tri, Cand& c0, Cand& c1) {
-  f3 o0[3], o1[3];
-  const int num = transform_clip(w, cpos, c, s, fov, width, height, o0, o1);
-  int n = 0;
-  if (num > 0) {
-    c0.p[0] = o0[0]; c0.p[1] = o0[1]; c0.p[2] = o0[2];
-    c0.key = tri * 2u;
-    if (cull_candidate(c0, two, width, height)) n = 1;
+// prearrange's handling of clip output k of one (triangle, surface): *num is
+// the number of clip outputs; returns whether output k survives the culls.
+__device__ __forceinline__ bool make_cand(const f3 w[3], f3 cpos, f3 c, f3 s, float fov, float width, float height,
+                                          bool two, uint32_t tri, int k, Cand& out, int* num) {
+  *num = transform_clip(w, cpos, c, s, fov, width, height, k, out.p);
+  out.key = tri * 2u + (uint32_t)k;
+  return k < *num && cull_candidate(out, two, width, height);
+}
+
+// The second clip outputs of a warp's triangles (has: the lane has one), from
+// their vertices again: a near-clip split is rare, and the common path keeps
+// no registers for it.  Every lane of the warp must call it.
+template <bool VIEW>
+__device__ __noinline__ void emit_second(const SceneDev& sc, const Workspace& ws, uint32_t tri, bool has, f3 pos, f3 c,
+                                         f3 s, float fov, uint32_t surface, const Surface* surfs, SetupSums* sums) {
+  const Surface& S = surfs[surface];
+  Cand cand;
+  bool act = false;
+  if (has) {
+    f3 wv[3];
+    uint32_t o_id;
+    int num, flags;
+    load_world(sc, tri, wv, &o_id, &flags);
+    act = make_cand(wv, pos, c, s, fov, (float)S.width, (float)S.height, (flags & kFlagTwoSided) > 0, tri, 1, cand,
+                    &num);
   }
-  if (num > 1) {
-    Cand& d = n ? c1 : c0;
-    d.p[0] = o1[0]; d.p[1] = o1[1]; d.p[2] = o1[2];
-    d.key = tri * 2u + 1u;
-    if (cull_candidate(d, two, width, height)) n++;
-  }
-  return n;
+  SetupCounts cnt;
+  emit<VIEW>(cand, act, surface, S, ws, cnt);
+  setup_add(sums, cnt);
 }
 
 // prearrange (cl2.cl:4271-4409), one thread per (triangle, view).
-__global__ void __launch_bounds__(256) k_setup_views(SceneDev sc, const ViewParams* __restrict__ views,
-                                                     const Surface* __restrict__ surfs, Workspace ws) {
+__global__ void __launch_bounds__(256, 5) k_setup_views(const __grid_constant__ SceneDev sc,
+                                                     const ViewParams* __restrict__ views,
+                                                     const Surface* __restrict__ surfs,
+                                                     const __grid_constant__ Workspace ws) {
+  __shared__ SetupSums sums;
+  if (threadIdx.x == 0) sums.clear();
+  __syncthreads();
   uint32_t tri = blockIdx.x * blockDim.x + threadIdx.x;
   const ViewParams& V = views[blockIdx.y];
   const Surface& S = surfs[V.surface];
-  Cand c0, c1;
-  int n = 0;
-  // the object cull (k_object_cull), when the pass has one: the object id
-  // alone decides
+  SetupCounts cnt;
+  // the object cull (k_object_cull), when the pass has one, includes the
+  // reference's own object test.  A pass of one view reads the whole triangle
+  // at once (two rounds of loads); a pass of many views, which skips most
+  // objects in each, reads the object id alone first.
   bool live = tri < sc.ntris;
+  f3 wv[3];
+  uint32_t o_id = 0;
+  int flags = 0;
+  const f3 cpos = mk3(V.cpos[0], V.cpos[1], V.cpos[2]);
+  const bool whole = gridDim.y == 1;
+  if (live && (whole || !ws.vis)) load_world(sc, tri, wv, &o_id, &flags);
   if (live && ws.vis) {
-    const uint32_t o_id = __float_as_uint(__ldg(&sc.world[(size_t)tri * 3].w));
+    if (!whole) o_id = __float_as_uint(__ldg(&sc.world[(size_t)tri * 3].w));
     live = (__ldg(ws.vis + (size_t)blockIdx.y * ws.vis_words + (o_id >> 5)) >> (o_id & 31)) & 1u;
+  } else if (live) {
+    live = !(fast_length3(sub3(ld3(sc.descs[o_id].world_pos), cpos)) > kDepthFar);
   }
   // a warp with nothing to set up (objects are mostly contiguous runs of
   // triangles) leaves before emit's warp-wide work
-  if (!__any_sync(0xFFFFFFFFu, live)) return;
-  if (live) {
-    f3 wv[3];
-    uint32_t o_id;
-    load_world(sc, tri, wv, &o_id);
-    const gbr_obj_g_descriptor* G = sc.descs + o_id;
-    f3 cpos = mk3(V.cpos[0], V.cpos[1], V.cpos[2]);
-    if (!(fast_length3(sub3(ld3(G->world_pos), cpos)) > kDepthFar)) {
-      f3 c = mk3(V.ccos[0], V.ccos[1], V.ccos[2]);
-      f3 s = mk3(V.csin[0], V.csin[1], V.csin[2]);
-      const bool two = (__ldg(&G->feature_flag) & kFlagTwoSided) > 0;
-      n = make_cands(wv, cpos, c, s, V.fov, (float)S.width, (float)S.height, two, tri, c0, c1);
-    }
+  if (!__any_sync(0xFFFFFFFFu, live)) {
+    setup_done(&sums, ws);
+    return;
   }
-  add_frags(ws, emit(c0, c1, n, V.surface, surfs, ws, true));
+  Cand cand;
+  int num = 0;
+  bool act = false;
+  const f3 c = mk3(V.ccos[0], V.ccos[1], V.ccos[2]), s = mk3(V.csin[0], V.csin[1], V.csin[2]);
+  if (live) {
+    if (!whole && ws.vis) load_world(sc, tri, wv, &o_id, &flags);
+    act = make_cand(wv, cpos, c, s, V.fov, (float)S.width, (float)S.height, (flags & kFlagTwoSided) > 0, tri, 0, cand,
+                    &num);
+  }
+  emit<true>(cand, act, V.surface, S, ws, cnt);
+  if (__any_sync(0xFFFFFFFFu, num > 1))
+    emit_second<true>(sc, ws, tri, num > 1, cpos, c, s, V.fov, V.surface, surfs, &sums);
+  setup_add(&sums, cnt);
+  setup_done(&sums, ws);
 }
 
 // prearrange_realtime_shadowing (cl2.cl:4419-4636), one thread per (triangle, light job).
-__global__ void __launch_bounds__(128, 6) k_setup_shadow(SceneDev sc, const ShadowJob* __restrict__ jobs,
-                                                      const Surface* __restrict__ surfs, Workspace ws) {
+__global__ void __launch_bounds__(128, 7) k_setup_shadow(const __grid_constant__ SceneDev sc,
+                                                      const ShadowJob* __restrict__ jobs,
+                                                      const Surface* __restrict__ surfs,
+                                                      const __grid_constant__ Workspace ws) {
+  __shared__ SetupSums sums;
+  if (threadIdx.x == 0) sums.clear();
+  __syncthreads();
   uint32_t tri = blockIdx.x * blockDim.x + threadIdx.x;
   const ShadowJob& J = jobs[blockIdx.y];
+  SetupCounts cnt;
   const float L = (float)kLightBufferDim;
   int mask = 0;
   f3 wv[3];
@@ -530,29 +660,30 @@ __global__ void __launch_bounds__(128, 6) k_setup_shadow(SceneDev sc, const Shad
   bool two = false;
   if (tri < sc.ntris) {
     uint32_t o_id;
-    load_world(sc, tri, wv, &o_id);
-    const gbr_obj_g_descriptor* G = sc.descs + o_id;
-    int ff = __ldg(&G->feature_flag);
+    int ff;
+    load_world(sc, tri, wv, &o_id, &ff);
     bool is_static = (ff & kFlagIsStatic) > 0;
     two = (ff & kFlagTwoSided) > 0;
-    f3 wp = ld3(G->world_pos);
+    f3 wp = ld3(sc.descs[o_id].world_pos);
     if (is_static == (J.only_static != 0) && !(fast_length3(sub3(wp, lpos)) > kDepthFar)) {
       for (int k = 0; k < 3; k++) mask |= 1 << ret_cubeface(wv[k], lpos);
     }
   }
-  unsigned long long frags = 0;
   for (int face = 0; face < 6; face++) {
     if (!__any_sync(0xFFFFFFFFu, mask & (1 << face))) continue;  // warp-uniform
-    Cand c0, c1;
-    int n = 0;
-    if (mask & (1 << face)) {
-      f3 c = mk3(sc.face_cos[face][0], sc.face_cos[face][1], sc.face_cos[face][2]);
-      f3 s = mk3(sc.face_sin[face][0], sc.face_sin[face][1], sc.face_sin[face][2]);
-      n = make_cands(wv, lpos, c, s, kLFov, L, L, two, tri, c0, c1);
-    }
-    frags += emit(c0, c1, n, J.surface_base + face, surfs, ws, false);
+    const f3 c = mk3(sc.face_cos[face][0], sc.face_cos[face][1], sc.face_cos[face][2]);
+    const f3 s = mk3(sc.face_sin[face][0], sc.face_sin[face][1], sc.face_sin[face][2]);
+    const uint32_t surface = J.surface_base + face;
+    Cand cand;
+    int num = 0;
+    bool act = false;
+    if (mask & (1 << face)) act = make_cand(wv, lpos, c, s, kLFov, L, L, two, tri, 0, cand, &num);
+    emit<false>(cand, act, surface, surfs[surface], ws, cnt);
+    if (__any_sync(0xFFFFFFFFu, num > 1))
+      emit_second<false>(sc, ws, tri, num > 1, lpos, c, s, kLFov, surface, surfs, &sums);
   }
-  add_frags(ws, frags);
+  setup_add(&sums, cnt);
+  setup_done(&sums, ws);
 }
 
 // Each fine tile's surface (binary search over tile_base) and global coarse
@@ -636,6 +767,13 @@ __device__ void block_scan_array(uint32_t* count, uint32_t* off, uint32_t n, uin
   if (threadIdx.x == 0) *total = carry;
 }
 
+// The pass's scratch must hold every visible triangle and every tile of its
+// bbox4 (the limits callers know), although fewer are stored.
+__device__ __forceinline__ void check_scratch(const Workspace& ws) {
+  if (ws.ctr->vis > ws.rec_cap) ws.ctr->overflow |= 1u;
+  if (ws.ctr->bins > ws.bin_cap) ws.ctr->overflow |= 2u;
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan(Workspace ws) {
   __shared__ uint32_t sh[kScanChunk];
   __shared__ uint32_t swarp[32];
@@ -644,8 +782,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Workspace ws) {
   block_scan_array(ws.coarse_count, ws.coarse_off, ws.ncoarse, &ws.ctr->coarse_total, sh, swarp, &sctot);
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint64_t need = (uint64_t)ws.ctr->fine_total + ws.ctr->coarse_total;
-    if (need > ws.bin_cap) ws.ctr->overflow |= 2u;
+    check_scratch(ws);
   }
 }
 
@@ -751,46 +888,59 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(Workspace ws, uint32_
   if (blockIdx.x == nchunks - 1 && threadIdx.x == 0) {
     const uint32_t total = base + ws.scan_part[blockIdx.x];
     ws.ctr->fine_total = total;
-    if ((uint64_t)total + ws.ctr->coarse_total > ws.bin_cap) ws.ctr->overflow |= 2u;
+    check_scratch(ws);
   }
 }
 
 // Scatter record indices into their tile bins (cursor atomics aggregated
-// across the warp).
+// across the warp).  Records in coarse bins are taken one per warp from the
+// setup's list at the end of the bins, as long as the list and the bins do not
+// meet: large triangles often follow one another, and 32 of them in one warp
+// are a chain of hundreds of atomics (1,000 screen-covering triangles at
+// 2560x1440: fill 220 -> 15 us).
 __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __restrict__ surfs) {
   const uint32_t nrec = min(ws.ctr->nrec, ws.rec_cap);
   if (ws.ctr->overflow) return;
   const uint32_t coarse_base = ws.ctr->fine_total;
-  const uint32_t stride = gridDim.x * blockDim.x;
+  const uint32_t stride = gridDim.x * blockDim.x, ncoarse = ws.ctr->ncoarse;
+  const bool list = (uint64_t)coarse_base + ws.ctr->coarse_total + ncoarse <= ws.bin_cap;
   for (uint32_t r0 = blockIdx.x * blockDim.x; r0 < nrec; r0 += stride) {
     const uint32_t r = r0 + threadIdx.x;
     const bool valid = r < nrec;
-    Foot f{0, 0, 0, 0, false};
+    Foot f{0, -1, 0, -1, false};
     const Surface* S = surfs;
-    int total = 0;
     if (valid) {
-      float4 q = __ldg(reinterpret_cast<const float4*>(ws.rec + r) + 3);
+      const float4 q = __ldg(reinterpret_cast<const float4*>(ws.rec + r) + 3);
       S = surfs + __float_as_uint(q.z);
-      f = footprint(__float_as_uint(q.x), __float_as_uint(q.y), ws);
-      total = foot_count(f);
+      int ref;
+      f = footprint(__float_as_uint(q.x), __float_as_uint(q.y), __float_as_uint(q.w), ws, &ref);
     }
-    int maxt = total;
-    for (int o = 16; o > 0; o >>= 1) maxt = max(maxt, __shfl_xor_sync(0xFFFFFFFFu, maxt, o));
-    for (int it = 0; it < maxt; it++) {
-      const bool act = it < total;
-      const uint32_t tile = act ? foot_tile(f, it, *S) : 0u;
-      const uint32_t pf = agg_inc(ws.fine_count, tile, act && !f.coarse);
-      const uint32_t pc = agg_inc(ws.coarse_count, tile, act && f.coarse);
-      if (act) {
-        const uint32_t pos = f.coarse ? coarse_base + ws.coarse_off[tile] + pc : ws.fine_off[tile] + pf;
-        ws.bins[pos] = r;
-      }
+    each_fine_tile(
+        f, valid && !f.coarse ? foot_count(f) : 0, S, r,
+        [&](uint32_t tile, bool on) {
+          const uint32_t pos = agg_inc(ws.fine_count, tile, on);
+          if (on) ws.bins[ws.fine_off[tile] + pos] = r;
+        },
+        [&](uint32_t rr, uint32_t tile) { ws.bins[ws.fine_off[tile] + atomicAdd(&ws.fine_count[tile], 1u)] = rr; });
+    each_coarse_tile(f, valid && f.coarse && !list, S, r, [&](uint32_t rr, uint32_t tile) {
+      ws.bins[coarse_base + ws.coarse_off[tile] + atomicAdd(&ws.coarse_count[tile], 1u)] = rr;
+    });
+  }
+  if (!list) return;
+  const uint32_t warps = stride / 32, lane = threadIdx.x & 31;
+  for (uint32_t i = blockIdx.x + gridDim.x * (threadIdx.x / 32); i < ncoarse; i += warps) {
+    const uint32_t r = ws.bins[ws.bin_cap - 1 - i];
+    const float4 q = __ldg(reinterpret_cast<const float4*>(ws.rec + r) + 3);
+    const Surface& S = surfs[__float_as_uint(q.z)];
+    int ref;
+    const Foot f = footprint(__float_as_uint(q.x), __float_as_uint(q.y), __float_as_uint(q.w), ws, &ref);
+    const uint32_t w = (uint32_t)(f.tx1 - f.tx0 + 1), n = (uint32_t)foot_count(f);
+    for (uint32_t k = lane; k < n; k += 32) {
+      const uint32_t tile = S.ctile_base + (f.ty0 + k / w) * S.ctiles_x + f.tx0 + k % w;
+      ws.bins[coarse_base + ws.coarse_off[tile] + atomicAdd(&ws.coarse_count[tile], 1u)] = r;
     }
   }
 }
-
-
-
 
 // kernel1 + kernel2 for one 16x16 tile: depth min, then the canonical id.
 //
@@ -1086,8 +1236,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             const uint32_t bw = (uint32_t)(bx1 - bx0), pw = (bw + 1) >> 1;
             area = pw * (uint32_t)(by1 - by0);
             geo = (uint32_t)(bx0 - tx0) | ((uint32_t)(by0 - ty0) << 4) | (bw << 8) | (((65536u + pw - 1) / pw) << 13);
-            // the walk rule of the bbox's left column, once per row of this tile
-            if ((int)(xr & 0xFFFF) >= tx0) skip = walk_skip_rows(xr, yr, by0, by1, ty0, chunk);
+            // the walk rule of the bbox's left column, once per row of this
+            // tile (a tight box has left that column out)
+            if ((int)(xr & 0xFFFF) >= tx0 && !__float_as_uint(q3.w)) skip = walk_skip_rows(xr, yr, by0, by1, ty0, chunk);
           }
         }
         // Depth cull.  A record that covers every coverable pixel of the tile

@@ -321,6 +321,28 @@ GBR_HD void bbox4(f3 p0, f3 p1, f3 p2, float width, float height, float mm[4]) {
   mm[3] = clampf_(max3f(y0, y1, y2), 0.0f, height - 1.0f);
 }
 
+// The box of the pixels a small triangle can cover, smaller than bbox4: x and
+// y its rounded vertices, mm its bbox4 on a w x h surface (w <= 3840, h <=
+// 2160).  For vertices on the surface at most 64 apart every term of the
+// coverage test below is an integer below 2^24 and exact, and its tolerances
+// (1e-4, and 1e-4 of half the area of at most 2048) stay below one: it is the
+// closed triangle.  So the column left of the vertices and the row above
+// them, which bbox4 includes, have no pixel (the walk rule, which only skips
+// pixels of that column, then skips none), and a triangle without area has
+// none at all.  Returns kBoxTight with mm shrunk, kBoxEmpty with mm shrunk and
+// nothing to cover, or kBoxAny with mm as it is.
+enum { kBoxAny = 0, kBoxTight = 1, kBoxEmpty = 2 };
+GBR_HD int tight_box(f3 x, f3 y, float w, float h, float mm[4]) {
+  const float x0 = min3f(x.x, x.y, x.z), x1 = max3f(x.x, x.y, x.z);
+  const float y0 = min3f(y.x, y.y, y.z), y1 = max3f(y.x, y.y, y.z);
+  if (!(x0 >= 1.0f && y0 >= 0.0f && x1 <= w && y1 <= h && x1 - x0 <= 64.0f && y1 - y0 <= 64.0f)) return kBoxAny;
+  const float area2 = (x.y - x.x) * (y.z - y.x) - (x.z - x.x) * (y.y - y.x);  // exact
+  if (area2 != area2) return kBoxAny;  // a NaN vertex
+  mm[0] = x0;
+  mm[2] = y0;
+  return area2 == 0.0f || mm[0] >= mm[1] || mm[2] >= mm[3] ? kBoxEmpty : kBoxTight;
+}
+
 // Edge-function coverage test of integer pixel (px,py) against the rounded
 // triangle (cl2.cl:4798-4807, point_in_tri), split into per-triangle
 // constants and a per-pixel part with the same evaluation tree.

@@ -438,12 +438,12 @@ __device__ int reflection_pixel(const SceneDev& sc, const ReflectCam& v, int x, 
   const uint32_t ssid = __ldg(&G->ssid);
   if (ssid != 0xFFFFFFFFu) {
     // the pixel's clip output, as prearrange wrote it to cutdown_tris
-    f3 w[3], o0[3], o1[3];
+    f3 w[3], tp[3];
     uint32_t oid;
-    load_world(sc, tri, w, &oid);
-    const int n = transform_clip(w, v.cpos, v.cc, v.cs, v.fov, (float)W, (float)H, o0, o1);
+    int flags;
+    load_world(sc, tri, w, &oid, &flags);
+    const int n = transform_clip(w, v.cpos, v.cc, v.cs, v.fov, (float)W, (float)H, (int)sub, tp);
     if ((int)sub >= n) return 0;
-    const f3* tp = sub ? o1 : o0;
     const f3 xpv = mk3(roundf(tp[0].x), roundf(tp[1].x), roundf(tp[2].x));
     const f3 ypv = mk3(roundf(tp[0].y), roundf(tp[1].y), roundf(tp[2].y));
     const float rc = rconstant(xpv, ypv);

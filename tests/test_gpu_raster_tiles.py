@@ -72,3 +72,42 @@ def test_hidden_cube_face_records():
     dyn, _ = O.shadow(sc)
     assert np.array_equal(gs.cubemaps()[:len(dyn)], dyn)
     gs.close()
+
+
+def test_triangles_without_a_pixel():
+    """Triangles that round to a line or a point are counted as visible and draw nothing."""
+    rng = np.random.default_rng(4)
+    w, h = 200, 120
+    tl = []
+    for i in range(300):
+        c = rng.integers(5, (w - 5, h - 5))
+        r = rng.uniform(-0.4, 0.4, (2, 3))
+        if i % 3 == 0:  # three points of one pixel row
+            r[0] = (0, 3.0, 7.0)
+        tl.append(screen_tri(c[0] + r[0], c[1] + r[1], rng.uniform(100, 900), w, h))
+    sc = tri_scene(tl, w, h, descs=np.stack(TWO_SIDED))
+    gs = GpuScene(sc)
+    got = gs.render(sc.cameras[0], sc.views[0]).numpy()
+    ref = O.render(sc, O.build_textures(sc.tex_sizes, sc.tex_pixels), sc.cameras[0], sc.views[0])
+    assert (ref["depth"] == 0xFFFFFFFF).all() and np.array_equal(got["depth"], ref["depth"])
+    st = gs.stats()
+    assert st["view_records"] == 300 and st["view_samples"] == 0 and st["fragments_ref"] == ref["fragments"]
+    gs.close()
+
+
+@pytest.mark.parametrize("n", [900, 9000])
+def test_coarse_records(n):
+    """Every record in the coarse bins: listed at the end of the bins (900), or too many for that (9000)."""
+    rng = np.random.default_rng(n)
+    w, h, leg = 640, 480, 60
+    x, y, z = rng.uniform(0, w - leg, n), rng.uniform(0, h - leg, n), rng.uniform(100, 3000, n)
+    sc = tri_scene([screen_tri([a, a + leg, a], [b, b, b + leg], d, w, h) for a, b, d in zip(x, y, z)], w, h,
+                   descs=np.stack(TWO_SIDED))
+    gs = GpuScene(sc)
+    gs.set_tuning(S.PASS_VIEW, fine_max_tiles=1, coarse_tile=64)
+    got = gs.render(sc.cameras[0], sc.views[0]).numpy()
+    ref = O.render(sc, O.build_textures(sc.tex_sizes, sc.tex_pixels), sc.cameras[0], sc.views[0])
+    assert np.array_equal(got["depth"], ref["depth"]) and np.array_equal(got["id"], ref["id"])
+    st, cap = gs.stats(), 4 * (n + 1024)
+    assert st["retries"] == 0 and st["view_records"] == n and (st["view_bin_entries"] + n > cap) == (n == 9000)
+    gs.close()
