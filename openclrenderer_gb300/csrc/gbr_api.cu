@@ -83,13 +83,10 @@ gbr_status reserve_pass(WorkMem& w, const PassShape& sh, bool view) {
   TRY(w.rec.reserve(w.rec_target));
   if (view) TRY(w.srec.reserve(w.rec_target));
   TRY(w.bins.reserve(w.bin_target));
-  TRY(w.fine_count.reserve(sh.nfine));
+  TRY(w.counts.reserve((size_t)kCounterWords + sh.nfine + sh.ncoarse));
   TRY(w.fine_off.reserve(sh.nfine));
   TRY(w.tiles.reserve(sh.nfine));
-  TRY(w.coarse_count.reserve(sh.ncoarse));
   TRY(w.coarse_off.reserve(sh.ncoarse));
-  TRY(w.scan_part.reserve(scan_chunks(sh.nfine)));
-  TRY(w.ctr.reserve(1));
   if (view) TRY(w.pix_rec.reserve(sh.npix));
   if (view) TRY(w.tile_empty.reserve(sh.nfine));
   if (view) TRY(w.vis.reserve((size_t)std::max<uint32_t>(sh.nitems, 1) * std::max<uint32_t>((sh.nobjects + 31) / 32, 1)));
@@ -263,43 +260,40 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
   ws.rec = wm.rec.p;
   ws.srec = view ? wm.srec.p : nullptr;
   ws.rec_cap = (uint32_t)std::min<size_t>(wm.rec.cap, 0xFFFFFFF0u);
-  ws.fine_count = wm.fine_count.p;
+  ws.ctr = reinterpret_cast<Counters*>(wm.counts.p);
+  ws.fine_count = wm.counts.p + kCounterWords;
+  ws.coarse_count = ws.fine_count + sh.nfine;
+  ws.ncounts = kCounterWords + sh.nfine + sh.ncoarse;
   ws.fine_off = wm.fine_off.p;
   ws.nfine = sh.nfine;
-  ws.coarse_count = wm.coarse_count.p;
   ws.coarse_off = wm.coarse_off.p;
   ws.ncoarse = sh.ncoarse;
   ws.bins = wm.bins.p;
   ws.bin_cap = (uint32_t)std::min<size_t>(wm.bins.cap, 0xFFFFFFF0u);
-  ws.scan_part = wm.scan_part.p;
   const bool table = pass_tile_table(view, sh);
   ws.tiles = table ? wm.tiles.p : nullptr;
+  ws.list = !view && !table ? reinterpret_cast<uint32_t*>(wm.tiles.p) : nullptr;
   // views: the object cull needs the world cache (and with it the radii)
   const bool cull = view && sd.world && s->objr.p && sd.ndescs && sh.nobjects == sd.ndescs && sh.nitems <= 65535;
   ws.vis = cull ? wm.vis.p : nullptr;
   ws.vis_words = cull ? (sd.ndescs + 31) / 32 : 0;
   ws.pack_keys = view && sd.ntris < (1u << 22) - 1;
-  ws.ctr = wm.ctr.p;
   ws.fine_max = tu.fine_max;
   ws.coarse_shift = tu.coarse_shift;
-  CU(cudaMemsetAsync(ws.ctr, 0, sizeof(Counters), geom));
-  CU(cudaMemsetAsync(ws.fine_count, 0, sizeof(uint32_t) * std::max<uint32_t>(sh.nfine, 1), geom));
-  CU(cudaMemsetAsync(ws.coarse_count, 0, sizeof(uint32_t) * std::max<uint32_t>(sh.ncoarse, 1), geom));
   auto mark = [&](int k, cudaStream_t on) -> cudaError_t { return ev ? cudaEventRecord(ev[k], on) : cudaSuccess; };
   CU(mark(0, geom));
   if (view) {
-    if (cull) CU(launch_object_cull(sd, wm.views.p, wm.surf.p, sh.nitems, s->objr.p, ws.vis_words, wm.vis.p, geom));
+    CU(launch_begin_views(sd, sh.one_view, sh.one_surf, wm.views.p, wm.surf.p, sh.nitems, s->objr.p, ws, geom));
     CU(launch_setup_views(sd, wm.views.p, sh.nitems, wm.surf.p, ws, geom));
   } else {
     // the setup writes small triangles straight into the faces
-    CU(launch_clear_surfaces(wm.surf.p, sh.nsurf, geom));
+    CU(launch_begin_faces(wm.surf.p, sh.nsurf, ws, geom));
     CU(launch_setup_shadow(sd, wm.jobs.p, sh.nitems, wm.surf.p, ws, geom));
   }
   CU(mark(1, geom));
   const bool prep = view && sh.shade;
   const bool on_side = prep && side && side->stream;
-  if (table) CU(launch_tile_table(ws, wm.surf.p, sh.nsurf, geom));
-  CU(launch_scan(ws, geom));
+  CU(launch_offsets(ws, wm.surf.p, sh.nsurf, sh.tiles_per_surface, geom));
   CU(mark(2, geom));
   CU(launch_fill(ws, wm.surf.p, geom));
   CU(mark(3, geom));
@@ -417,7 +411,7 @@ gbr_status enqueue_pass(gbr_scene* s, bool view, const PassShape& sh, cudaStream
   if (view) TRY(ensure_side(s));
   TRY(launch_pass(s, wm, s->tune[view ? GBR_PASS_VIEW : GBR_PASS_SHADOW], view, sh, counter_slot(s, view), ev, st,
                   geom, s->geom_done, view ? &s->side : nullptr));
-  s->stats.launches += pass_kernels(view, sh.shade, sh.nfine, &sh);
+  s->stats.launches += pass_kernels(view, sh.shade, &sh);
   if (view) s->view_shaded = sh.shade;
   return GBR_OK;
 }
@@ -881,10 +875,22 @@ gbr_status gbr_shadow_pass(gbr_scene* s, void* stream) {
     return GBR_OK;
   }
   WorkMem& wm = s->ws_shadow;
+  const void *old_surf = wm.surf.p, *old_jobs = wm.jobs.p;
   TRY(wm.surf.reserve(surfs.size()));
   TRY(wm.jobs.reserve(jobs.size()));
-  CU(cudaMemcpyAsync(wm.surf.p, surfs.data(), surfs.size() * sizeof(Surface), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(wm.jobs.p, jobs.data(), jobs.size() * sizeof(ShadowJob), cudaMemcpyHostToDevice, st));
+  // the faces and jobs only change with the lights and the tuning: copied when
+  // they differ from what the device holds (the previous pass, whichever its
+  // stream, has been waited for above)
+  const size_t sb = surfs.size() * sizeof(Surface), jb = jobs.size() * sizeof(ShadowJob);
+  std::vector<uint8_t> held(sb + jb);
+  memcpy(held.data(), surfs.data(), sb);
+  memcpy(held.data() + sb, jobs.data(), jb);
+  if (held != wm.faces_held || old_surf != wm.surf.p || old_jobs != wm.jobs.p) {
+    wm.faces_held.clear();
+    CU(cudaMemcpyAsync(wm.surf.p, surfs.data(), sb, cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync(wm.jobs.p, jobs.data(), jb, cudaMemcpyHostToDevice, st));
+    wm.faces_held = std::move(held);
+  }
   // the stream's work before this pass: what a view pass on the same stream
   // may run after while this pass renders
   TRY(ensure_aux(s));
@@ -969,8 +975,10 @@ static gbr_status render_views(gbr_scene* s, uint32_t n, const gbr_camera* cams,
     geom = s->aux;
     CU(cudaStreamWaitEvent(geom, s->pre_geom, 0));
   }
-  CU(cudaMemcpyAsync(wm.surf.p, surfs.data(), n * sizeof(Surface), cudaMemcpyHostToDevice, geom));
-  CU(cudaMemcpyAsync(wm.views.p, vp.data(), n * sizeof(ViewParams), cudaMemcpyHostToDevice, geom));
+  if (n > 1) {  // (a single view travels with the pass's first launch)
+    CU(cudaMemcpyAsync(wm.surf.p, surfs.data(), n * sizeof(Surface), cudaMemcpyHostToDevice, geom));
+    CU(cudaMemcpyAsync(wm.views.p, vp.data(), n * sizeof(ViewParams), cudaMemcpyHostToDevice, geom));
+  }
   PassShape sh;
   sh.nitems = sh.nsurf = n;
   sh.nfine = tb;

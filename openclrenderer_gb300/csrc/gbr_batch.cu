@@ -179,8 +179,8 @@ gbr_status launch_graph(gbr_batch* b, const gbr_camera* cams, cudaStream_t st) {
   CU(cudaGraphLaunch(b->exec, st));
   CU(cudaEventRecord(b->done, st));
   b->launches++;
-  b->s->stats.launches += pass_kernels(true, b->vshape.shade, b->vshape.nfine, &b->vshape) +
-                          (b->sshape.nitems ? pass_kernels(false, false, b->sshape.nfine, &b->sshape) : 0u);
+  b->s->stats.launches += pass_kernels(true, b->vshape.shade, &b->vshape) +
+                          (b->sshape.nitems ? pass_kernels(false, false, &b->sshape) : 0u);
   b->in_flight = true;
   b->last_stream = st;
   return GBR_OK;
@@ -442,7 +442,7 @@ gbr_status gbr_batch_get_info(gbr_batch* b, gbr_batch_info* out) {
   uint64_t bytes = 0;
   for (const WorkMem* w : {&b->wv, &b->wsh}) {
     bytes += w->rec.cap * sizeof(RasterRec) + w->srec.cap * sizeof(ShadeRec) + w->bins.cap * 4;
-    bytes += (w->fine_count.cap + w->fine_off.cap + w->coarse_count.cap + w->coarse_off.cap) * 4;
+    bytes += (w->counts.cap + w->fine_off.cap + w->coarse_off.cap) * 4;
     bytes += (w->pix_rec.cap + w->pix_depth.cap) * 4 + w->tile_empty.cap;
   }
   out->scratch_bytes = bytes;

@@ -116,9 +116,15 @@ struct Counters {
   uint32_t fine_total, coarse_total;
   uint32_t ncoarse;             // records in coarse bins: their list runs down from the end of the bins
   uint32_t vis;                 // visible triangles: the records, and those that cover no pixel
+  uint32_t nlist;               // depth-only passes: tiles with records (Workspace::list)
   unsigned long long bins;      // tiles of the visible triangles' bbox4
   unsigned long long samples;   // covered pixel-samples (point_in_tri passes) of the depth pass
 };
+
+// The counters and the tile counts behind them are cleared as one run of words
+// (WorkMem::counts): Counters, then fine_count, then coarse_count.
+constexpr uint32_t kCounterWords = 64;
+static_assert(sizeof(Counters) <= 4 * kCounterWords, "counters");
 
 struct SceneDev {
   const gbr_triangle* tris;
@@ -162,17 +168,18 @@ struct Workspace {
   RasterRec* rec;
   ShadeRec* srec;  // may be null (shadow passes)
   uint32_t rec_cap;
-  uint32_t* fine_count;
-  uint32_t* fine_off;
+  uint32_t* fine_count;  // records per tile
+  uint32_t* fine_off;    // the bins' starts, then (the fill's cursors) their ends
   uint32_t nfine;
   uint32_t* coarse_count;
   uint32_t* coarse_off;
   uint32_t ncoarse;
   uint32_t* bins;
   uint32_t bin_cap;
-  // per fine tile: its surface and its global coarse tile (launch_tile_table)
-  const uint2* tiles;
-  uint32_t* scan_part;  // per chunk of fine counts (scan_chunks), or null: one-block scan
+  // per fine tile: its surface and its global coarse tile, or null
+  uint2* tiles;
+  uint32_t* list;       // depth-only passes: the fine tiles that have records (Counters::nlist), or null
+  uint32_t ncounts;     // words from ctr on that a pass starts by clearing
   const uint32_t* vis;  // views: object cull bits (k_object_cull), vis_words per view, or null
   uint32_t vis_words;
   uint32_t pack_keys;   // views: every key (2 * triangle + 1) is below 2^23 - 1 (32-bit id resolve)
@@ -191,20 +198,24 @@ struct Workspace {
 // ---- launchers (gbr_kernels.cu) ----
 // World-space cache (world may be null: objects only) and the per-object table.
 cudaError_t launch_world(const SceneDev& sc, float4* world, float4* objq, uint32_t* objr, cudaStream_t st);
-// Object cull bits of a view pass (words = ceil(ndescs / 32) per view); needs
-// the per-object table and the radii of the world-space cache.
-cudaError_t launch_object_cull(const SceneDev& sc, const ViewParams* d_views, const Surface* d_surf, uint32_t nviews,
-                               const uint32_t* objr, uint32_t words, uint32_t* vis, cudaStream_t st);
+// First kernel of a view pass: clears the counters, writes the one view given
+// in host memory (null: the caller has filled d_views / d_surf) and, when
+// ws.vis is set, the object cull bits (which need the per-object table and the
+// radii of the world-space cache).
+cudaError_t launch_begin_views(const SceneDev& sc, const ViewParams* one_view, const Surface* one_surf,
+                               ViewParams* d_views, Surface* d_surf, uint32_t nviews, const uint32_t* objr,
+                               const Workspace& ws, cudaStream_t st);
+// First kernel of a depth-only pass: clears the surfaces (16-byte aligned) to
+// UINT_MAX and the counters to 0.
+cudaError_t launch_begin_faces(const Surface* d_surf, uint32_t nsurf, const Workspace& ws, cudaStream_t st);
 cudaError_t launch_setup_views(const SceneDev& sc, const ViewParams* d_views, uint32_t nviews,
                                const Surface* d_surf, const Workspace& ws, cudaStream_t st);
 cudaError_t launch_setup_shadow(const SceneDev& sc, const ShadowJob* d_jobs, uint32_t njobs,
                                 const Surface* d_surf, const Workspace& ws, cudaStream_t st);
-// One block when the fine counts fit one chunk (or scan_part is null), else
-// scan_chunks(nfine) blocks in two kernels.
-cudaError_t launch_scan(const Workspace& ws, cudaStream_t st);
-// ws.tiles for the pass's nsurf surfaces (ws.nfine fine tiles, ws.coarse_shift).
-cudaError_t launch_tile_table(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, cudaStream_t st);
-uint32_t scan_chunks(uint32_t nfine);
+// Bin offsets, and ws.tiles / ws.list where set (k_offsets); per_surface: the
+// common tile count when every surface has the same size, else 0.
+cudaError_t launch_offsets(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, uint32_t per_surface,
+                           cudaStream_t st);
 cudaError_t launch_fill(const Workspace& ws, const Surface* d_surf, cudaStream_t st);
 // Views that shade: every record's setup output becomes its shade constants
 // (prep_shade).  Needs the setup done; kernel3 needs it done.
@@ -243,8 +254,6 @@ cudaError_t launch_texture_upload(uchar4* atlas, const uint32_t* nums, const uin
 cudaError_t launch_mips(uchar4* atlas, const uint32_t* nums, const uint32_t* sizes,
                         uint32_t mipmap_start, const int32_t* tsizes, uint32_t ntex,
                         int32_t max_size, cudaStream_t st);
-// depth-only passes: every surface's depth to UINT_MAX (16-byte aligned buffers)
-cudaError_t launch_clear_surfaces(const Surface* d_surf, uint32_t nsurf, cudaStream_t st);
 cudaError_t launch_atomic_rate(uint32_t* g, uint32_t nwords, int iters, int shared_mode, uint32_t blocks,
                                cudaStream_t st);
 cudaError_t launch_fill_u32(uint32_t* p, uint32_t v, size_t n, cudaStream_t st);

@@ -448,15 +448,38 @@ __global__ void __launch_bounds__(256) k_world(SceneDev sc, float4* __restrict__
 // hence the far-clip condition.)  The margins (a relative 1e-3 of the radius
 // and of the distance, plus one unit) are orders of magnitude above the
 // float rounding of the per-triangle transform.
-__global__ void __launch_bounds__(256) k_object_cull(SceneDev sc, const ViewParams* __restrict__ views,
-                                                     const Surface* __restrict__ surfs, const uint32_t* __restrict__ objr,
-                                                     uint32_t words, uint32_t* __restrict__ vis) {
-  const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t v = blockIdx.y;
+//
+// The first kernel of a view pass: cull_blocks blocks do that (0: no object
+// cull), the others clear the pass's counters (ncounts words) and, for a pass
+// of one view given with the launch (one), write its parameters where the
+// other kernels read them.  One launch instead of three clears, two copies and
+// the cull.
+__global__ void __launch_bounds__(256) k_begin_views(SceneDev sc, const __grid_constant__ ViewParams one_view,
+                                                     const __grid_constant__ Surface one_surf, bool one,
+                                                     ViewParams* __restrict__ views, Surface* __restrict__ surfs,
+                                                     uint32_t nviews, const uint32_t* __restrict__ objr,
+                                                     uint32_t words, uint32_t* __restrict__ vis,
+                                                     uint32_t cull_blocks, uint32_t* __restrict__ counts,
+                                                     uint32_t ncounts) {
+  if (blockIdx.x >= cull_blocks) {
+    const uint32_t b = blockIdx.x - cull_blocks;
+    for (uint32_t i = b * blockDim.x + threadIdx.x; i < ncounts; i += (gridDim.x - cull_blocks) * blockDim.x)
+      counts[i] = 0;
+    if (one && b == 0) {
+      static_assert(sizeof(ViewParams) % 4 == 0 && sizeof(ViewParams) / 4 <= 256 && sizeof(Surface) / 4 <= 256, "");
+      if (threadIdx.x < sizeof(ViewParams) / 4)
+        reinterpret_cast<uint32_t*>(views)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&one_view)[threadIdx.x];
+      if (threadIdx.x < sizeof(Surface) / 4)
+        reinterpret_cast<uint32_t*>(surfs)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&one_surf)[threadIdx.x];
+    }
+    return;
+  }
+  const uint32_t per_view = cull_blocks / nviews, v = blockIdx.x / per_view;
+  const uint32_t o = (blockIdx.x % per_view) * blockDim.x + threadIdx.x;
   bool keep = false;
   if (o < sc.ndescs) {
-    const ViewParams& V = views[v];
-    const Surface& S = surfs[V.surface];
+    const ViewParams& V = one ? one_view : views[v];
+    const Surface& S = one ? one_surf : surfs[V.surface];
     const f3 cpos = mk3(V.cpos[0], V.cpos[1], V.cpos[2]);
     const float4 q2 = __ldg(sc.objq + (size_t)o * kObjQuads + 2);
     const f3 wp = mk3(q2.x, q2.y, q2.z);
@@ -686,104 +709,76 @@ __global__ void __launch_bounds__(128, 7) k_setup_shadow(const __grid_constant__
   setup_done(&sums, ws);
 }
 
-// Each fine tile's surface (binary search over tile_base) and global coarse
-// tile: the raster's and kernel3's first loads.
-__global__ void __launch_bounds__(256) k_tile_table(const Surface* __restrict__ surfs, uint32_t nsurf,
-                                                    uint32_t nfine, int coarse_shift, uint2* __restrict__ tiles) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nfine) return;
-  uint32_t lo = 0, hi = nsurf - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (surfs[mid].tile_base <= t) lo = mid; else hi = mid - 1;
-  }
-  const Surface& S = surfs[lo];
-  const uint32_t lt = t - S.tile_base;
-  const int tx = lt % S.tiles_x, ty = lt / S.tiles_x;
-  tiles[t] = make_uint2(lo, S.ctile_base + (ty >> coarse_shift) * S.ctiles_x + (tx >> coarse_shift));
-}
-
-// Exclusive scan of fine and coarse tile counts (one block of 1024 threads);
-// counts are reset to zero to serve as fill cursors.  Rounds of 8192 counts
-// are staged in shared memory with coalesced loads, each thread scans 8
-// contiguous values, and a block scan joins the threads.
-constexpr int kScanThreads = 1024;
-constexpr int kScanPer = 8;
-constexpr int kScanChunk = kScanThreads * kScanPer;
-
-__device__ __forceinline__ uint32_t block_scan_1024(uint32_t v, uint32_t* swarp, uint32_t* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t incl = v;
+// Warp-aggregated allocation of n slots from *counter; every lane of the
+// warp must call it (n may be 0).  Returns this lane's first slot.
+__device__ __forceinline__ uint32_t warp_alloc(uint32_t* counter, uint32_t n) {
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  uint32_t incl = n;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= o) incl += t;
+    const uint32_t v = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += v;
   }
-  if (lane == 31) swarp[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t w = swarp[lane];
-    uint32_t wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, o);
-      if (lane >= o) wi += t;
-    }
-    swarp[lane] = wi - w;
-    if (lane == 31) *total = wi;
-  }
-  __syncthreads();
-  return swarp[warp] + incl - v;
+  const uint32_t total = __shfl_sync(full, incl, 31);
+  uint32_t base = 0;
+  if (lane == 31 && total) base = atomicAdd(counter, total);
+  return __shfl_sync(full, base, 31) + incl - n;
 }
 
-__device__ void block_scan_array(uint32_t* count, uint32_t* off, uint32_t n, uint32_t* total, uint32_t* sh,
-                                 uint32_t* swarp, uint32_t* sctot) {
-  uint32_t carry = 0;
-  for (uint32_t c0 = 0; c0 < n; c0 += kScanChunk) {
-    const uint32_t m = min((uint32_t)kScanChunk, n - c0);
-    for (uint32_t i = threadIdx.x; i < (uint32_t)kScanChunk; i += kScanThreads) sh[i] = i < m ? count[c0 + i] : 0u;
-    __syncthreads();
-    uint32_t v[kScanPer], sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-      v[k] = sh[threadIdx.x * kScanPer + k];
-      sum += v[k];
-    }
-    const uint32_t excl = block_scan_1024(sum, swarp, sctot);
-    uint32_t run = carry + excl;
-#pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-      sh[threadIdx.x * kScanPer + k] = run;
-      run += v[k];
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < m; i += kScanThreads) {
-      off[c0 + i] = sh[i];
-      count[c0 + i] = 0;
-    }
-    carry += *sctot;
-    __syncthreads();
+// Bin offsets: every fine tile's bin, and every coarse tile's, gets its place
+// from a counter, a warp's tiles at a time (the order of the bins is free:
+// what a tile resolves does not depend on it, so no scan is needed).  fine_off
+// and coarse_off then serve as the fill's cursors: after it they are the
+// bins' ends.  Also, where asked for,
+//   ws.tiles  each fine tile's surface (binary search over tile_base) and
+//             global coarse tile: the first loads of the raster and kernel3;
+//   ws.list   depth-only passes with per_surface tiles on every surface: the
+//             tiles that have records (a cube face's are mostly empty).
+// One launch for the scan's one or two and the tile table's: 3 us where the
+// one-block scan of a 1080p view took 8 and the chunked one 15.
+__global__ void __launch_bounds__(256) k_offsets(Workspace ws, const Surface* __restrict__ surfs, uint32_t nsurf,
+                                                 uint32_t per_surface) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t c = t < ws.nfine ? ws.fine_count[t] : 0u;
+  const uint32_t off = warp_alloc(&ws.ctr->fine_total, c);
+  if (t < ws.nfine) ws.fine_off[t] = off;
+  const uint32_t cc = t < ws.ncoarse ? ws.coarse_count[t] : 0u;
+  if ((t & ~31u) < ws.ncoarse) {  // warp-uniform
+    const uint32_t coff = warp_alloc(&ws.ctr->coarse_total, cc);
+    if (t < ws.ncoarse) ws.coarse_off[t] = coff;
   }
-  if (threadIdx.x == 0) *total = carry;
-}
-
-// The pass's scratch must hold every visible triangle and every tile of its
-// bbox4 (the limits callers know), although fewer are stored.
-__device__ __forceinline__ void check_scratch(const Workspace& ws) {
-  if (ws.ctr->vis > ws.rec_cap) ws.ctr->overflow |= 1u;
-  if (ws.ctr->bins > ws.bin_cap) ws.ctr->overflow |= 2u;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan(Workspace ws) {
-  __shared__ uint32_t sh[kScanChunk];
-  __shared__ uint32_t swarp[32];
-  __shared__ uint32_t sctot;
-  block_scan_array(ws.fine_count, ws.fine_off, ws.nfine, &ws.ctr->fine_total, sh, swarp, &sctot);
-  block_scan_array(ws.coarse_count, ws.coarse_off, ws.ncoarse, &ws.ctr->coarse_total, sh, swarp, &sctot);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    check_scratch(ws);
+  if (t == 0) {
+    // the scratch must hold every visible triangle and every tile of its
+    // bbox4 (the limits callers know), although fewer are stored
+    if (ws.ctr->vis > ws.rec_cap) ws.ctr->overflow |= 1u;
+    if (ws.ctr->bins > ws.bin_cap) ws.ctr->overflow |= 2u;
   }
+  if (!ws.tiles && !ws.list) return;
+  bool busy = false;
+  if (t < ws.nfine) {
+    uint32_t s = 0;
+    if (per_surface) {
+      s = t / per_surface;
+    } else {
+      uint32_t hi = nsurf - 1;
+      while (s < hi) {
+        const uint32_t mid = (s + hi + 1) >> 1;
+        if (surfs[mid].tile_base <= t) s = mid; else hi = mid - 1;
+      }
+    }
+    const Surface& S = surfs[s];
+    const uint32_t lt = t - S.tile_base;
+    const int tx = lt % S.tiles_x, ty = lt / S.tiles_x;
+    const uint32_t ct = S.ctile_base + (ty >> ws.coarse_shift) * S.ctiles_x + (tx >> ws.coarse_shift);
+    if (ws.tiles) ws.tiles[t] = make_uint2(s, ct);
+    busy = c > 0 || ws.coarse_count[ct] > 0;
+  }
+  if (!ws.list) return;
+  const unsigned who = __ballot_sync(0xFFFFFFFFu, busy);
+  const uint32_t at = warp_alloc(&ws.ctr->nlist, (threadIdx.x & 31) == 0 ? (uint32_t)__popc(who) : 0u);
+  const uint32_t first = __shfl_sync(0xFFFFFFFFu, at, 0);
+  if (busy) ws.list[first + (uint32_t)__popc(who & ((1u << (threadIdx.x & 31)) - 1u))] = t;
 }
 
 // Barycentrics (cl2.cl:5372-5384) split into the per-triangle part and the
@@ -856,42 +851,6 @@ __global__ void __launch_bounds__(256, 4) k_prep(SceneDev sc, Workspace ws) {
     prep_shade(sc, ws.srec + r);
 }
 
-// Many tiles (batches of views): the fine counts are scanned in chunks of
-// kScanChunk, one block each, into offsets relative to the chunk, with each
-// chunk's total in scan_part; one more block scans the coarse counts whole.
-// k_scan_add then adds the totals of the chunks before each chunk.
-__global__ void __launch_bounds__(kScanThreads) k_scan_chunks(Workspace ws, uint32_t nchunks) {
-  __shared__ uint32_t sh[kScanChunk];
-  __shared__ uint32_t swarp[32];
-  __shared__ uint32_t sctot;
-  if (blockIdx.x == nchunks) {
-    block_scan_array(ws.coarse_count, ws.coarse_off, ws.ncoarse, &ws.ctr->coarse_total, sh, swarp, &sctot);
-    return;
-  }
-  const uint32_t c0 = blockIdx.x * (uint32_t)kScanChunk;
-  const uint32_t m = min((uint32_t)kScanChunk, ws.nfine - c0);
-  block_scan_array(ws.fine_count + c0, ws.fine_off + c0, m, ws.scan_part + blockIdx.x, sh, swarp, &sctot);
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_add(Workspace ws, uint32_t nchunks) {
-  __shared__ uint32_t base;
-  if (threadIdx.x < 32) {
-    uint32_t sum = 0;
-    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 32) sum += ws.scan_part[i];
-    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
-    if (threadIdx.x == 0) base = sum;
-  }
-  __syncthreads();
-  const uint32_t c0 = blockIdx.x * (uint32_t)kScanChunk;
-  const uint32_t m = min((uint32_t)kScanChunk, ws.nfine - c0);
-  for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) ws.fine_off[c0 + i] += base;
-  if (blockIdx.x == nchunks - 1 && threadIdx.x == 0) {
-    const uint32_t total = base + ws.scan_part[blockIdx.x];
-    ws.ctr->fine_total = total;
-    check_scratch(ws);
-  }
-}
-
 // Scatter record indices into their tile bins (cursor atomics aggregated
 // across the warp).  Records in coarse bins are taken one per warp from the
 // setup's list at the end of the bins, as long as the list and the bins do not
@@ -918,12 +877,12 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
     each_fine_tile(
         f, valid && !f.coarse ? foot_count(f) : 0, S, r,
         [&](uint32_t tile, bool on) {
-          const uint32_t pos = agg_inc(ws.fine_count, tile, on);
-          if (on) ws.bins[ws.fine_off[tile] + pos] = r;
+          const uint32_t pos = agg_inc(ws.fine_off, tile, on);
+          if (on) ws.bins[pos] = r;
         },
-        [&](uint32_t rr, uint32_t tile) { ws.bins[ws.fine_off[tile] + atomicAdd(&ws.fine_count[tile], 1u)] = rr; });
+        [&](uint32_t rr, uint32_t tile) { ws.bins[atomicAdd(&ws.fine_off[tile], 1u)] = rr; });
     each_coarse_tile(f, valid && f.coarse && !list, S, r, [&](uint32_t rr, uint32_t tile) {
-      ws.bins[coarse_base + ws.coarse_off[tile] + atomicAdd(&ws.coarse_count[tile], 1u)] = rr;
+      ws.bins[coarse_base + atomicAdd(&ws.coarse_off[tile], 1u)] = rr;
     });
   }
   if (!list) return;
@@ -937,7 +896,7 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
     const uint32_t w = (uint32_t)(f.tx1 - f.tx0 + 1), n = (uint32_t)foot_count(f);
     for (uint32_t k = lane; k < n; k += 32) {
       const uint32_t tile = S.ctile_base + (f.ty0 + k / w) * S.ctiles_x + f.tx0 + k % w;
-      ws.bins[coarse_base + ws.coarse_off[tile] + atomicAdd(&ws.coarse_count[tile], 1u)] = r;
+      ws.bins[coarse_base + atomicAdd(&ws.coarse_off[tile], 1u)] = r;
     }
   }
 }
@@ -1098,7 +1057,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   uint32_t* lists = sm.lists;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {  // the tile's surface and bins
-    const uint32_t foff = ws.fine_off[tile], fcnt = ws.fine_count[tile], ftot = ws.ctr->fine_total;
+    const uint32_t fcnt = ws.fine_count[tile], foff = ws.fine_off[tile] - fcnt, ftot = ws.ctr->fine_total;
     uint32_t s, ct;
     if (ws.tiles) {  // two rounds of loads
       const uint2 tt = ws.tiles[tile];
@@ -1115,8 +1074,8 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
     sm.s = s;
     lists[0] = foff;
     lists[1] = fcnt;
-    lists[2] = ftot + ws.coarse_off[ct];
     lists[3] = ws.coarse_count[ct];
+    lists[2] = ftot + ws.coarse_off[ct] - lists[3];
     ssamples = 0;
     sm.szcap = kDepthClear;
   }
@@ -1395,6 +1354,22 @@ __global__ void __launch_bounds__(NT, (ID ? 1024 : 1280) / NT) k_raster(Workspac
   // surfaces of one size (cube faces) come as grid rows: surface = blockIdx.y
   const uint32_t tile = gridDim.y > 1 ? surfs[blockIdx.y].tile_base + blockIdx.x : tile0 + blockIdx.x;
   raster_tile<NT, ID, CC>(ws, surfs, nsurf, tile, gridDim.y > 1 ? (int)blockIdx.y : -1, sm);
+}
+
+// The tiles of ws.list (surfaces of per_surface tiles each) of a depth-only
+// pass, by as many blocks as fit at once: 24,576 tiles of a cubemap of which
+// some 4,000 have records took 30 us as a block each, mostly to start them.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1280 / NT) k_raster_list(Workspace ws, const Surface* __restrict__ surfs,
+                                                               uint32_t nsurf, uint32_t per_surface) {
+  __shared__ RasterSmem<NT, false> sm;
+  if (ws.ctr->overflow) return;
+  const uint32_t n = ws.ctr->nlist;
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint32_t tile = ws.list[i];
+    raster_tile<NT, false>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm);
+    __syncthreads();  // the next tile reuses the shared memory
+  }
 }
 
 // ---- kernel3 ------------------------------------------------------------------
@@ -2429,15 +2404,21 @@ __global__ void k_flush_objects(gbr_obj_g_descriptor* descs, const gbr_object_fl
   G->feature_flag = f.feature_flag;
 }
 
-// Clear every surface of a depth-only pass to UINT_MAX before its setup
-// rasterises small candidates into them (blockIdx.y = surface).
-__global__ void __launch_bounds__(256) k_clear_surfaces(const Surface* __restrict__ surfs) {
+// The first kernel of a depth-only pass: every surface to UINT_MAX before the
+// setup rasterises small candidates into it (blockIdx.y = surface), and the
+// pass's counters to 0 (the last grid row).
+__global__ void __launch_bounds__(256) k_begin_faces(const Surface* __restrict__ surfs, uint32_t nsurf,
+                                                     uint32_t* __restrict__ counts, uint32_t ncounts) {
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  if (blockIdx.y == nsurf) {
+    for (size_t i = first; i < ncounts; i += step) counts[i] = 0;
+    return;
+  }
   const Surface& S = surfs[blockIdx.y];
   const size_t n = (size_t)S.width * S.height;
   uint4* d4 = reinterpret_cast<uint4*>(S.depth);
   const uint4 v = make_uint4(kDepthClear, kDepthClear, kDepthClear, kDepthClear);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += (size_t)gridDim.x * blockDim.x)
-    d4[i] = v;
+  for (size_t i = first; i < n / 4; i += step) d4[i] = v;
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) S.depth[(n & ~(size_t)3) + threadIdx.x] = kDepthClear;
 }
 
@@ -2489,11 +2470,20 @@ cudaError_t launch_world(const SceneDev& sc, float4* world, float4* objq, uint32
   return cudaGetLastError();
 }
 
-cudaError_t launch_object_cull(const SceneDev& sc, const ViewParams* d_views, const Surface* d_surf, uint32_t nviews,
-                               const uint32_t* objr, uint32_t words, uint32_t* vis, cudaStream_t st) {
-  if (!nviews || !words) return cudaSuccess;
-  if (!sc.objq || !objr || !vis || nviews > 65535) return cudaErrorInvalidValue;
-  k_object_cull<<<dim3((words * 32 + 255) / 256, nviews), 256, 0, st>>>(sc, d_views, d_surf, objr, words, vis);
+cudaError_t launch_begin_views(const SceneDev& sc, const ViewParams* one_view, const Surface* one_surf,
+                               ViewParams* d_views, Surface* d_surf, uint32_t nviews, const uint32_t* objr,
+                               const Workspace& ws, cudaStream_t st) {
+  if (!nviews) return cudaErrorInvalidValue;
+  const bool one = nviews == 1 && one_view && one_surf;
+  uint32_t cull_blocks = 0;
+  if (ws.vis && ws.vis_words) {
+    if (!sc.objq || !objr) return cudaErrorInvalidValue;
+    cull_blocks = (ws.vis_words * 32 + 255) / 256 * nviews;
+  }
+  const uint32_t clear_blocks = std::min<uint32_t>((ws.ncounts + 1023) / 1024, (uint32_t)num_sms() * 2);
+  k_begin_views<<<cull_blocks + std::max<uint32_t>(clear_blocks, 1), 256, 0, st>>>(
+      sc, one ? *one_view : ViewParams{}, one ? *one_surf : Surface{}, one, d_views, d_surf, nviews, objr,
+      ws.vis_words, const_cast<uint32_t*>(ws.vis), cull_blocks, reinterpret_cast<uint32_t*>(ws.ctr), ws.ncounts);
   return cudaGetLastError();
 }
 
@@ -2520,26 +2510,13 @@ cudaError_t launch_setup_shadow(const SceneDev& sc, const ShadowJob* d_jobs, uin
   return cudaGetLastError();
 }
 
-cudaError_t launch_tile_table(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, cudaStream_t st) {
-  if (!ws.nfine) return cudaSuccess;
-  if (!ws.tiles || !nsurf) return cudaErrorInvalidValue;
-  k_tile_table<<<(ws.nfine + 255) / 256, 256, 0, st>>>(d_surf, nsurf, ws.nfine, ws.coarse_shift,
-                                                       const_cast<uint2*>(ws.tiles));
+cudaError_t launch_offsets(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, uint32_t per_surface,
+                           cudaStream_t st) {
+  if ((ws.tiles || ws.list) && !nsurf) return cudaErrorInvalidValue;
+  const uint32_t n = std::max(std::max(ws.nfine, ws.ncoarse), 1u);
+  k_offsets<<<(n + 255) / 256, 256, 0, st>>>(ws, d_surf, nsurf, per_surface);
   return cudaGetLastError();
 }
-
-cudaError_t launch_scan(const Workspace& ws, cudaStream_t st) {
-  const uint32_t nchunks = (ws.nfine + kScanChunk - 1) / kScanChunk;
-  if (nchunks <= 1 || !ws.scan_part) {
-    k_scan<<<1, kScanThreads, 0, st>>>(ws);
-  } else {
-    k_scan_chunks<<<nchunks + 1, kScanThreads, 0, st>>>(ws, nchunks);
-    k_scan_add<<<nchunks, kScanThreads, 0, st>>>(ws, nchunks);
-  }
-  return cudaGetLastError();
-}
-
-uint32_t scan_chunks(uint32_t nfine) { return (nfine + kScanChunk - 1) / kScanChunk; }
 
 cudaError_t launch_prep(const SceneDev& sc, const Workspace& ws, cudaStream_t st) {
   if (!ws.srec) return cudaErrorInvalidValue;
@@ -2555,6 +2532,15 @@ cudaError_t launch_fill(const Workspace& ws, const Surface* d_surf, cudaStream_t
 cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, uint32_t ntiles,
                           bool with_id, int threads, cudaStream_t st, uint32_t tiles_per_surface, uint32_t tile0) {
   if (!ntiles) return cudaSuccess;
+  if (!with_id && ws.list && tiles_per_surface) {
+    const uint32_t blocks = std::min<uint32_t>(ntiles, (uint32_t)num_sms() * (1280 / threads));
+    switch (threads) {
+      case 128: k_raster_list<128><<<blocks, 128, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
+      case 512: k_raster_list<512><<<blocks, 512, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
+      default: k_raster_list<256><<<blocks, 256, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
+    }
+    return cudaGetLastError();
+  }
   const int wid = with_id ? 1 : 0;
   // surfaces of equal size: one grid row per surface, no search for the owner
   const dim3 grid = (tile0 == 0 && tiles_per_surface && nsurf > 1 && nsurf <= 65535 &&
@@ -2674,9 +2660,9 @@ cudaError_t launch_flush_objects(gbr_obj_g_descriptor* descs, const gbr_object_f
   return cudaGetLastError();
 }
 
-cudaError_t launch_clear_surfaces(const Surface* d_surf, uint32_t nsurf, cudaStream_t st) {
-  if (!nsurf) return cudaSuccess;
-  k_clear_surfaces<<<dim3(64, nsurf), 256, 0, st>>>(d_surf);
+cudaError_t launch_begin_faces(const Surface* d_surf, uint32_t nsurf, const Workspace& ws, cudaStream_t st) {
+  if (!nsurf) return cudaErrorInvalidValue;
+  k_begin_faces<<<dim3(64, nsurf + 1), 256, 0, st>>>(d_surf, nsurf, reinterpret_cast<uint32_t*>(ws.ctr), ws.ncounts);
   return cudaGetLastError();
 }
 

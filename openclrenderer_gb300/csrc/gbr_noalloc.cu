@@ -57,11 +57,9 @@ constexpr size_t kMaxCoarseTiles = 1024;
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // byte offsets inside the scratch array
-constexpr size_t kOffCtr = 0;
-constexpr size_t kOffFineCount = align256(kOffCtr + sizeof(Counters));
-constexpr size_t kOffFineOff = align256(kOffFineCount + 4 * kMaxFineTiles);
-constexpr size_t kOffCoarseCount = align256(kOffFineOff + 4 * kMaxFineTiles);
-constexpr size_t kOffCoarseOff = align256(kOffCoarseCount + 4 * kMaxCoarseTiles);
+constexpr size_t kOffCounts = 0;  // Counters, fine counts, coarse counts
+constexpr size_t kOffFineOff = align256(kOffCounts + 4 * (kCounterWords + kMaxFineTiles + kMaxCoarseTiles));
+constexpr size_t kOffCoarseOff = align256(kOffFineOff + 4 * kMaxFineTiles);
 constexpr size_t kOffSurface = align256(kOffCoarseOff + 4 * kMaxCoarseTiles);
 constexpr size_t kOffView = align256(kOffSurface + sizeof(Surface));
 constexpr size_t kOffRec = align256(kOffView + sizeof(ViewParams));
@@ -215,11 +213,12 @@ extern "C" gbr_status gbr_render_view_noalloc(const gbr_device_scene* sc, const 
   }
 
   Workspace ws{};
-  ws.ctr = reinterpret_cast<Counters*>(base + kOffCtr);
-  ws.fine_count = reinterpret_cast<uint32_t*>(base + kOffFineCount);
+  ws.ctr = reinterpret_cast<Counters*>(base + kOffCounts);
+  ws.fine_count = reinterpret_cast<uint32_t*>(base + kOffCounts) + kCounterWords;
+  ws.ncounts = kCounterWords + nfine + ncoarse;
   ws.fine_off = reinterpret_cast<uint32_t*>(base + kOffFineOff);
   ws.nfine = nfine;
-  ws.coarse_count = reinterpret_cast<uint32_t*>(base + kOffCoarseCount);
+  ws.coarse_count = ws.fine_count + nfine;
   ws.coarse_off = reinterpret_cast<uint32_t*>(base + kOffCoarseOff);
   ws.ncoarse = ncoarse;
   ws.rec = reinterpret_cast<RasterRec*>(base + kOffRec);
@@ -244,12 +243,8 @@ extern "C" gbr_status gbr_render_view_noalloc(const gbr_device_scene* sc, const 
     e = (call);                                              \
     if (e != cudaSuccess) return nfail(GBR_CUDA_ERROR, what, e); \
   } while (0)
-  NA_CU(cudaMemcpyAsync(d_surf, &S, sizeof S, cudaMemcpyHostToDevice, s), "copy of the surface failed");
-  NA_CU(cudaMemcpyAsync(d_view, &V, sizeof V, cudaMemcpyHostToDevice, s), "copy of the view failed");
-  // everything that must start at zero: counters and tile counts
-  NA_CU(cudaMemsetAsync(ws.ctr, 0, sizeof(Counters), s), "clear failed");
-  NA_CU(cudaMemsetAsync(ws.fine_count, 0, 4 * (size_t)nfine, s), "clear failed");
-  NA_CU(cudaMemsetAsync(ws.coarse_count, 0, 4 * (size_t)ncoarse, s), "clear failed");
+  // the view's parameters, and everything that must start at zero: counters and tile counts
+  NA_CU(launch_begin_views(d, &V, &S, d_view, d_surf, 1, nullptr, ws, s), "begin launch failed");
   if (shade) {
     SceneDev obj = d;
     obj.objq = nullptr;
@@ -260,7 +255,7 @@ extern "C" gbr_status gbr_render_view_noalloc(const gbr_device_scene* sc, const 
           "texture table launch failed");
   }
   NA_CU(launch_setup_views(d, d_view, 1, d_surf, ws, s), "setup launch failed");
-  NA_CU(launch_scan(ws, s), "scan launch failed");
+  NA_CU(launch_offsets(ws, d_surf, 1, 0, s), "offsets launch failed");
   NA_CU(launch_fill(ws, d_surf, s), "fill launch failed");
   if (shade) NA_CU(launch_prep(d, ws, s), "shade constants launch failed");
   NA_CU(launch_raster(ws, d_surf, 1, nfine, true, kRasterThreads, s), "raster launch failed");

@@ -93,21 +93,22 @@ struct HostBuf {
 struct WorkMem {
   DevBuf<RasterRec> rec;
   DevBuf<ShadeRec> srec;
-  DevBuf<uint32_t> fine_count, fine_off, coarse_count, coarse_off, bins, scan_part;
+  DevBuf<uint32_t> counts;  // Counters, fine counts, coarse counts (kCounterWords)
+  DevBuf<uint32_t> fine_off, coarse_off, bins;
   DevBuf<uint8_t> tile_empty;  // views that shade: per fine tile, whether the raster wrote kernel3's output
-  DevBuf<uint2> tiles;         // per fine tile: surface, global coarse tile (Workspace::tiles)
-  DevBuf<Counters> ctr;
+  DevBuf<uint2> tiles;         // per fine tile (Workspace::tiles, or Workspace::list)
   DevBuf<uint32_t> pix_rec, pix_depth, pix_id;  // per view pixel
   DevBuf<uint8_t> pix_rgba;
   DevBuf<Surface> surf;
   DevBuf<ViewParams> views;
   DevBuf<ShadowJob> jobs;
+  std::vector<uint8_t> faces_held;  // the surfaces and jobs of the shadow pass as surf / jobs hold them
   DevBuf<uint32_t> sched, queue;  // fused raster -> shade pass: work order and queue words
   DevBuf<uint32_t> vis;           // views: object cull bits
   uint32_t rec_target = 0, bin_target = 0;
   void release() {
-    rec.release(); srec.release(); fine_count.release(); fine_off.release(); tile_empty.release(); tiles.release();
-    coarse_count.release(); coarse_off.release(); bins.release(); scan_part.release(); ctr.release();
+    rec.release(); srec.release(); counts.release(); fine_off.release(); tile_empty.release(); tiles.release();
+    coarse_off.release(); bins.release();
     pix_rec.release(); pix_depth.release(); pix_id.release(); pix_rgba.release();
     surf.release(); views.release(); jobs.release(); sched.release(); queue.release(); vis.release();
   }
@@ -291,16 +292,12 @@ inline bool pass_tile_table(bool view, const PassShape& sh) {
   return sh.nsurf > 1 && (view || !(sh.tiles_per_surface && sh.nsurf <= 65535 &&
                                     (uint64_t)sh.tiles_per_surface * sh.nsurf == sh.nfine));
 }
-// Kernel launches of one pass (for the launch statistics): views object
-// cull, setup, scan, fill, raster, and when shading the shade constants and
-// kernel3; depth-only passes clear, setup, scan, fill, raster; the tile
-// table when the pass needs it.  A scan over more than one chunk of fine
-// tiles is two kernels.
-// The fused raster -> shade pass is one kernel for two; pipelined groups are
-// two kernels per group.
-inline uint32_t pass_kernels(bool view, bool shade, uint32_t nfine, const PassShape* sh = nullptr) {
-  uint32_t k = (view ? (shade ? 7u : 5u) : 5u) + (scan_chunks(nfine) > 1 ? 1u : 0u);
-  if (sh && pass_tile_table(view, *sh)) k += 1;
+// Kernel launches of one pass (for the launch statistics): begin (clears and
+// object cull), setup, offsets, fill, raster, and when shading the shade
+// constants and kernel3.  The fused raster -> shade pass is one kernel for
+// two; pipelined groups are two kernels per group.
+inline uint32_t pass_kernels(bool view, bool shade, const PassShape* sh = nullptr) {
+  uint32_t k = view && shade ? 7u : 5u;
   if (sh && sh->nseg) k -= 1;
   if (sh && sh->ngroups > 1) k += 2 * (sh->ngroups - 1);
   return k;
