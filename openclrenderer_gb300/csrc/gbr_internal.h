@@ -69,7 +69,7 @@ struct __align__(16) ShadeRec {
 constexpr int kObjQuads = 4;
 
 // Per texture id, the atlas slot of each level (0 = the texture, 1..4 its
-// mips): (x, y) origin of the slot in its page, edge, page index (bits).
+// mips): (x, y) origin of the slot in its page (bits), edge, page index (bits).
 constexpr int kTexLevels = 1 + 4;
 
 // One raster target: a view, or one face of a shadow cubemap.

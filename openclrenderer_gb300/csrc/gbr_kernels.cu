@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(256) k_texture_levels(const uint32_t* __restri
   const uint32_t w = sizes[page];
   const uint32_t hnum = (uint32_t)kTexPage / w;
   const uint32_t row = which / hnum, col = which - row * hnum;
-  texlv[i] = make_float4((float)(col * w), (float)(row * w), (float)w, __uint_as_float(page));
+  texlv[i] = make_float4(__uint_as_float(col * w), __uint_as_float(row * w), (float)w, __uint_as_float(page));
 }
 
 // World-space vertices of a triangle, its object and the object's feature
@@ -1386,15 +1386,16 @@ __device__ __forceinline__ float u8f(uint32_t b) { return (float)(uint8_t)b; }
 // read_tex_array_all_precalculated (cl2.cl:823-851) in one atlas slot of the
 // texture level table: (ox, oy) is the slot origin in its page, tnum * width
 // in the reference, an integer below 2048 and so exact in float, which makes
-// fma(tnum, width, c) = ox + c.
+// its fma(tnum, width, c) = ox + c.
 struct TexSlot {
-  float ox, oy, width;
+  int ox, oy;
+  float width;
   const uchar4* page;
 };
 __device__ __forceinline__ TexSlot level_slot(const SceneDev& sc, float4 lv) {
   TexSlot t;
-  t.ox = lv.x;
-  t.oy = lv.y;
+  t.ox = __float_as_int(lv.x);
+  t.oy = __float_as_int(lv.y);
   t.width = lv.z;
   t.page = sc.atlas + (size_t)__float_as_uint(lv.w) * kTexPage * kTexPage;
   return t;
@@ -1405,19 +1406,14 @@ __device__ __forceinline__ f4 texel(const TexSlot& ts, int ix, int iy) {
   return r;
 }
 
-// The column (row) of a texel of the bilinear footprint at pos (+ 1 for the
-// second): the reference clamps the float coordinate to [0.001, w - 0.001]
-// and truncates o + c, o the slot origin.  pos is an integer-valued float
-// (floor), so that is o + clamp(pos, 0, w - 1) in integers: 0.001 truncates
-// to 0, w - 0.001 to w - 1 (o + w <= 2048 keeps o + w - 0.001 below o + w in
-// float), and a NaN coordinate clamps to 0.001, for both texels.
-__device__ __forceinline__ int texel_coord(float pos, int plus, int w) {
-  if (pos != pos) return 0;
-  const int p = min((int)pos, w) + plus;  // saturating conversion; below INT_MAX after the min
-  return min(max(p, 0), w - 1);
-}
-
-// The four texels of a bilinear footprint and its weights.
+// The four texels of a bilinear footprint at (mx, my) of a slot, and its
+// weights.  The reference clamps the float coordinates floor(m) and floor(m) +
+// 1 to [0.001, w - 0.001] and truncates o + c, o the slot origin: in integers
+// that is o + clamp(floor(m), 0, w - 1) (0.001 truncates to 0, w - 0.001 to w
+// - 1; o + w <= 2048 keeps o + w - 0.001 below o + w in float).  Coordinates
+// come from texture_mod, so floor(m) is not negative; the conversion and the
+// clamps keep any other in the slot all the same, and a NaN, whose weights
+// make the result NaN whatever the texels are.
 struct Footprint {
   int x0, x1, y0, y1;
   float ux, uy;
@@ -1425,9 +1421,10 @@ struct Footprint {
 __device__ __forceinline__ Footprint footprint_at(const TexSlot& ts, float mx, float my) {
   Footprint f;
   const float posx = floorf(mx), posy = floorf(my);
-  const int w = (int)ts.width, ox = (int)ts.ox, oy = (int)ts.oy;
-  f.x0 = ox + texel_coord(posx, 0, w), f.x1 = ox + texel_coord(posx, 1, w);
-  f.y0 = oy + texel_coord(posy, 0, w), f.y1 = oy + texel_coord(posy, 1, w);
+  const int w = (int)ts.width;
+  const int px = __vimin_s32_relu((int)posx, w), py = __vimin_s32_relu((int)posy, w);
+  f.x0 = ts.ox + min(px, w - 1), f.x1 = ts.ox + __viaddmin_s32(px, 1, w - 1);
+  f.y0 = ts.oy + min(py, w - 1), f.y1 = ts.oy + __viaddmin_s32(py, 1, w - 1);
   f.ux = mx - posx, f.uy = my - posy;
   return f;
 }
@@ -1571,7 +1568,10 @@ __device__ float generate_ssao(int x, int y, uint32_t seed2, uint32_t d, const u
     acc = 25 * (int)(ssao_tap(__ldca(depth + (size_t)ssao_coord_int(y, 0, H) * W + ssao_coord_int(x, 0, W)), c8) -
                      kSsaoTapZero);
   } else {
-    const int i1 = min((int)roundf(world_rad), 8192), i2 = min((int)roundf(2.0f * world_rad), 8192);  // views: < 4096
+    // roundf of a value >= 0: the truncation of v + 0.5, that sum rounded toward
+    // zero (it never passes an integer).  Views are below 4096.
+    const int i1 = min(__float2int_rz(__fadd_rz(world_rad, 0.5f)), 8192);
+    const int i2 = min(__float2int_rz(__fadd_rz(2.0f * world_rad, 0.5f)), 8192);
     const int off[5] = {-i2, -i1, 0, i1, i2};
     int wx[5];
 #pragma unroll
@@ -1593,10 +1593,9 @@ __device__ float generate_ssao(int x, int y, uint32_t seed2, uint32_t d, const u
 
 // generate_hard_occlusion (cl2.cl:2536-2701), SMOOTH_SHADOWS.  Inlined: as
 // a call it cost kernel3 spills around it (1080p kernel3 0.236 -> 0.233 ms
-// inlined)
-__device__ __forceinline__ float hard_occlusion(const SceneDev& sc, f3 lpos, f3 normal, f3 ptl, const uint32_t* buf,
-                                int face, f3 gpos, int shnum) {
-  ptl = fast_normalize3(ptl);
+// inlined).  ptl: pixel to light, rinv: its approximate reciprocal length.
+__device__ __forceinline__ float hard_occlusion(const SceneDev& sc, f3 lpos, f3 normal, f3 ptl, float rinv,
+                                                const uint32_t* buf, int face, f3 gpos, int shnum) {
   f3 c = mk3(sc.face_cos[face][0], sc.face_cos[face][1], sc.face_cos[face][2]);
   f3 s = mk3(sc.face_sin[face][0], sc.face_sin[face][1], sc.face_sin[face][2]);
   f3 local = rot_cs(gpos, lpos, c, s);
@@ -1606,16 +1605,32 @@ __device__ __forceinline__ float hard_occlusion(const SceneDev& sc, f3 lpos, f3 
   float px = clampf_(post.x, 3.0f, kLightBufferDim - 4.0f);
   float py = clampf_(post.y, 3.0f, kLightBufferDim - 4.0f);
   int ix = f2i_sat(px), iy = f2i_sat(py);
-  float acos_res = rational_acos(clampf_(dot3(normal, ptl), 0.05f, 0.95f));
-  float bias = clampf_(kShadowBias * gbr_tanf(acos_res), 0.1f * kShadowBias, kShadowBias);
-  uint32_t cond = 0;  // bit (yy+1)*4 + (xx+1)
+  // The bias is 50 tan(angle of incidence), at most 50: with the cosine below
+  // kBiasFullCos it is 50 whatever the cosine is, so neither the exact unit
+  // vector nor its arc cosine and tangent are needed.
+  float bias = kShadowBias;
+  if (!(dot3(normal, ptl) * rinv <= kBiasFullCos - 0.01f)) bias = shadow_bias(dot3(normal, fast_normalize3(ptl)));
+  // The taps' test dpth > depth_to_dist(d) + bias in depth units: it holds
+  // below lo and fails above hi; a tap between them (next to none) has all of
+  // them tested as they stand.
+  uint32_t lo, hi;
+  const bool limits = shadow_limits(dpth, bias, &lo, &hi);
+  const uint32_t* row = map + (iy - 1) * kLightBufferDim + ix - 1;
+  uint32_t cond = 0, near = 0xFFFFFFFFu;  // bit (yy+1)*4 + (xx+1)
 #pragma unroll
-  for (int yy = -1; yy <= 2; yy++)
-#pragma unroll
-    for (int xx = -1; xx <= 2; xx++) {
-      float ldp = depth_to_dist(__ldg(map + (iy + yy) * kLightBufferDim + ix + xx));
-      if (dpth > ldp + bias) cond |= 1u << ((yy + 1) * 4 + xx + 1);
+  for (int k = 0; k < 16; k++) {
+    const uint32_t d = __ldg(row + (k >> 2) * kLightBufferDim + (k & 3));
+    if (d < lo) cond |= 1u << k;
+    near = min(near, d - lo);
+  }
+  if (near <= hi - lo || !limits) {
+    cond = 0;
+#pragma unroll 1
+    for (int k = 0; k < 16; k++) {
+      const float ldp = depth_to_dist(__ldg(row + (k >> 2) * kLightBufferDim + (k & 3)));
+      if (dpth > ldp + bias) cond |= 1u << k;
     }
+  }
   // The 3x3 bilinear blend of the 4x4 tests: every tap has the same
   // fractional offsets (ux, uy), so the sum of the nine bilinear_interpolate
   // calls is separable, with column weights (1 - ux, 1, 1, ux) and row
@@ -1719,14 +1734,17 @@ constexpr float kLightCutoff = 0.1f;
 // margins below cover the approximate colour-path arithmetic of that test
 // (relative errors of a few 1e-7).  -1: always under the cutoff; +inf: no
 // early test (shadow lights, whose cutoff decides the cubemap later shadow
-// lights read, and degenerate radii).
+// lights read); the largest float: only infinite distances (degenerate radii,
+// whose attenuation is then under the cutoff too).  A NaN position makes the
+// reciprocal radius NaN, and with it the attenuation.
 constexpr int kLightQuads = 3;
 __device__ __forceinline__ void stage_light(const gbr_light* L, bool linear, float4* dst) {
   f3 c = mk3(L->col[0], L->col[1], L->col[2]);
   if (linear) c = mk3(gamma_fwd(c.x), gamma_fwd(c.y), gamma_fwd(c.z));
   const float radius = L->radius, brightness = L->brightness;
   const float b10 = 10.0f * brightness;
-  float cut2 = __int_as_float(0x7F800000);
+  float cut2 = L->shadow ? __int_as_float(0x7F800000) : 3.4028235e38f;
+  const float psum = L->pos[0] + L->pos[1] + L->pos[2];
   if (!L->shadow && radius > 0.0f && b10 == b10) {
     if (b10 <= 1.0f) {
       cut2 = -1.0f;
@@ -1740,7 +1758,7 @@ __device__ __forceinline__ void stage_light(const gbr_light* L, bool linear, flo
   const float bw = L->shadow ? brightness : brightness * (1.0f / (1.0f - kLightCutoff));
   dst[0] = make_float4(L->pos[0], L->pos[1], L->pos[2], cut2);
   dst[1] = make_float4(c.x, c.y, c.z, bw);
-  dst[2] = make_float4(radius, __fdividef(1.0f, radius), L->diffuse,
+  dst[2] = make_float4(radius, psum == psum ? __fdividef(1.0f, radius) : psum, L->diffuse,
                        __uint_as_float((L->shadow ? 1u : 0u) | (L->is_static ? 2u : 0u)));
 }
 
@@ -1969,7 +1987,7 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
       float occlusion = 1.0f;
       if (lflags & 2u) {  // is_static
         int face = ret_cubeface(gpos, lpos);
-        occlusion = 1.0f - hard_occlusion(sc, lpos, normal, ptl, sc.shadow_static, face, gpos, static_num);
+        occlusion = 1.0f - hard_occlusion(sc, lpos, normal, ptl, rinv, sc.shadow_static, face, gpos, static_num);
         static_num++;
       }
       const float tt = fdiv(fsqrt(d2s), LC.x) + 1.0f;
@@ -1979,7 +1997,7 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
       if (illum <= 0) continue;
       if (recv_dyn) {
         int face = ret_cubeface(gpos, lpos);
-        float dyn = 1.0f - hard_occlusion(sc, lpos, normal, ptl, sc.shadow_dyn, face, gpos, shnum);
+        float dyn = 1.0f - hard_occlusion(sc, lpos, normal, ptl, rinv, sc.shadow_dyn, face, gpos, shnum);
         occlusion = fmin_(occlusion, dyn);
         shnum++;
       }
@@ -2007,11 +2025,14 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
       continue;
     }
     // a light without shadows: its occlusion is 1
-    // the approximate square root; 0, +inf and NaN are their own square roots
-    const float distance = (d2 > 0.0f && d2 <= 3.4028235e38f) ? d2 * rinv : d2;
+    // the approximate square root (0 * inf is NaN, which the maximum turns into
+    // 0; infinite distances are past every cut2)
+    const float distance = fmax_(d2 * rinv, 0.0f);
     const float tt = fma_(distance, LC.y, 1.0f);
-    const float illum = fma_(LB.w, crcp(tt * tt), -kLightCutoff / (1.0f - kLightCutoff));
-    if (illum <= 0) continue;
+    float illum = fma_(LB.w, crcp(tt * tt), -kLightCutoff / (1.0f - kLightCutoff));
+    // at most 0 only between the cutoff and the conservative early test: such a
+    // light then adds exactly nothing (a select, not another divergent exit)
+    illum = illum <= 0.0f ? 0.0f : illum;
     ptl = mul3s(ptl, rinv);
     const float light = fmax_(cdot3(ptl, lnormal), 0.0f);
     const float dscale = fma_(amb1, light, ambient) * ((LC.z * g_diffuse) * illum);
@@ -2024,10 +2045,11 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
     const float vdh = fmax_(0.0f, (1.0f + vl) * rh);
     const float ndh = fmax_(0.0f, (ndv_raw + nl) * rh);
     const float ndl = fmax_(0.0f, nl);
+    const float alpha = c_rational_acos(ndh);
+    const float ex = ((alpha * alpha) * nr2) * 1.4426950408889634f;
+    const float microfacet = 0.8346f * ex2_ftz(ex);
     const float omv = 1.0f - vdh, omv2 = omv * omv;
     const float fresnel = fma_(0.6f, (omv2 * omv2) * omv, 0.4f);
-    const float alpha = c_rational_acos(ndh);
-    const float microfacet = 0.8346f * ex2_ftz(((alpha * alpha) * nr2) * 1.4426950408889634f);
     const float sv = (2.0f * ndh) * crcp(vdh);
     const float geometric = min3f(1.0f, sv * ndv, sv * ndl);
     const float spec = ((fresnel * microfacet) * geometric) * r_pndv;
@@ -2125,10 +2147,10 @@ __device__ __forceinline__ void shade_tile(const SceneDev& sc, const ViewParams*
   }
 }
 
-// 1080p terrain: 2,760 instructions per pixel (3,350 before the
+// 1080p terrain: 2,690 instructions per pixel (3,350 before the
 // approximations as single instructions, the SSAO counts without compares,
-// packed texel blends and the view in the constant bank), 187 us (223); 64
-// sphere views 2.18 ms (2.62).  It is bound by instruction issue (77 %
+// packed texel blends, integer texel coordinates and the view in the constant
+// bank), 183 us (223); 64 sphere views 2.13 ms (2.62).  It is bound by instruction issue (77 %
 // active).  The lights' shared memory is sized by the scene: with room for
 // kMaxLights the L1 lost 3 points of its hit rate (1.4 % of the batch's time).
 // Tiles of 128 or 64 pixels per block were slower (203 / 212 us): their
@@ -2197,13 +2219,9 @@ __global__ void __launch_bounds__(kTilePixels, 4) k_shade(SceneDev sc,
       s_rowy[i] = fdiv((float)(y0 + i) - (float)S.height / 2.0f, V.fov);
   }
   __syncthreads();
-  uint32_t base = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < NW; w++) {
-    const uint32_t c = s_warp[w];
-    base += w < warp ? c : 0u;
-    total += c;
-  }
+  const uint32_t wc = lane < NW ? s_warp[lane] : 0u;
+  const uint32_t base = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wc : 0u);
+  const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, wc);
   if (cov) {
     const uint32_t k = base + __popc(m & ((1u << lane) - 1u));
     s_px[k] = (uint32_t)lp;

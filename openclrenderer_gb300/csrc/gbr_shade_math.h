@@ -49,4 +49,25 @@ GBR_HD bool ssao_exact(float dep) {
   return dep >= 8.0f && (dep + 1.0f) - dep == 1.0f && (dep + 2.0f) - dep == 2.0f;
 }
 
+// The shadow bias of generate_hard_occlusion for a cosine of incidence (cl2.cl:2604-2608).
+GBR_HD float shadow_bias(float cosine) {
+  const float acos_res = rational_acos(clampf_(cosine, 0.05f, 0.95f));
+  return clampf_(kShadowBias * gbr_tanf(acos_res), 0.1f * kShadowBias, kShadowBias);
+}
+// shadow_bias is kShadowBias for every cosine up to this one (checked for
+// every float of its range): beyond 45 degrees the tangent exceeds 1.
+constexpr float kBiasFullCos = 0.70f;
+
+// Limits of a shadow tap's test dpth > depth_to_dist(d) + bias (bias at most
+// 50): true for every d < *lo, false for every d > *hi.  The limit is dpth -
+// bias in depth units; 10 * 2^-24 of dpth to either side cover the at most 7
+// roundings of the two forms.  Returns false where the limit is near the end
+// of the range and says nothing.
+GBR_HD bool shadow_limits(float dpth, float bias, uint32_t* lo, uint32_t* hi) {
+  const float lim = dpth - bias, slack = dpth * 6e-7f;
+  *lo = f2u_sat((lim - slack) * (kMulInt / kDepthFar));
+  *hi = f2u_sat((lim + slack) * (kMulInt / kDepthFar));
+  return lim < 349000.0f;
+}
+
 }  // namespace gbr

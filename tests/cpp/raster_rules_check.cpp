@@ -2,8 +2,9 @@
 // for: walk_first_late_row against walk_row_late over every width <= W, top
 // row < H and row (a row before it must not be late), and box_bounds against
 // depth_at and edge_inside at every pixel of random triangles' boxes; tight_box
-// against edge_inside at every pixel of their bbox4; and ssao_tap against
-// ssao_count wherever ssao_exact holds.
+// against edge_inside at every pixel of their bbox4; ssao_tap against ssao_count
+// wherever ssao_exact holds; shadow_bias below kBiasFullCos; and shadow_limits
+// against the test they bracket.
 // Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
 #include <cmath>
 #include <cstdio>
@@ -112,6 +113,26 @@ int main(int argc, char** argv) {
                (uint32_t)ssao_count(depth_scaled(d), t[0], t[1], t[2], t[3], t[4]);
     }
   }
+  // every cosine up to kBiasFullCos has the full bias
+  long cosines = 0;
+  for (float c = 0.05f; c <= kBiasFullCos; c = nextafterf(c, 2.0f)) cosines += shadow_bias(c) != kShadowBias;
+  long shadow = 0;
+  for (int i = 0; i < n; i++) {
+    const float dpth = (i & 3) ? powf(10.0f, uni(-3.0f, 5.54f)) : uni(0.0f, 120.0f), bias = uni(5.0f, 50.0f);
+    uint32_t lo, hi;
+    if (!shadow_limits(dpth, bias, &lo, &hi)) continue;
+    for (int k = 0; k < 24; k++) {
+      const uint32_t near = (k & 1) ? lo : hi, step = 1u << (rng() % 12);
+      uint32_t d = (k & 2) ? near + rng() % step : near - rng() % step;
+      if (k == 20) d = 0;
+      if (k == 21) d = kDepthClear;
+      if (k > 21) d = rng();
+      const bool t = dpth > depth_to_dist(d) + bias;
+      shadow += (d < lo && !t) || (d > hi && t);
+    }
+  }
+  printf("cosines=%ld shadow=%ld\n", cosines, shadow);
+  bad += cosines + shadow;
   printf("taps=%ld inexact=%ld wrong=%ld\n", taps, inexact, wrong);
   bad += wrong;
   printf("early=%ld late=%ld boxes=%d full=%ld bounded=%ld bad=%ld\n", early, late, n, full, bounded, bad);
