@@ -32,17 +32,20 @@ constexpr int kFineMaxTiles = 16;            // more fine tiles than this -> coa
 constexpr int kRasterThreads = 128;  // threads of one raster CTA (default tuning)
 constexpr int kMaxLights = 256;              // lights a scene may hold (staged in shared memory)
 
+constexpr uint32_t kRecTight = 1u;   // the box is tight_box's: one column and row less than bbox4
+constexpr uint32_t kRecInside = 2u;  // on_surface: rows can be narrowed to spans
+
 // Per visible clipped triangle on one surface: everything kernel1/kernel2
 // need per pixel, precomputed once (64 bytes).
 struct __align__(16) RasterRec {
   float A, B, C, bound;  // depth plane; (2.0001*area)*sign
-  float s0, sa, sb, sign;
+  float s0, sa, sb, unused;  // the coverage test's terms, times its sign
   float t0, ta, tb;
   uint32_t key;          // views: 2*triangle + clip sub-index (canonical id)
   uint32_t xr;           // minx | maxx << 16
   uint32_t yr;           // miny | maxy << 16
   uint32_t surface;
-  uint32_t tight;        // the box is tight_box's: one column and row less than bbox4
+  uint32_t kind;         // kRec*
 };
 
 // Per visible clipped triangle of a view: kernel3's per-triangle constants,

@@ -39,6 +39,30 @@ __device__ __forceinline__ uint32_t agg_inc(uint32_t* counter, uint32_t key, boo
   return res;
 }
 
+// Colour-only arithmetic of the light loop: every use below feeds the colour
+// continuously (no comparison, rounding or index depends on it), so the
+// approximate division is covered by the 1/255 colour tolerance.  The
+// hardware's approximations, taken as single instructions: __fdividef,
+// rsqrtf and __expf compute the same values but wrap them in three or four
+// more for subnormal operands and results, which here are either exact zeros
+// or far below a colour level.  (1080p kernel3 3,350 -> 3,060 instructions
+// per pixel, 223 -> 210 us.)
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float crcp(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return r;
+}
+
 // A visible clipped triangle before it becomes a record.  (The second
 // triangle of a split at the near clip, which is rare, is made after the first
 // one is done with, so that only one is held at a time.)
@@ -47,6 +71,7 @@ struct Cand {
   float mm[4];  // bbox4, or the smaller box of tight_box
   float area;   // of bbox4
   int box;      // tight_box
+  bool inside;  // on_surface
   uint32_t key;
 };
 
@@ -65,6 +90,7 @@ __device__ __forceinline__ bool cull_candidate(Cand& c, bool two_sided, float w,
   bbox4(p[0], p[1], p[2], w, h, c.mm);
   c.area = (c.mm[1] - c.mm[0]) * (c.mm[3] - c.mm[2]);
   c.box = tight_box(xpv, ypv, w, h, c.mm);
+  c.inside = on_surface(xpv, ypv, w, h);
   return c.area > 0.0f;
 }
 
@@ -78,22 +104,24 @@ __device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, Raster
   *rc = rconstant(xpv, ypv);
   plane_const(depths, xpv, ypv, *rc, &R.A, &R.B, &R.C);
   EdgeTest e = make_edge(xpv.x, ypv.x, xpv.y, ypv.y, xpv.z, ypv.z);
-  R.s0 = e.s0; R.sa = e.sa; R.sb = e.sb; R.sign = e.sign;
-  R.t0 = e.t0; R.ta = e.ta; R.tb = e.tb; R.bound = e.bound;
+  // (a sign change commutes with rounding: the sign is folded in)
+  R.s0 = e.s0 * e.sign; R.sa = e.sa * e.sign; R.sb = e.sb * e.sign;
+  R.t0 = e.t0 * e.sign; R.ta = e.ta * e.sign; R.tb = e.tb * e.sign;
+  R.bound = e.bound;
   R.key = c.key;
   R.xr = (uint32_t)c.mm[0] | ((uint32_t)c.mm[1] << 16);
   R.yr = (uint32_t)c.mm[2] | ((uint32_t)c.mm[3] << 16);
   R.surface = surface;
-  R.tight = c.box == kBoxTight ? 1u : 0u;
+  R.kind = (c.box == kBoxTight ? kRecTight : 0u) | (c.inside ? kRecInside : 0u);
 }
 
 __device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& R) {
   float4* d = reinterpret_cast<float4*>(dst);
   d[0] = make_float4(R.A, R.B, R.C, R.bound);
-  d[1] = make_float4(R.s0, R.sa, R.sb, R.sign);
+  d[1] = make_float4(R.s0, R.sa, R.sb, 0.0f);
   d[2] = make_float4(R.t0, R.ta, R.tb, __uint_as_float(R.key));
   d[3] = make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), __uint_as_float(R.surface),
-                     __uint_as_float(R.tight));
+                     __uint_as_float(R.kind));
 }
 
 // Tile footprint of a record: inclusive fine tiles, or coarse tiles when its
@@ -106,7 +134,8 @@ struct Foot {
   bool coarse;
 };
 __device__ __forceinline__ int foot_count(const Foot& f) { return (f.tx1 - f.tx0 + 1) * (f.ty1 - f.ty0 + 1); }
-__device__ __forceinline__ Foot footprint(uint32_t xr, uint32_t yr, uint32_t tight, const Workspace& ws, int* ref) {
+__device__ __forceinline__ Foot footprint(uint32_t xr, uint32_t yr, uint32_t kind, const Workspace& ws, int* ref) {
+  const uint32_t tight = kind & kRecTight;
   const int minx = xr & 0xFFFF, maxx = xr >> 16, miny = yr & 0xFFFF, maxy = yr >> 16;
   int bx0 = (minx - (int)tight) >> 4, by0 = max(miny - (int)tight, 0) >> 4;  // tight: minx >= 1
   Foot f;
@@ -203,12 +232,10 @@ __device__ __forceinline__ void each_coarse_tile(const Foot& f, bool coarse, con
   }
 }
 
-// point_in_tri of a record at pixel (px, py).
-__device__ __forceinline__ bool rec_in_tri(const float4 q[3], int px, int py) {
-  float fx = (float)px, fy = (float)py;
-  float sgn = q[1].w;
-  float s = ((q[1].x + q[1].y * fx) + q[1].z * fy) * sgn;
-  float t = ((q[2].x + q[2].y * fx) + q[2].z * fy) * sgn;
+// point_in_tri of a record at pixel (fx, fy).
+__device__ __forceinline__ bool rec_in_tri(const float4 q[3], float fx, float fy) {
+  const float s = (q[1].x + q[1].y * fx) + q[1].z * fy;
+  const float t = (q[2].x + q[2].y * fx) + q[2].z * fy;
   return s > -0.0001f && t > -0.0001f && (s + t) < q[0].w;
 }
 
@@ -271,21 +298,20 @@ __device__ __forceinline__ uint32_t direct_raster(const Cand& c, uint32_t surfac
   RasterRec R;
   float rc;
   make_rec(c, surface, R, &rc);
-  const float4 q[4] = {make_float4(R.A, R.B, R.C, R.bound), make_float4(R.s0, R.sa, R.sb, R.sign),
-                       make_float4(R.t0, R.ta, R.tb, __uint_as_float(R.key)),
-                       make_float4(__uint_as_float(R.xr), __uint_as_float(R.yr), 0.0f, 0.0f)};
+  const float4 q[3] = {make_float4(R.A, R.B, R.C, R.bound), make_float4(R.s0, R.sa, R.sb, 0.0f),
+                       make_float4(R.t0, R.ta, R.tb, 0.0f)};
   const int x0 = (int)(R.xr & 0xFFFF), x1 = (int)(R.xr >> 16), y0 = (int)(R.yr & 0xFFFF), y1 = (int)(R.yr >> 16);
   uint32_t hits = 0;
   // row by row: the walk rule of the row's left-column pixel, then point_in_tri
   // (walk_skip_rows: 0 at once unless the bbox touches the top of the face;
   // a bbox of at most 64 pixels has at most 64 rows)
   uint64_t skip = 0;
-  if (!R.tight)
+  if (!(R.kind & kRecTight))
     skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, S.chunk) |
            ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, S.chunk) << 32);
   for (int y = y0; y < y1; y++) {
     for (int x = x0 + (int)((skip >> (y - y0)) & 1u); x < x1; x++)
-      if (rec_in_tri(q, x, y)) {
+      if (rec_in_tri(q, (float)x, (float)y)) {
         atomicMin(S.depth + (size_t)y * S.width + x, depth_at(R.A, R.B, R.C, (float)x, (float)y));
         hits++;
       }
@@ -351,7 +377,7 @@ __device__ __forceinline__ void emit(const Cand& c, bool act, uint32_t surface, 
   if (rec) {
     int ref;
     f = footprint((uint32_t)c.mm[0] | ((uint32_t)c.mm[1] << 16), (uint32_t)c.mm[2] | ((uint32_t)c.mm[3] << 16),
-                  c.box != kBoxAny ? 1u : 0u, ws, &ref);
+                  c.box != kBoxAny ? kRecTight : 0u, ws, &ref);
     cnt.vis++;
     cnt.bins += (uint32_t)ref;
   }
@@ -905,28 +931,34 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 //
 // The tile's records (its fine bin, then its coarse tile's bin) are staged NT
 // at a time in shared memory, keeping those whose bbox meets the tile.  Each
-// contributes the horizontal pixel pairs of its bbox clipped to the tile (a
-// test covers one pair: the record's loads and decode serve two pixels); one
-// block scan (packing the record count and the pair count) compacts them and
-// lays all (record, pair) tests of the chunk end to end.  Each warp takes one
-// contiguous range of that list, finds its first record by binary search,
-// and then maps 32 tests at a time to records with one ballot of the record
-// starts inside the window (every staged record has at least one pair, so
-// at most 32 start there), so small and large triangles are load-balanced
-// alike.  Pass 0 resolves the minimum depth with shared-memory atomicMin;
-// pass 1 the minimum packed (key << 32 | record) among tests within +-20 of
-// the final depth.  Both are minima, so neither bin order nor thread order
-// changes the result.  Pass 0 keeps its covered pixels in a list per warp
-// (kHitCap, compacted in place when it fills: an entry 20 or more behind the
-// pixel's depth so far never passes), and pass 1 runs over those lists; only a
-// tile whose lists overflow all the same tests its records again.
+// contributes the rows of its bbox in the tile; one block scan (packing the
+// record count and the row count) compacts the records and lays all rows of
+// the chunk end to end.  Each warp takes one contiguous share of that list, 32
+// rows at a time: it maps rows to records with one ballot of the record starts
+// inside the window (every staged record has a row, so at most 32 start
+// there), narrows each lane's row to the span that the three edges leave
+// (row_span; for records with vertices off the surface the row stays whole),
+// and lays the spans' horizontal pixel pairs end to end in turn.  Those are
+// tested 32 at a time, mapped to spans as rows are to records: a pair costs
+// one decode and record load for two exact tests, and small, large and thin
+// triangles are load-balanced alike.  Pass 0 resolves the minimum depth with
+// shared-memory atomicMin; pass 1 the minimum packed (key << 32 | record)
+// among tests within +-20 of the final depth.  Both are minima, so neither bin
+// order nor thread order changes the result.  Pass 0 keeps its covered pixels
+// in a list per warp (kHitCap, compacted in place when it fills: an entry 20
+// or more behind the pixel's depth so far never passes), and pass 1 runs over
+// those lists; only a tile whose lists overflow all the same tests its records
+// again.
 //
 // Measured (launch alone, before -> now; bound by instruction issue, 72 %
 // active, and by the barriers between chunks): 1080p terrain 114 -> 81 us, 9
 // ragged views of a 500k-triangle scene 689 -> 431 us (tiles of several chunks
 // no longer stage and test everything twice; the walk rule costs a comparison
 // per record), 2560x1440 under 1,000 screen-covering triangles 22.4 -> 0.43 ms
-// (the depth cull at staging).
+// (the depth cull at staging).  Then tight boxes and fewer records: 69 us
+// (terrain).  Rows narrowed to spans instead of all pairs of the bbox: 64
+// sphere views 1.01 -> 0.97 ms, 4K 210 -> 191 us, cube faces with large walls
+// 141 -> 121 us, 1080p terrain 68 -> 67 us.
 constexpr int kHitCap = 256;  // entries of a warp's list: about 100 are used in a tile of 1.2 layers
 // 512-thread CTAs keep no lists (their static shared memory stays under 48 KB)
 // and re-test in the id pass.
@@ -1007,13 +1039,18 @@ __device__ __noinline__ uint32_t compact_hits(uint2* hits, uint32_t n, const uin
   return kept;
 }
 
+// Spans a warp holds at once: fewer than 32 that wait, and those of 32 rows.
+constexpr uint32_t kSpanRing = 64;
+
 // Shared memory of one tile's raster (NT threads; ID: views).
 template <int NT, bool ID>
 struct RasterSmem {
   float4 srec[3][NT];  // the staged records' first three float4, one array each (conflict-free stores)
   uint32_t sidx[NT];
   uint32_t soff[NT + 1];
-  uint32_t sgeo[NT];  // lx0 | ly0 << 4 | bw << 8 | ceil(65536 / pairs per row) << 13
+  uint32_t sgeo[NT];   // lx0 | ly0 << 4 | bw << 8 | kRecTight << 13 | kRecInside << 13
+  float2 sinv[NT];     // reciprocal x slopes of t and of bound - s - t (that of s: srec[1].w)
+  uint2 spans[NT / 32][kSpanRing];  // per warp: spans of rows that can be covered
   // bit ly: the walk skips the record's left-column pixel in tile row ly (0
   // when that column lies left of the tile)
   uint16_t sskip[NT];
@@ -1176,7 +1213,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       }
       if (!(resident && pass == 1)) {
         if (pass != 0 || c0 != 0) __syncthreads();  // the previous chunk's readers are done
-        uint32_t area = 0, r = 0, geo = 0, skip = 0;
+        uint32_t rows = 0, r = 0, geo = 0, skip = 0;
         int bx0 = 0, bx1 = 0, by0 = 0, by1 = 0;
         float4 q0, q1, q2, q3;
         if ((uint32_t)tid < m) {
@@ -1191,13 +1228,12 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           bx0 = max((int)(xr & 0xFFFF), tx0), bx1 = min((int)(xr >> 16), tx0 + kTile);
           by0 = max((int)(yr & 0xFFFF), ty0), by1 = min((int)(yr >> 16), ty0 + kTile);
           if (bx1 > bx0 && by1 > by0) {
-            // the tests are horizontal pixel pairs: ceil(bw / 2) per row
-            const uint32_t bw = (uint32_t)(bx1 - bx0), pw = (bw + 1) >> 1;
-            area = pw * (uint32_t)(by1 - by0);
-            geo = (uint32_t)(bx0 - tx0) | ((uint32_t)(by0 - ty0) << 4) | (bw << 8) | (((65536u + pw - 1) / pw) << 13);
+            const uint32_t kind = __float_as_uint(q3.w);
+            rows = (uint32_t)(by1 - by0);
+            geo = (uint32_t)(bx0 - tx0) | ((uint32_t)(by0 - ty0) << 4) | ((uint32_t)(bx1 - bx0) << 8) | (kind << 13);
             // the walk rule of the bbox's left column, once per row of this
             // tile (a tight box has left that column out)
-            if ((int)(xr & 0xFFFF) >= tx0 && !__float_as_uint(q3.w)) skip = walk_skip_rows(xr, yr, by0, by1, ty0, chunk);
+            if ((int)(xr & 0xFFFF) >= tx0 && !(kind & kRecTight)) skip = walk_skip_rows(xr, yr, by0, by1, ty0, chunk);
           }
         }
         // Depth cull.  A record that covers every coverable pixel of the tile
@@ -1208,14 +1244,14 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
         // comes from the chunks before this one and the warp's own records.
         // (Coverable: a bbox ends at the surface's last column and row, which
         // stay clear.)
-        const bool whole = area && bx0 == tx0 && by0 == ty0 && bx1 == min(tx0 + kTile, S.width - 1) &&
+        const bool whole = rows && bx0 == tx0 && by0 == ty0 && bx1 == min(tx0 + kTile, S.width - 1) &&
                            by1 == min(ty0 + kTile, S.height - 1) && !skip;
         uint32_t zcap = __shfl_sync(0xFFFFFFFFu, sm.szcap, 0);
         if (__any_sync(0xFFFFFFFFu, whole) || zcap != kDepthClear) {
           bool full = false;
           uint32_t dlo = 0, dhi = kDepthClear;
-          if (area)
-            full = box_bounds(q0.x, q0.y, q0.z, EdgeTest{q1.x, q1.y, q1.z, q2.x, q2.y, q2.z, q1.w, q0.w}, bx0, by0,
+          if (rows)
+            full = box_bounds(q0.x, q0.y, q0.z, EdgeTest{q1.x, q1.y, q1.z, q2.x, q2.y, q2.z, 1.0f, q0.w}, bx0, by0,
                               bx1 - 1, by1 - 1, &dlo, &dhi);
           const uint32_t bound = __reduce_min_sync(0xFFFFFFFFu, full && whole ? dhi : kDepthClear);
           if (bound < zcap) {
@@ -1225,18 +1261,19 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           uint32_t hidden = 0;
           if (full && zcap < kDepthClear - kBufError && dlo >= zcap + kBufError) {
             hidden = (uint32_t)((bx1 - bx0) * (by1 - by0)) - (uint32_t)__popc(skip);
-            area = 0;
+            rows = 0;
           }
           if (pass == 0) wsamples += __reduce_add_sync(0xFFFFFFFFu, hidden);
         }
-        const uint32_t word = area ? (area | (1u << kCountShift)) : 0u;
+        const uint32_t word = rows ? (rows | (1u << kCountShift)) : 0u;
         uint32_t tot = 0;
         const uint32_t off = block_excl_scan1<NT>(word, swarp, &tot);
-        if (area) {
+        if (rows) {
           const uint32_t slot = off >> kCountShift;
           srec[0][slot] = q0;
-          srec[1][slot] = q1;
+          srec[1][slot] = make_float4(q1.x, q1.y, q1.z, span_slope(q1.y));
           srec[2][slot] = q2;
+          sm.sinv[slot] = make_float2(span_slope(q2.y), span_slope(-(q1.y + q2.y)));
           sidx[slot] = r;
           sgeo[slot] = geo;
           sskip[slot] = (uint16_t)skip;
@@ -1250,73 +1287,110 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       }
       const uint32_t nstaged = sscan >> kCountShift;
       const uint32_t total = soff[nstaged];
-      // this warp's contiguous range of the test list, in windows of 32
-      const uint32_t per = ((total + NW * 32 - 1) / (NW * 32)) * 32;
+      // this warp's contiguous share of the row list, in windows of 32 (a
+      // few rows may hold many pixels: shares are equal, not whole windows)
+      const uint32_t per = (total + NW - 1) / NW;
       const uint32_t start = min(total, (uint32_t)warp * per), end = min(total, start + per);
       if (start < end) {
-        // first record: the last staged record with soff <= start (warp-uniform)
-        int rec = 0, hi = (int)nstaged - 1;
-        while (rec < hi) {
-          const int mid = (rec + hi + 1) >> 1;
-          if (soff[mid] <= start) rec = mid; else hi = mid - 1;
-        }
+        // first record: the last staged record with soff <= start (warp-uniform;
+        // soff increases, so that is their number)
+        int rec = -1;
+        for (uint32_t k = lane; k < nstaged + lane; k += 32)
+          rec += __popc(__ballot_sync(0xFFFFFFFFu, k < nstaged && soff[k] <= start));
+        uint2* spans = sm.spans[warp];
+        // spans appended and the pixel pairs in them; pairs done, and the span
+        // the next one lies in
+        uint32_t nspans = 0, npairs = 0, done = 0, cur = 0;
+        const unsigned below = (1u << lane) - 1u, upto_lane = (2u << lane) - 1u;
 #pragma unroll 1
         for (uint32_t base = start; base < end; base += 32) {
           // record starts inside (base, base + 32): at most 32 records
           const uint32_t nxt = (uint32_t)rec + 1 + lane;
           const uint32_t pos = nxt < nstaged ? soff[nxt] - base : 32u;
           const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, pos < 32u ? (1u << pos) : 0u);
-          const uint32_t upto = lane == 31 ? starts : starts & ((2u << lane) - 1u);
-          const uint32_t lo = (uint32_t)rec + __popc(upto);
-          const uint32_t t = base + lane;
-          bool h0 = false, h1 = false;
-          int x = 0, y = 0, p = 0;
-          float4 q[3];
-          if (t < end) {
-            // test t of the record: the pixel pair (lx, ly), (lx + 1, ly)
-            const uint32_t geo = sgeo[lo];
-            const uint32_t local = t - soff[lo];
-            const uint32_t bw = (geo >> 8) & 0x1F, pw = (bw + 1) >> 1;
-            const uint32_t ry = (local * (geo >> 13)) >> 16, rp = local - ry * pw;
-            const int lx = (int)(geo & 0xF) + 2 * (int)rp, ly = (int)((geo >> 4) & 0xF) + (int)ry;
-            q[0] = srec[0][lo], q[1] = srec[1][lo], q[2] = srec[2][lo];
-            x = tx0 + lx, y = ty0 + ly, p = ly * kTile + lx;
-            // the walk rule from the staged mask (only a row's first pixel
-            // can be the bbox's left column), then point_in_tri
-            h0 = !(rp == 0 && ((sskip[lo] >> ly) & 1)) && rec_in_tri(q, x, y);
-            h1 = 2 * rp + 1 < bw && rec_in_tri(q, x + 1, y);
-          }
-          const unsigned b0 = __ballot_sync(0xFFFFFFFFu, h0), b1 = __ballot_sync(0xFFFFFFFFu, h1);
-          const uint32_t n0 = (uint32_t)__popc(b0), n1 = (uint32_t)__popc(b1);
-          if (pass == 0) {
-            wsamples += n0 + n1;
-            if (listing && nh + n0 + n1 > (uint32_t)kHitCap) {  // warp-uniform
-              nh = compact_hits(hits, nh, sdepth);
-              listing = nh + n0 + n1 <= (uint32_t)kHitCap;
+          uint32_t pairs = 0, span = 0;
+          if (base + lane < end) {
+            // the lane's row of a record, and the span of it that can be covered
+            const uint32_t row_rec = (uint32_t)rec + __popc(starts & upto_lane), geo = sgeo[row_rec];
+            const int ly = (int)((geo >> 4) & 0xF) + (int)(base + lane - soff[row_rec]);
+            int xa = (int)(geo & 0xF), xb = xa + (int)((geo >> 8) & 0x1F) - 1;
+            // the walk rule: only a row's first pixel can be the bbox's left column
+            xa += (int)((sskip[row_rec] >> ly) & 1u);
+            if (geo & (kRecInside << 13)) {
+              const float4 q1 = srec[1][row_rec], q2 = srec[2][row_rec];
+              const float2 inv = sm.sinv[row_rec];
+              const float ftx = (float)tx0, fy = (float)(ty0 + ly);
+              row_span((q1.x + q1.z * fy) + q1.y * ftx, (q2.x + q2.z * fy) + q2.y * ftx, srec[0][row_rec].w, q1.w,
+                       inv.x, inv.y, (geo & (kRecTight << 13)) != 0, &xa, &xb);
+            }
+            if (xb >= xa) {
+              pairs = (uint32_t)(xb - xa + 2) >> 1;
+              span = row_rec | ((uint32_t)ly << 10) | ((uint32_t)xa << 14) | ((uint32_t)xb << 18);
             }
           }
-          auto resolve = [&](int px, int pp, uint32_t slot) {
-            const uint32_t d = depth_at(q[0].x, q[0].y, q[0].z, (float)px, (float)y);
+          // the record of row base + 32: lane 31's, or the next one if it starts there
+          rec += __popc(starts);
+          if ((uint32_t)rec + 1 < nstaged && soff[rec + 1] == base + 32) rec++;
+          // append the spans, their pixel pairs laid end to end
+          uint32_t first = pairs;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, first, o);
+            if (lane >= o) first += v;
+          }
+          const unsigned who = __ballot_sync(0xFFFFFFFFu, pairs != 0);
+          __syncwarp();  // (readers of the spans overwritten here are done)
+          if (pairs)
+            spans[(nspans + __popc(who & below)) % kSpanRing] = make_uint2(npairs + first - pairs, span);
+          npairs += __shfl_sync(0xFFFFFFFFu, first, 31);
+          nspans += (uint32_t)__popc(who);
+          __syncwarp();
+          // test them 32 at a time; fewer wait for the next rows
+          const uint32_t least = base + 32 < end ? 32u : 1u;
+#pragma unroll 1
+          for (; npairs - done >= least; done += min(32u, npairs - done)) {
+            if (cur + 1 < nspans && spans[(cur + 1) % kSpanRing].x <= done) cur++;
+            const uint32_t sn = cur + 1 + lane;
+            const uint32_t sp = sn < nspans ? spans[sn % kSpanRing].x - done : 32u;
+            const uint32_t sstarts = __reduce_or_sync(0xFFFFFFFFu, sp < 32u ? (1u << sp) : 0u);
+            const uint2 e = spans[(cur + (uint32_t)__popc(sstarts & upto_lane)) % kSpanRing];
+            cur += (uint32_t)__popc(sstarts);
+            const uint32_t lo = e.y & 0x3FF;
+            const int ly = (int)((e.y >> 10) & 0xF), lx = (int)((e.y >> 14) & 0xF) + 2 * (int)(done + lane - e.x);
+            const int p = ly * kTile + lx;
+            const float4 q[3] = {srec[0][lo], srec[1][lo], srec[2][lo]};
+            const float fx = (float)(tx0 + lx), fy = (float)(ty0 + ly);
+            const bool on = done + lane < npairs;
+            const bool h0 = on && rec_in_tri(q, fx, fy);
+            const bool h1 = on && lx < (int)(e.y >> 18) && rec_in_tri(q, fx + 1.0f, fy);
+            const unsigned b0 = __ballot_sync(0xFFFFFFFFu, h0), b1 = __ballot_sync(0xFFFFFFFFu, h1);
+            const uint32_t n0 = (uint32_t)__popc(b0), n1 = (uint32_t)__popc(b1);
             if (pass == 0) {
-              atomicMin(&sdepth[swz32(pp)], d);
-              if (listing) hits[slot] = make_uint2(d, (uint32_t)pp | ((resident ? lo : sidx[lo]) << 8));
-            } else {
-              const uint32_t fd = sdepth[swz32(pp)];
-              if (d > fd - kBufError && d < fd + kBufError) {
-                if (packed)
-                  atomicMin(sid32 + swz32(pp), (__float_as_uint(q[2].w) << kSlotBits) | lo);
-                else
-                  atomicMin(&sid[swz64(pp)], ((unsigned long long)__float_as_uint(q[2].w) << 32) | sidx[lo]);
+              wsamples += n0 + n1;
+              if (listing && nh + n0 + n1 > (uint32_t)kHitCap) {  // warp-uniform
+                nh = compact_hits(hits, nh, sdepth);
+                listing = nh + n0 + n1 <= (uint32_t)kHitCap;
               }
             }
-          };
-          const unsigned below = (1u << lane) - 1u;
-          if (h0) resolve(x, p, nh + (uint32_t)__popc(b0 & below));
-          if (h1) resolve(x + 1, p + 1, nh + n0 + (uint32_t)__popc(b1 & below));
-          if (pass == 0 && listing) nh += n0 + n1;
-          // the record of test base + 32: lane 31's, or the next one if it starts there
-          rec = (int)((uint32_t)rec + __popc(starts));
-          if ((uint32_t)rec + 1 < nstaged && soff[rec + 1] == base + 32) rec++;
+            auto resolve = [&](float px, int pp, uint32_t slot) {
+              const uint32_t d = depth_at(q[0].x, q[0].y, q[0].z, px, fy);
+              if (pass == 0) {
+                atomicMin(&sdepth[swz32(pp)], d);
+                if (listing) hits[slot] = make_uint2(d, (uint32_t)pp | ((resident ? lo : sidx[lo]) << 8));
+              } else {
+                const uint32_t fd = sdepth[swz32(pp)];
+                if (d > fd - kBufError && d < fd + kBufError) {
+                  if (packed)
+                    atomicMin(sid32 + swz32(pp), (__float_as_uint(q[2].w) << kSlotBits) | lo);
+                  else
+                    atomicMin(&sid[swz64(pp)], ((unsigned long long)__float_as_uint(q[2].w) << 32) | sidx[lo]);
+                }
+              }
+            };
+            if (h0) resolve(fx, p, nh + (uint32_t)__popc(b0 & below));
+            if (h1) resolve(fx + 1.0f, p + 1, nh + n0 + (uint32_t)__popc(b1 & below));
+            if (pass == 0 && listing) nh += n0 + n1;
+          }
         }
       }
     }
@@ -1662,29 +1736,6 @@ __device__ __forceinline__ f4 vertex_col(uint32_t c) {
 }
 
 
-// Colour-only arithmetic of the light loop: every use below feeds the colour
-// continuously (no comparison, rounding or index depends on it), so the
-// approximate division is covered by the 1/255 colour tolerance.  The
-// hardware's approximations, taken as single instructions: __fdividef,
-// rsqrtf and __expf compute the same values but wrap them in three or four
-// more for subnormal operands and results, which here are either exact zeros
-// or far below a colour level.  (1080p kernel3 3,350 -> 3,060 instructions
-// per pixel, 223 -> 210 us.)
-__device__ __forceinline__ float ex2_ftz(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float crcp(float b) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return r;
-}
 __device__ __forceinline__ f3 cnormalize(f3 a) {
   float r = rsqrt_ftz(dot3(a, a));
   return mk3(a.x * r, a.y * r, a.z * r);

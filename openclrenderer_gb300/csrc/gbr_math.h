@@ -343,6 +343,14 @@ GBR_HD int tight_box(f3 x, f3 y, float w, float h, float mm[4]) {
   return area2 == 0.0f || mm[0] >= mm[1] || mm[2] >= mm[3] ? kBoxEmpty : kBoxTight;
 }
 
+// Do the rounded vertices all lie on a w x h surface (w <= 3840, h <= 2160)?
+// Every term of the coverage test below at a pixel of the surface is then an
+// integer below 2^24, and exact.
+GBR_HD bool on_surface(f3 x, f3 y, float w, float h) {
+  return x.x >= 0.0f && x.y >= 0.0f && x.z >= 0.0f && y.x >= 0.0f && y.y >= 0.0f && y.z >= 0.0f && x.x <= w &&
+         x.y <= w && x.z <= w && y.x <= h && y.y <= h && y.z <= h;
+}
+
 // Edge-function coverage test of integer pixel (px,py) against the rounded
 // triangle (cl2.cl:4798-4807, point_in_tri), split into per-triangle
 // constants and a per-pixel part with the same evaluation tree.
@@ -369,6 +377,38 @@ GBR_HD bool edge_inside(const EdgeTest& e, float px, float py) {
   float s = ((e.s0 + e.sa * px) + e.sb * py) * e.sign;
   float t = ((e.t0 + e.ta * px) + e.tb * py) * e.sign;
   return s > -0.0001f && t > -0.0001f && (s + t) < e.bound;
+}
+
+// Reciprocal of an edge function's x slope (for row_span), approximate on the
+// device; a slope of 0 as a large number, which puts its crossing left of
+// every pixel or right of it.
+GBR_HD float span_slope(float a) {
+#if defined(__CUDA_ARCH__)
+  return a == 0.0f ? 1e30f : __fdividef(1.0f, a);
+#else
+  return a == 0.0f ? 1e30f : 1.0f / a;
+#endif
+}
+// Narrows the pixels [*xa, *xb] of a row, columns relative to one where the
+// edge functions are s and t, of a record whose vertices are on_surface, to
+// those that edge_inside can hold at: between the crossings of s, t and bound
+// - s - t (is, it, iu: span_slope of their x slopes).  Those are integers
+// (apart from bound's tolerance), exact or, for s + t of a large triangle, off
+// by less than 4: half a unit (4 units) to the safe side, and 0.01 pixel for
+// the reciprocals.
+GBR_HD void row_span(float s, float t, float bound, float is, float it, float iu, bool small, int* xa, int* xb) {
+  const float rs = (-0.5f - s) * is, rt = (-0.5f - t) * it;
+  const float ru = ((small ? -0.5f : -4.0f) - ((bound - s) - t)) * iu;
+  const float inf = 3.4028235e38f;
+  const float lo = fmax_(fmax_(is > 0.0f ? rs : -inf, it > 0.0f ? rt : -inf), iu > 0.0f ? ru : -inf);
+  const float hi = fmin_(fmin_(is > 0.0f ? inf : rs, it > 0.0f ? inf : rt), iu > 0.0f ? inf : ru);
+#if defined(__CUDA_ARCH__)
+  const int a = __float2int_ru(lo - 0.01f), b = __float2int_rd(hi + 0.01f);
+#else
+  const int a = f2i_sat(ceilf(lo - 0.01f)), b = f2i_sat(floorf(hi + 0.01f));
+#endif
+  *xa = a > *xa ? a : *xa;
+  *xb = b < *xb ? b : *xb;
 }
 
 // Quantised depth of a covered pixel (cl2.cl:5113-5115).

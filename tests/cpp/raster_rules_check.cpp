@@ -2,7 +2,7 @@
 // for: walk_first_late_row against walk_row_late over every width <= W, top
 // row < H and row (a row before it must not be late), and box_bounds against
 // depth_at and edge_inside at every pixel of random triangles' boxes; tight_box
-// against edge_inside at every pixel of their bbox4; ssao_tap against ssao_count
+// and row_span against edge_inside at the pixels of their bbox4; ssao_tap against ssao_count
 // wherever ssao_exact holds; shadow_bias below kBiasFullCos; and shadow_limits
 // against the test they bracket.
 // Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
@@ -59,12 +59,12 @@ int main(int argc, char** argv) {
         if (d < lo || d > hi || (f && !edge_inside(e, (float)px, (float)py))) bad++;
       }
   }
-  long tight = 0, empty = 0, outside = 0;
+  long tight = 0, empty = 0, outside = 0, spans = 0;
   const float sizes[5][2] = {{3840, 2160}, {1024, 1024}, {1920, 1080}, {64, 48}, {17, 9}};
   for (int i = 0; i < n; i++) {
     const float w = sizes[i % 5][0], h = sizes[i % 5][1];
     // around the surface and its far corner, extents from sub-pixel to over 64, some collinear
-    const float span = powf(10.0f, uni(-0.5f, 2.0f)), cx = (i & 8) ? w : uni(0, w), cy = (i & 8) ? h : uni(0, h);
+    const float span = powf(10.0f, uni(-0.5f, 3.0f)), cx = (i & 8) ? w : uni(0, w), cy = (i & 8) ? h : uni(0, h);
     f3 p[3];
     for (int k = 0; k < 3; k++) p[k] = mk3(cx + uni(-span, span), cy + uni(-span, span), 100.0f);
     if (!(rng() & 7)) p[2] = mk3(p[0].x + 2.0f * (p[1].x - p[0].x), p[0].y + 2.0f * (p[1].y - p[0].y), 100.0f);
@@ -77,15 +77,28 @@ int main(int argc, char** argv) {
     const int kind = tight_box(xv, yv, w, h, tm);
     tight += kind == kBoxTight;
     empty += kind == kBoxEmpty;
+    EdgeTest e = make_edge(xv.x, yv.x, xv.y, yv.y, xv.z, yv.z);
+    if (on_surface(xv, yv, w, h)) {  // the spans of rows, 16 columns at a time from a column near the triangle
+      EdgeTest f = e;
+      f.s0 *= e.sign, f.sa *= e.sign, f.sb *= e.sign, f.t0 *= e.sign, f.ta *= e.sign, f.tb *= e.sign;
+      const float tx = 16.0f * floorf(uni(mm[0], mm[1]) / 16.0f);
+      for (float py = mm[2]; py < mm[3]; py += (mm[3] - mm[2] > 80 ? 7 : 1)) {
+        int xa = 0, xb = 15;
+        row_span((f.s0 + f.sb * py) + f.sa * tx, (f.t0 + f.tb * py) + f.ta * tx, f.bound, span_slope(f.sa),
+                 span_slope(f.ta), span_slope(-(f.sa + f.ta)), kind != kBoxAny, &xa, &xb);
+        spans += xa > 0 || xb < 15;
+        for (int k = 0; k < 16; k++)
+          if ((k < xa || k > xb) && edge_inside(e, tx + (float)k, py)) outside++;
+      }
+    }
     if (kind == kBoxAny) continue;
-    const EdgeTest e = make_edge(xv.x, yv.x, xv.y, yv.y, xv.z, yv.z);
     for (float py = mm[2]; py < mm[3]; py++)
       for (float px = mm[0]; px < mm[1]; px++) {
         const bool in = px >= tm[0] && px < tm[1] && py >= tm[2] && py < tm[3];
         if ((!in || kind == kBoxEmpty) && edge_inside(e, px, py)) outside++;
       }
   }
-  printf("tight=%ld empty=%ld outside=%ld\n", tight, empty, outside);
+  printf("tight=%ld empty=%ld spans=%ld outside=%ld\n", tight, empty, spans, outside);
   bad += outside;
   long taps = 0, inexact = 0, wrong = 0;
   for (int i = 0; i < n; i++) {
@@ -136,5 +149,5 @@ int main(int argc, char** argv) {
   printf("taps=%ld inexact=%ld wrong=%ld\n", taps, inexact, wrong);
   bad += wrong;
   printf("early=%ld late=%ld boxes=%d full=%ld bounded=%ld bad=%ld\n", early, late, n, full, bounded, bad);
-  return early == 0 && late > 0 && bad == 0 && tight > 0 && empty > 0 && taps > 0 && inexact > 0 && full > 0 && bounded > 0 ? 0 : 1;
+  return early == 0 && late > 0 && bad == 0 && tight > 0 && empty > 0 && spans > 0 && taps > 0 && inexact > 0 && full > 0 && bounded > 0 ? 0 : 1;
 }

@@ -8,7 +8,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 def test_shortcuts(tmp_path):
     """No row before walk_first_late_row is late (every width <= 800, top row < 600; run with
     3840 2160 the program covers the whole range), box_bounds encloses every
-    pixel's depth, tight_box leaves no covered pixel out, ssao_tap counts as ssao_count
+    pixel's depth, tight_box and row_span leave no covered pixel out, ssao_tap counts as ssao_count
     does, and the shadow bias and limits hold."""
     exe = tmp_path / "rrc"
     subprocess.run(["g++", "-O2", "-std=c++17", "-fopenmp", "-ffp-contract=off", "-I",
