@@ -10,86 +10,114 @@
 
 namespace gbr {
 
+// A light with shafts as the marches read it: its projection (screen x, y and
+// camera z) and its colour times its intensity.
+struct ShaftLight {
+  f3 spos, col;
+};
+
 // screenspace_godrays (cl2.cl:1792-1917) for pixel (x, y) of a view: light
-// shafts of every light with godray_intensity > 0, marched from the pixel
-// towards the light's screen position over the depth buffer.  cc / cs: the
-// camera's cosines and sines.  Returns the RGBA colour before quantisation.
-__device__ f4 godrays_pixel(int x, int y, const uint32_t* depth, const uint8_t* rgba_in, int W, int H, float fov,
-                        const gbr_light* __restrict__ lights, uint32_t nlights, f3 cpos, f3 cc, f3 cs) {
+// shafts of every light with godray_intensity > 0 (nshafts of them), marched
+// from the pixel towards the light's screen position over the depth buffer.
+// Returns the RGBA colour before quantisation.
+__device__ f4 godrays_pixel(int x, int y, const uint32_t* __restrict__ depth, const uint8_t* rgba_in, int W, int H,
+                            const ShaftLight* shafts, uint32_t nshafts) {
   const float samples = 80.f;
   const uint32_t my_depth = depth[(size_t)y * W + x];
   f4 my_col = read_linear_rgba8(rgba_in, W, H, (float)x - 0.25f, (float)y - 0.25f);
   const float decay_factor = 0.97f, weight = 0.01f;
   const float step = 400.f / samples;  // max_length / samples
-  for (uint32_t i = 0; i < nlights; i++) {
-    const gbr_light& L = lights[i];
-    const float ray_intensity = L.godray_intensity;
-    if (ray_intensity <= 0) continue;
+  const f3 original = mk3((float)x, (float)y, depth_to_dist(my_depth));
+  // a step is occluded where its distance is below the pixel's own - 5: in
+  // depth units, one integer comparison.  (The reference also requires cdepth
+  // != UINT_MAX; an empty pixel is at 350000, never below 349995.)
+  const uint32_t occluded_below = nshafts ? depth_below(original.z - 5.0f) : 0u;
+  const float xmax = (float)W - 1.0f, ymax = (float)H - 1.0f;
+  for (uint32_t i = 0; i < nshafts; i++) {
     float idecay = 1.f;
     f3 iter_col = mk3(0, 0, 0);
-    const f3 lpos = mk3(L.pos[0], L.pos[1], L.pos[2]);
-    const f3 slpos = depth_project1(rot_cs(lpos, cpos, cc, cs), (float)W, (float)H, fov);
-    f3 current = mk3((float)x, (float)y, depth_to_dist(my_depth));
-    f3 dest = slpos;
-    const f3 original = current;
-    if (slpos.z < 0) dest = add3(sub3(current, dest), current);
-    const float vx = fabsf(current.x - dest.x), vy = fabsf(current.y - dest.y);
+    f3 dest = shafts[i].spos;
+    const f3 cval = shafts[i].col;
+    if (dest.z < 0) dest = add3(sub3(original, dest), original);
+    const float vx = fabsf(original.x - dest.x), vy = fabsf(original.y - dest.y);
     const float mnum = vx > vy ? vx : vy;
-    f3 dir = sub3(dest, current);
-    dir = mk3(fdiv(dir.x, mnum), fdiv(dir.y, mnum), fdiv(dir.z, mnum));
-    dir = mul3s(dir, step);
-    const f3 cval = mul3s(mk3(L.col[0], L.col[1], L.col[2]), ray_intensity);
-    const float thr = original.z - 5.0f;
-    // depth_to_dist(d) < thr exactly when depth_scaled(d) < thr * 2^32 (the
-    // scaling by 2^-32 commutes with rounding): one multiplication per step
-    const float thr_scaled = thr * kTwo32;
-    const float xmax = (float)W - 1.0f, ymax = (float)H - 1.0f;
+    f3 dir = sub3(dest, original);
+    const float dx = fdiv(dir.x, mnum) * step, dy = fdiv(dir.y, mnum) * step;
     // steps j with (float)j < mnum and j < samples
     const int n = mnum > 0.0f ? (int)fminf(ceilf(mnum), samples) : 0;
-    float cx = current.x, cy = current.y;
+    float cx = original.x, cy = original.y;
     // A march whose whole segment, one step past its end, keeps 0.05 px inside
     // the screen needs no bounds tests: the positions move monotonically along
     // dir, and 80 float additions below 4096 stray from the exact line by less
     // than 0.01 px.  (Every comparison fails on NaN.)
-    const float ex = cx + (float)n * dir.x, ey = cy + (float)n * dir.y;
+    const float ex = cx + (float)n * dx, ey = cy + (float)n * dy;
     const bool inside = cx >= 0.05f && ex >= 0.05f && cx <= xmax - 0.05f && ex <= xmax - 0.05f &&
                         cy >= 0.05f && ey >= 0.05f && cy <= ymax - 0.05f && ey <= ymax - 0.05f;
     // Eight steps at a time: their positions (the same running sums as the
     // reference's current += dir), then their depth loads in flight together,
     // then the decay chain in order.  The reference skips the rest of the
     // march once it leaves the screen; an unoccluded step adds exactly 0.
-    for (int j0 = 0; j0 < n; j0 += 8) {
-      float px[8], py[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        px[k] = cx;
-        py[k] = cy;
-        cx += dir.x;
-        cy += dir.y;
-      }
-      int m = min(8, n - j0);
-      if (!inside) {
-#pragma unroll
-        for (int k = 7; k >= 0; k--)
-          if (px[k] < 0 || py[k] < 0 || px[k] >= xmax || py[k] >= ymax) m = min(m, k);
-      }
-      uint32_t dv[8];
-#pragma unroll
-      // (cvt.rzi: truncation, NaN -> 0, so a NaN march stays in bounds as in the oracle)
-      for (int k = 0; k < 8; k++)
-        dv[k] = k < m ? __ldg(depth + (size_t)__float2int_rz(py[k]) * W + __float2int_rz(px[k])) : 0u;
+    auto resolve = [&](const uint32_t (&dv)[8], int m) {
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         if (k < m) {
-          // (the reference also requires cdepth != UINT_MAX; an empty pixel is at
-          // 350000, never below thr = the pixel's own distance - 5 <= 349995)
-          if (depth_scaled(dv[k]) < thr_scaled) {
+          if (dv[k] < occluded_below) {
             idecay *= 0.9f;
             iter_col = add3(iter_col, mul3s(mul3s(cval, idecay), weight));
           }
           idecay *= decay_factor;
         }
       }
+    };
+    int j0 = 0;
+    if (inside) {
+      // positions in [0, 4096): truncated by adding 2^23 rounded toward zero
+      // (the low bits are the integer), off the conversion pipe, which three
+      // conversions a step kept as busy as the issue slots
+      const uint32_t magic = 0x4B000000u * (uint32_t)W + 0x4B000000u;
+      for (; j0 + 8 <= n; j0 += 8) {
+        uint32_t dv[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const uint32_t ix = __float_as_uint(__fadd_rz(cx, 8388608.0f)), iy = __float_as_uint(__fadd_rz(cy, 8388608.0f));
+          dv[k] = __ldg(depth + (iy * (uint32_t)W + ix - magic));
+          cx += dx;
+          cy += dy;
+        }
+        uint32_t nearest = dv[0];
+#pragma unroll
+        for (int k = 1; k < 8; k++) nearest = min(nearest, dv[k]);
+        if (nearest < occluded_below) {
+          resolve(dv, 8);
+        } else {  // nothing in the way: the decay alone
+#pragma unroll
+          for (int k = 0; k < 8; k++) idecay *= decay_factor;
+        }
+      }
+    }
+    for (; j0 < n; j0 += 8) {
+      int m = min(8, n - j0);
+      uint32_t dv[8];
+      {
+        float px[8], py[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          px[k] = cx;
+          py[k] = cy;
+          cx += dx;
+          cy += dy;
+        }
+        if (!inside) {
+#pragma unroll
+          for (int k = 7; k >= 0; k--)
+            if (px[k] < 0 || py[k] < 0 || px[k] >= xmax || py[k] >= ymax) m = min(m, k);
+        }
+#pragma unroll
+        // (cvt.rzi: truncation, NaN -> 0, so a NaN march stays in bounds as in the oracle)
+        for (int k = 0; k < 8; k++)
+          dv[k] = k < m ? __ldg(depth + (size_t)__float2int_rz(py[k]) * W + __float2int_rz(px[k])) : 0u;
+      }
+      resolve(dv, m);
       if (m < 8) break;
     }
     my_col.x += iter_col.x;
@@ -103,14 +131,35 @@ __device__ f4 godrays_pixel(int x, int y, const uint32_t* depth, const uint8_t* 
   return r;
 }
 
-// engine::draw_godrays (engine.cpp:1463-1482): one thread per pixel.
+// engine::draw_godrays (engine.cpp:1463-1482): one thread per pixel.  The
+// lights with shafts, in order, are projected once per block.  Bound by
+// instruction issue (the decay chain of a march is sequential).
 __global__ void __launch_bounds__(256) k_godrays(const uint32_t* __restrict__ depth, const uint8_t* __restrict__ in,
                                                  uint8_t* __restrict__ out, int W, int H, float fov,
                                                  const gbr_light* __restrict__ lights, uint32_t nlights, f3 cpos,
                                                  f3 cc, f3 cs) {
+  __shared__ ShaftLight shafts[kMaxLights];
+  __shared__ uint32_t nshafts;
+  if (threadIdx.x < 32) {
+    uint32_t n = 0;
+    for (uint32_t i0 = 0; i0 < nlights; i0 += 32) {
+      const uint32_t i = i0 + threadIdx.x;
+      const bool on = i < nlights && !(lights[i].godray_intensity <= 0);
+      const unsigned who = __ballot_sync(0xFFFFFFFFu, on);
+      if (on) {
+        const gbr_light& L = lights[i];
+        ShaftLight& s = shafts[n + __popc(who & ((1u << threadIdx.x) - 1u))];
+        s.spos = depth_project1(rot_cs(mk3(L.pos[0], L.pos[1], L.pos[2]), cpos, cc, cs), (float)W, (float)H, fov);
+        s.col = mul3s(mk3(L.col[0], L.col[1], L.col[2]), L.godray_intensity);
+      }
+      n += (uint32_t)__popc(who);
+    }
+    if (threadIdx.x == 0) nshafts = n;
+  }
+  __syncthreads();
   const int x = blockIdx.x * 16 + (threadIdx.x & 15), y = blockIdx.y * 16 + (threadIdx.x >> 4);
   if (x >= W || y >= H) return;
-  const f4 c = godrays_pixel(x, y, depth, in, W, H, fov, lights, nlights, cpos, cc, cs);
+  const f4 c = godrays_pixel(x, y, depth, in, W, H, shafts, nshafts);
   reinterpret_cast<uint32_t*>(out)[(size_t)y * W + x] = pack_rgba(c.x, c.y, c.z, c.w);
 }
 
@@ -251,6 +300,69 @@ cudaError_t launch_pseudo_aa(const uint32_t* depth, const uint32_t* ids, const u
 // capped at 50 px, is averaged over that many bilinear taps centred on the
 // pixel.  Objects with a pixel on screen are marked in seen[] for the history
 // update.
+// Bytes LO and HI of t over 255, as RN(x * hi + RN(x * lo)) with 1 / 255 = hi +
+// lo: equal to u8_over_255 for every byte (two packed operations, not three).
+template <int LO, int HI>
+__device__ __forceinline__ float2 over_255(uint32_t t) {
+  const float2 m = make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7440 | LO)),
+                               __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7440 | HI)));
+  const float2 x = __fadd2_rn(m, dup2(-8388608.0f));
+  return __ffma2_rn(x, dup2(kInv255Hi), __fmul2_rn(x, dup2(kInv255Lo)));
+}
+// o (+)= w * texel t
+__device__ __forceinline__ void add_texel(uint32_t t, float w, bool first, f4& o) {
+  const float2 w2 = dup2(w), rg = __fmul2_rn(w2, over_255<0, 1>(t)), ba = __fmul2_rn(w2, over_255<2, 3>(t));
+  o.x = first ? rg.x : __fadd_rn(o.x, rg.x);
+  o.y = first ? rg.y : __fadd_rn(o.y, rg.y);
+  o.z = first ? ba.x : __fadd_rn(o.z, ba.x);
+  o.w = first ? ba.y : __fadd_rn(o.w, ba.y);
+}
+
+// read_linear_rgba8 with two channels per packed instruction: the bytes as
+// 2^23 + b less 2^23, their quotients by 255, and the weighted texels, which
+// are then added in the same order.  (Added one channel at a
+// time: the assembler contracts a packed product and a packed sum into one
+// rounding, --fmad=false or not.)  (A shared table of the 256 quotients took 16 lookups a tap,
+// with bank conflicts, and bound the pass.)
+__device__ __forceinline__ f4 read_linear_packed(const uint8_t* __restrict__ img, int W, int H, float cx, float cy) {
+  const float u = cx - 0.5f, v = cy - 0.5f;
+  const float fi = floorf(u), fj = floorf(v);
+  const float a = u - fi, b = v - fj;
+  const int i0 = (int)fi, j0 = (int)fj;
+  const int xs[2] = {min(max(i0, 0), W - 1), min(max(i0 + 1, 0), W - 1)};
+  const int ys[2] = {min(max(j0, 0), H - 1), min(max(j0 + 1, 0), H - 1)};
+  const float ia = 1.0f - a, ib = 1.0f - b;
+  const float wt[4] = {ia * ib, a * ib, ia * b, a * b};
+  f4 o;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint32_t t = rgba8_word(img, (size_t)ys[k >> 1] * W + xs[k & 1]);
+    add_texel(t, wt[k], k == 0, o);
+  }
+  return o;
+}
+
+// read_linear_packed at (cx + 0.5, cy + 0.5) for 1 <= cx <= W - 2, 1 <= cy <= H
+// - 2, where nothing is clamped; the floors by addition of 2^23 rounded toward
+// zero, whose low bits are the coordinates.
+__device__ __forceinline__ f4 read_linear_inner(const uint8_t* __restrict__ img, int W, float cx, float cy) {
+  const float u = (cx + 0.5f) - 0.5f, v = (cy + 0.5f) - 0.5f;
+  const float zu = __fadd_rz(u, 8388608.0f), zv = __fadd_rz(v, 8388608.0f);
+  const float a = u - (zu - 8388608.0f), b = v - (zv - 8388608.0f);
+  const uint32_t magic = 0x4B000000u * (uint32_t)W + 0x4B000000u;
+  const uint32_t* p = reinterpret_cast<const uint32_t*>(img) +
+                      (__float_as_uint(zv) * (uint32_t)W + __float_as_uint(zu) - magic);
+  const uint32_t* q = p + W;
+  const uint32_t t0 = __ldg(p), t1 = __ldg(p + 1), t2 = __ldg(q), t3 = __ldg(q + 1);
+  const float ia = 1.0f - a, ib = 1.0f - b;
+  f4 o;
+  add_texel(t0, ia * ib, true, o);
+  add_texel(t1, a * ib, false, o);
+  add_texel(t2, ia * b, false, o);
+  add_texel(t3, a * b, false, o);
+  return o;
+}
+
 struct MotionCam {
   f3 cpos, cc, cs, opos, oc, os;
   float fov, strength, cam_w;
@@ -263,16 +375,6 @@ __global__ void __launch_bounds__(256) k_motion_blur(const gbr_triangle* __restr
                                                      const uint32_t* __restrict__ ids, const uint8_t* __restrict__ in,
                                                      uint8_t* __restrict__ out, int W, int H, MotionCam a,
                                                      uint32_t* __restrict__ seen, uint32_t ntris) {
-  // the 256 quotients c / 255 of a channel byte (u8_over_255), read by every
-  // bilinear tap from shared memory
-  __shared__ float s255[256];
-  s255[threadIdx.x] = u8_over_255(threadIdx.x);
-  __syncthreads();
-  struct Tab {
-    const float* t;
-    __device__ float operator()(uint32_t c) const { return t[c]; }
-  };
-  const Tab tab{s255};
   const int x = blockIdx.x * 16 + (threadIdx.x & 15), y = blockIdx.y * 16 + (threadIdx.x >> 4);
   if (x >= W || y >= H) return;
   const size_t p = (size_t)y * W + x;
@@ -298,7 +400,7 @@ __global__ void __launch_bounds__(256) k_motion_blur(const gbr_triangle* __restr
   const f3 prev = depth_project1(rot_cs(last, a.opos, a.oc, a.os), (float)W, (float)H, a.fov);
   f4 acc;
   if (prev.z < 20.0f) {
-    acc = read_linear_rgba8_with(in, W, H, (float)x + 0.5f, (float)y + 0.5f, tab);
+    acc = read_linear_packed(in, W, H, (float)x + 0.5f, (float)y + 0.5f);
   } else {
     float mx = (float)x - prev.x, my = (float)y - prev.y;
     const float nx = (float)x - nocam.x, ny = (float)y - nocam.y;
@@ -320,9 +422,22 @@ __global__ void __launch_bounds__(256) k_motion_blur(const gbr_triangle* __restr
     float cx = (float)x - mx * 0.5f, cy = (float)y - my * 0.5f;  // mx / 2 exactly
     acc.x = acc.y = acc.z = acc.w = 0.0f;
     float cnt = 0.0f;
-    for (int i = 0; i < n; i++, cx += sx, cy += sy) {
+    // Taps that all keep a pixel and more inside the screen (they move
+    // monotonically, and 50 additions stray by less than 0.01 px) need no
+    // bounds tests or clamps.  (Every comparison fails on NaN.)
+    const float ex = cx + sx * (float)n, ey = cy + sy * (float)n;
+    const float xm = (float)W - 2.05f, ym = (float)H - 2.05f;
+    int i = 0;
+    if (cx >= 1.05f && ex >= 1.05f && cx <= xm && ex <= xm && cy >= 1.05f && ey >= 1.05f && cy <= ym && ey <= ym) {
+      for (; i < n; i++, cx += sx, cy += sy) {
+        const f4 c = read_linear_inner(in, W, cx, cy);
+        acc.x += c.x; acc.y += c.y; acc.z += c.z; acc.w += c.w;
+      }
+      cnt = (float)n;
+    }
+    for (; i < n; i++, cx += sx, cy += sy) {
       if (cx < 0 || cx >= (float)W || cy < 0 || cy >= (float)H) continue;
-      const f4 c = read_linear_rgba8_with(in, W, H, cx + 0.5f, cy + 0.5f, tab);
+      const f4 c = read_linear_packed(in, W, H, cx + 0.5f, cy + 0.5f);
       acc.x += c.x; acc.y += c.y; acc.z += c.z; acc.w += c.w;
       cnt += 1.0f;
     }
@@ -496,45 +611,54 @@ __device__ int reflection_pixel(const SceneDev& sc, const ReflectCam& v, int x, 
   // time: positions first (they do not depend on the loads), then their
   // depth loads in flight together, then the tests in order.
   const float ipz = rcp(vprev.z), isz = rcp(vstart.z);  // line_depth_point's reciprocals, loop-invariant
-  // a step on screen has 0 <= x < W and 0 <= y < H, or a NaN coordinate
-  // (every comparison of the test fails on NaN): f2i_sat is then a
-  // truncation, or 0 for NaN
-  auto on_screen_int = [](float c) { return c == c ? (int)c : 0; };
+  // A step is on screen when 0 <= x < W and 0 <= y < H or a coordinate is NaN
+  // (every comparison of the reference's test fails on NaN; it reads pixel 0
+  // then): the conversion rounds down and turns NaN into 0, so that is one
+  // unsigned comparison per coordinate.
+  auto at = [](float c) { return (uint32_t)__float2int_rd(c); };
   float a = 1.0f, stop = 0.0f;
   bool found = false;
   {
-    const float dd = depth_to_dist(__ldg(depth + (size_t)on_screen_int(sj.y) * W + on_screen_int(sj.x)));
+    const float dd = depth_to_dist(__ldg(depth + (size_t)at(sj.y) * W + at(sj.x)));
     if (dd < sj.z - 1.0f) {
       found = true;
       stop = dd;  // the refinement reads the depth where the march stopped on every try
     }
   }
   for (int i0 = 1; i0 < 200 && !found; i0 += 4) {
-    f3 pt[4];
+    float w[4];  // 1 / z of the steps
+    uint32_t px[4], py[4];
     int m = min(4, 200 - i0);  // the first step off screen, or past the last
     const float fi0 = (float)i0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       // ai = 1 + i and b = 1 - ai = -i, both exact (integers below 2^24)
       const float fi = fi0 + (float)k, ai = fi + 1.0f;
-      pt[k] = mk3(fma_(vprev.x, -fi, vstart.x * ai), fma_(vprev.y, -fi, vstart.y * ai), rcp(fma_(ipz, -fi, isz * ai)));
+      px[k] = at(fma_(vprev.x, -fi, vstart.x * ai));
+      py[k] = at(fma_(vprev.y, -fi, vstart.y * ai));
+      w[k] = fma_(ipz, -fi, isz * ai);
     }
 #pragma unroll
     for (int k = 3; k >= 0; k--)
-      if (pt[k].x < 0 || pt[k].y < 0 || pt[k].x >= fw || pt[k].y >= fh) m = min(m, k);
+      if (px[k] >= (uint32_t)W || py[k] >= (uint32_t)H) m = min(m, k);
     uint32_t dv[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      dv[k] = k < m ? __ldg(depth + (size_t)on_screen_int(pt[k].y) * W + on_screen_int(pt[k].x)) : 0u;
+    for (int k = 0; k < 4; k++) dv[k] = k < m ? __ldg(depth + (size_t)(py[k] * (uint32_t)W + px[k])) : 0u;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (found) break;
       if (k >= m) return 0;  // off screen (or past step 199) before the ray met anything
-      const float dd = depth_to_dist(dv[k]);
-      if (dd < pt[k].z - 1.0f) {
+      // dd < 1 / w - 1: with the approximate reciprocal (2^-23 of it off, the
+      // other roundings a few 2^-24) unless the two sides are too near to tell
+      const float za = crcp(w[k]);
+      const float gap = fma_(depth_scaled(dv[k]), -kInvMulInt, za - 1.0f);  // z - 1 - dd
+      bool hit = gap > 0.0f;
+      if (!(fabsf(gap) > fabsf(za) * 1e-6f + 1e-6f) || !(fabsf(za) < 1e30f))
+        hit = depth_to_dist(dv[k]) < rcp(w[k]) - 1.0f;
+      if (hit) {
         found = true;
         a = fi0 + (float)(k + 1);  // 1 + i
-        stop = dd;
+        stop = depth_to_dist(dv[k]);
       }
     }
   }

@@ -18,6 +18,28 @@ GBR_HD float depth_to_dist(uint32_t d) { return ((float)d * kInvMulInt) * kDepth
 constexpr float kTwo32 = 4294967296.0f;
 GBR_HD float depth_scaled(uint32_t d) { return (float)d * kDepthFar; }
 
+// The smallest d with depth_to_dist(d) >= t (UINT_MAX if there is none below
+// it): depth_to_dist(d) < t is d < depth_below(t), since depth_to_dist does
+// not decrease.  Bisected from a bracket 10 * 2^-24 of t wide to either side.
+GBR_HD uint32_t depth_below(float t) {
+  if (!(t > 0.0f)) return 0u;
+  const float slack = t * 6e-7f;
+  uint32_t lo = f2u_sat((t - slack) * (kMulInt / kDepthFar)), hi = f2u_sat((t + slack) * (kMulInt / kDepthFar));
+  hi += hi != 0xFFFFFFFFu;
+  while (lo < hi) {  // below lo: less than t; hi and above: not (or the end)
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (depth_to_dist(mid) < t)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// 1 / 255 = kInv255Hi + kInv255Lo: fma(x, hi, x * lo) is fdiv(x, 255.0f) for
+// every byte x (tests/cpp/raster_rules_check.cpp).
+constexpr float kInv255Hi = 0x1.010102p-8f, kInv255Lo = -0x1.fdfdfep-33f;
+
 // How many of the thresholds t0 < t1 < t2 < t3 < t4 lie below d2, i.e.
 // (d2 > t0) + ... + (d2 > t4): the thresholds dep + z (z = -2..2, dep <=
 // 350000) are strictly increasing in float, so the predicates are monotone and

@@ -4,7 +4,7 @@
 // depth_at and edge_inside at every pixel of random triangles' boxes; tight_box
 // and row_span against edge_inside at the pixels of their bbox4; ssao_tap against ssao_count
 // wherever ssao_exact holds; shadow_bias below kBiasFullCos; and shadow_limits
-// against the test they bracket.
+// and depth_below against the tests they stand for; and the two-part 1 / 255.
 // Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
 #include <cmath>
 #include <cstdio>
@@ -144,6 +144,13 @@ int main(int argc, char** argv) {
       shadow += (d < lo && !t) || (d > hi && t);
     }
   }
+  for (int i = 0; i < n; i++) {  // the limit, and the depths on either side of it
+    const float t = (i & 7) ? powf(10.0f, uni(-5.0f, 5.6f)) : uni(-10.0f, 10.0f);
+    const uint32_t d = depth_below(t);
+    shadow += (d > 0 && !(depth_to_dist(d - 1) < t)) || (d < kDepthClear && depth_to_dist(d) < t);
+  }
+  for (int c = 0; c < 256; c++)
+    shadow += fma_((float)c, kInv255Hi, (float)c * kInv255Lo) != fdiv((float)c, 255.0f);
   printf("cosines=%ld shadow=%ld\n", cosines, shadow);
   bad += cosines + shadow;
   printf("taps=%ld inexact=%ld wrong=%ld\n", taps, inexact, wrong);
