@@ -292,7 +292,8 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
   }
   CU(mark(1, geom));
   const bool prep = view && sh.shade;
-  const bool on_side = prep && side && side->stream;
+  const bool inline_prep = prep && sh.nsurf == 1;  // the shade constants in the raster's launch
+  const bool on_side = prep && !inline_prep && side && side->stream;
   CU(launch_offsets(ws, wm.surf.p, sh.nsurf, sh.tiles_per_surface, geom));
   CU(mark(2, geom));
   CU(launch_fill(ws, wm.surf.p, geom));
@@ -320,11 +321,12 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
     }
   } else {
     if (!fused)
-      CU(launch_raster(ws, wm.surf.p, sh.nsurf, sh.nfine, view, tu.raster_threads, geom, sh.tiles_per_surface));
+      CU(launch_raster(ws, wm.surf.p, sh.nsurf, sh.nfine, view, tu.raster_threads, geom, sh.tiles_per_surface, 0,
+                       inline_prep ? &sd : nullptr));
     CU(mark(4, geom));
   }
   if (view && s->mark_raster && !fused && !piped) CU(cudaEventRecord(s->raster_done, geom));
-  if (prep && !on_side) CU(launch_prep(sd, ws, geom));
+  if (prep && !inline_prep && !on_side) CU(launch_prep(sd, ws, geom));
   if (split && !piped) {
     CU(cudaEventRecord(join, geom));
     CU(cudaStreamWaitEvent(st, join, 0));
@@ -347,8 +349,10 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
     CU(mark(5, st));
   } else if (view && sh.shade) {
     CU(mark(6, st));
-    CU(launch_shade(sd, wm.views.p, sh.nitems, wm.surf.p, sh.nfine, ws, st, sh.features, 0, sh.one_view, sh.one_surf));
+    CU(launch_shade(sd, wm.views.p, sh.nitems, wm.surf.p, sh.nfine, ws, st, sh.features, 0, sh.one_view, sh.one_surf,
+                    sh.one_view ? host_ctr : nullptr));
     CU(mark(5, st));
+    if (sh.one_view) return GBR_OK;  // kernel3 has left the counters in host_ctr
   }
   CU(cudaMemcpyAsync(host_ctr, ws.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
   return GBR_OK;

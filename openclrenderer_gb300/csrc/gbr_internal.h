@@ -230,17 +230,20 @@ cudaError_t launch_texture_levels(const uint32_t* nums, const uint32_t* sizes, u
 // tiles_per_surface: the common tile count when every surface has the same
 // size (cube faces), else 0.
 // tile0: the first tile of the launch (ntiles tiles from there).
+// prep (a pass of one view): the launch also does launch_prep's work.
 cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t nsurf,
                           uint32_t ntiles, bool with_id, int threads, cudaStream_t st,
-                          uint32_t tiles_per_surface = 0, uint32_t tile0 = 0);
+                          uint32_t tiles_per_surface = 0, uint32_t tile0 = 0, const SceneDev* prep = nullptr);
 // features: some view has kernel3's optional switches on (gbr_view.flags).
 // Reads the pass's counters: nothing is shaded after an overflow.
 // one_view / one_surf: the view of a one-view pass in host memory, passed with
-// the launch (null: read from d_views / d_surf, as a captured launch must).
+// the launch (null: read from d_views / d_surf, as a captured launch must);
+// with them, host_ctr: where to leave the counters in mapped host memory.
 cudaError_t launch_shade(const SceneDev& sc, const ViewParams* d_views, uint32_t nviews,
                          const Surface* d_surf, uint32_t ntiles, const Workspace& ws,
                          cudaStream_t st, bool features = false, uint32_t tile0 = 0,
-                         const ViewParams* one_view = nullptr, const Surface* one_surf = nullptr);
+                         const ViewParams* one_view = nullptr, const Surface* one_surf = nullptr,
+                         Counters* host_ctr = nullptr);
 // The fused raster -> shade pass of many views: one cooperative persistent
 // launch over the work order sched (nseg segments, see k_raster_shade) with
 // the queue words (2 + views, zeroed before); raster tiles of threads (128 or

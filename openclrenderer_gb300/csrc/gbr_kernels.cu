@@ -1420,13 +1420,21 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   }
 }
 
+// prep_blocks (one view that shades): the first blocks of the grid compute the
+// shade constants instead, beside the tiles, which do not read them.
 template <int NT, bool ID, bool CC = false>
 __global__ void __launch_bounds__(NT, (ID ? 1024 : 1280) / NT) k_raster(Workspace ws, const Surface* __restrict__ surfs,
-                                                          uint32_t nsurf, uint32_t tile0) {
+                                                          uint32_t nsurf, uint32_t tile0, uint32_t prep_blocks,
+                                                          const __grid_constant__ SceneDev sc) {
   __shared__ RasterSmem<NT, ID> sm;
   if (ws.ctr->overflow) return;
+  if (ID && !CC && blockIdx.x < prep_blocks) {
+    const uint32_t nrec = min(ws.ctr->nrec, ws.rec_cap);
+    for (uint32_t r = blockIdx.x * NT + threadIdx.x; r < nrec; r += prep_blocks * NT) prep_shade(sc, ws.srec + r);
+    return;
+  }
   // surfaces of one size (cube faces) come as grid rows: surface = blockIdx.y
-  const uint32_t tile = gridDim.y > 1 ? surfs[blockIdx.y].tile_base + blockIdx.x : tile0 + blockIdx.x;
+  const uint32_t tile = gridDim.y > 1 ? surfs[blockIdx.y].tile_base + blockIdx.x : tile0 + blockIdx.x - prep_blocks;
   raster_tile<NT, ID, CC>(ws, surfs, nsurf, tile, gridDim.y > 1 ? (int)blockIdx.y : -1, sm);
 }
 
@@ -2227,12 +2235,16 @@ __global__ void __launch_bounds__(kTilePixels, 4) k_shade(SceneDev sc,
                                                const Counters* __restrict__ ctr,
                                                uint32_t rec_cap, uint32_t tile0,
                                                const uint8_t* __restrict__ tile_empty,
-                                               const uint2* __restrict__ tiles) {
+                                               const uint2* __restrict__ tiles, Counters* __restrict__ host_ctr) {
   constexpr int NW = kTilePixels / 32;
   extern __shared__ float4 s_lights[];  // kLightQuads per light of the scene
   __shared__ float s_colx[kTile + 1], s_rowy[kTile + 1];
   __shared__ uint32_t s_warp[NW];
   __shared__ uint32_t s_px[kTilePixels], s_d[kTilePixels], s_r[kTilePixels];
+  // (the counters are final: a copy in mapped host memory saves the pass a
+  // transfer at its end)
+  if (ONE && host_ctr && blockIdx.x == 0 && threadIdx.x < sizeof(Counters) / 4)
+    reinterpret_cast<uint32_t*>(host_ctr)[threadIdx.x] = reinterpret_cast<const uint32_t*>(ctr)[threadIdx.x];
   if (ctr->overflow) return;
   const uint32_t nrec = min(ctr->nrec, rec_cap);
   const uint32_t tile = tile0 + blockIdx.x;
@@ -2599,8 +2611,10 @@ cudaError_t launch_fill(const Workspace& ws, const Surface* d_surf, cudaStream_t
 }
 
 cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, uint32_t ntiles,
-                          bool with_id, int threads, cudaStream_t st, uint32_t tiles_per_surface, uint32_t tile0) {
+                          bool with_id, int threads, cudaStream_t st, uint32_t tiles_per_surface, uint32_t tile0,
+                          const SceneDev* prep) {
   if (!ntiles) return cudaSuccess;
+  if (prep && (!ws.srec || !with_id || ws.tiles)) return cudaErrorInvalidValue;
   if (!with_id && ws.list && tiles_per_surface) {
     const uint32_t blocks = std::min<uint32_t>(ntiles, (uint32_t)num_sms() * (1280 / threads));
     switch (threads) {
@@ -2611,37 +2625,39 @@ cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t n
     return cudaGetLastError();
   }
   const int wid = with_id ? 1 : 0;
+  const uint32_t pb = prep ? std::min<uint32_t>((prep->ntris + threads - 1) / threads, (uint32_t)num_sms() * 4) : 0;
+  const SceneDev sc = prep ? *prep : SceneDev{};
   // surfaces of equal size: one grid row per surface, no search for the owner
   const dim3 grid = (tile0 == 0 && tiles_per_surface && nsurf > 1 && nsurf <= 65535 &&
-                     tiles_per_surface * nsurf == ntiles) ? dim3(tiles_per_surface, nsurf) : dim3(ntiles);
+                     tiles_per_surface * nsurf == ntiles) ? dim3(tiles_per_surface, nsurf) : dim3(ntiles + pb);
   if (with_id && ws.tiles) {
     switch (threads) {
-      case 128: k_raster<128, true, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-      case 512: k_raster<512, true, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-      default: k_raster<256, true, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0); break;
+      case 128: k_raster<128, true, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+      case 512: k_raster<512, true, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+      default: k_raster<256, true, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
     }
     return cudaGetLastError();
   }
   switch (threads * 2 + wid) {
-    case 256: k_raster<128, false><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-    case 257: k_raster<128, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-    case 1024: k_raster<512, false><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-    case 1025: k_raster<512, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-    case 513: k_raster<256, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0); break;
-    default: k_raster<256, false><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0); break;
+    case 256: k_raster<128, false><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+    case 257: k_raster<128, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+    case 1024: k_raster<512, false><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+    case 1025: k_raster<512, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+    case 513: k_raster<256, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+    default: k_raster<256, false><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
   }
   return cudaGetLastError();
 }
 
 cudaError_t launch_shade(const SceneDev& sc, const ViewParams* d_views, uint32_t nviews, const Surface* d_surf,
                          uint32_t ntiles, const Workspace& ws, cudaStream_t st, bool features, uint32_t tile0,
-                         const ViewParams* one_view, const Surface* one_surf) {
+                         const ViewParams* one_view, const Surface* one_surf, Counters* host_ctr) {
   if (!ntiles) return cudaSuccess;
   if (!sc.objq || !sc.texlv || !ws.srec || (nviews > 1 && !ws.tiles)) return cudaErrorInvalidValue;
   const bool one = nviews == 1 && one_view && one_surf;
   auto go = [&](auto kernel) {
     kernel<<<ntiles, kTilePixels, sizeof(float4) * kLightQuads * sc.nlights, st>>>(sc, one ? *one_view : ViewParams{}, one ? *one_surf : Surface{}, d_views, d_surf,
-                                   ws.srec, ws.ctr, ws.rec_cap, tile0, ws.tile_empty, ws.tiles);
+                                   ws.srec, ws.ctr, ws.rec_cap, tile0, ws.tile_empty, ws.tiles, host_ctr);
   };
   if (features)
     one ? go(k_shade<true, true>) : go(k_shade<true, false>);

@@ -294,10 +294,10 @@ inline bool pass_tile_table(bool view, const PassShape& sh) {
 }
 // Kernel launches of one pass (for the launch statistics): begin (clears and
 // object cull), setup, offsets, fill, raster, and when shading the shade
-// constants and kernel3.  The fused raster -> shade pass is one kernel for
+// constants (in the raster's launch for one view) and kernel3.  The fused raster -> shade pass is one kernel for
 // two; pipelined groups are two kernels per group.
 inline uint32_t pass_kernels(bool view, bool shade, const PassShape* sh = nullptr) {
-  uint32_t k = view && shade ? 7u : 5u;
+  uint32_t k = view && shade ? (sh && sh->nsurf == 1 ? 6u : 7u) : 5u;
   if (sh && sh->nseg) k -= 1;
   if (sh && sh->ngroups > 1) k += 2 * (sh->ngroups - 1);
   return k;
