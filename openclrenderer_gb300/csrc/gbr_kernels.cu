@@ -99,8 +99,7 @@ __device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, Raster
   const f3* p = c.p;
   f3 xpv = mk3(roundf(p[0].x), roundf(p[1].x), roundf(p[2].x));
   f3 ypv = mk3(roundf(p[0].y), roundf(p[1].y), roundf(p[2].y));
-  f3 depths = mk3(rcp(fdiv(p[0].z, kDepthFar)), rcp(fdiv(p[1].z, kDepthFar)),
-                  rcp(fdiv(p[2].z, kDepthFar)));
+  f3 depths = mk3(rcp(over_far(p[0].z)), rcp(over_far(p[1].z)), rcp(over_far(p[2].z)));
   *rc = rconstant(xpv, ypv);
   plane_const(depths, xpv, ypv, *rc, &R.A, &R.B, &R.C);
   EdgeTest e = make_edge(xpv.x, ypv.x, xpv.y, ypv.y, xpv.z, ypv.z);
@@ -292,12 +291,14 @@ __device__ __forceinline__ void write_rec(const Cand& c, uint32_t r, uint32_t su
 // and a minimum does not depend on order -- instead of becoming a record.
 constexpr float kDirectArea = 64.0f;
 
-// kernel1 of one small candidate into its surface's depth; returns the
-// covered pixel count.
-__device__ __forceinline__ uint32_t direct_raster(const Cand& c, uint32_t surface, const Surface& S) {
+// kernel1 of one small candidate into its cube face; returns the covered
+// pixel count.  (Rows narrowed to their exact spans, with no test per pixel,
+// were 5 % fewer instructions and 8 us slower on a 1M-triangle terrain: the
+// lanes' spans differ more than their rows.)
+__device__ __forceinline__ uint32_t direct_raster(const Cand& c, uint32_t* __restrict__ face) {
   RasterRec R;
   float rc;
-  make_rec(c, surface, R, &rc);
+  make_rec(c, 0u, R, &rc);
   const float4 q[3] = {make_float4(R.A, R.B, R.C, R.bound), make_float4(R.s0, R.sa, R.sb, 0.0f),
                        make_float4(R.t0, R.ta, R.tb, 0.0f)};
   const int x0 = (int)(R.xr & 0xFFFF), x1 = (int)(R.xr >> 16), y0 = (int)(R.yr & 0xFFFF), y1 = (int)(R.yr >> 16);
@@ -307,12 +308,12 @@ __device__ __forceinline__ uint32_t direct_raster(const Cand& c, uint32_t surfac
   // a bbox of at most 64 pixels has at most 64 rows)
   uint64_t skip = 0;
   if (!(R.kind & kRecTight))
-    skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, S.chunk) |
-           ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, S.chunk) << 32);
+    skip = (uint64_t)walk_skip_rows(R.xr, R.yr, y0, min(y1, y0 + 32), y0, kOpSizeLight) |
+           ((uint64_t)walk_skip_rows(R.xr, R.yr, y0 + 32, y1, y0 + 32, kOpSizeLight) << 32);
   for (int y = y0; y < y1; y++) {
     for (int x = x0 + (int)((skip >> (y - y0)) & 1u); x < x1; x++)
       if (rec_in_tri(q, (float)x, (float)y)) {
-        atomicMin(S.depth + (size_t)y * S.width + x, depth_at(R.A, R.B, R.C, (float)x, (float)y));
+        atomicMin(face + (y * kLightBufferDim + x), depth_at(R.A, R.B, R.C, (float)x, (float)y));
         hits++;
       }
   }
@@ -370,7 +371,7 @@ __device__ __forceinline__ void emit(const Cand& c, bool act, uint32_t surface, 
     const float chunk = (float)S.chunk;
     cnt.frags += c.area <= chunk ? 1u : (uint32_t)ceilf(fdiv(c.area, chunk));
   }
-  if (direct && c.box != kBoxEmpty) cnt.samples += direct_raster(c, surface, S);
+  if (direct && c.box != kBoxEmpty) cnt.samples += direct_raster(c, S.depth);
   if (!__any_sync(full, rec)) return;
   const bool store = rec && c.box != kBoxEmpty;
   Foot f{0, -1, 0, -1, false};

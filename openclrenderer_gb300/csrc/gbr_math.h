@@ -86,7 +86,13 @@ GBR_HD float fsqrt(float a) {
 #endif
 }
 GBR_HD float fma_(float a, float b, float c) { return fmaf(a, b, c); }
-GBR_HD float rcp(float x) { return fdiv(1.0f, x); }
+GBR_HD float rcp(float x) {
+#if defined(__CUDA_ARCH__)
+  return __frcp_rn(x);  // the same value as 1.0f / x, correctly rounded, for less
+#else
+  return 1.0f / x;
+#endif
+}
 // OpenCL float min/max are undefined for NaN operands; pinned to IEEE
 // minNum/maxNum (a NaN operand is ignored), which is what GPU min/max do.
 GBR_HD float fmin_(float x, float y) { return fminf(x, y); }
@@ -117,6 +123,14 @@ GBR_HD int32_t f2i_sat(float q) {
   if (q <= -2147483648.0f) return (-2147483647 - 1);
   return (int32_t)q;
 #endif
+}
+
+// fdiv(z, kDepthFar) for a vertex depth: with 1 / 350000 = hi + lo, RN(z * hi
+// + RN(z * lo)) is the correctly rounded quotient for every z from 1e-6 to 1e12
+// (tests/cpp/raster_rules_check.cpp goes through all of them).
+constexpr float kInvFarHi = 0x1.7f7aaep-19f, kInvFarLo = 0x1.658bb2p-45f;
+GBR_HD float over_far(float z) {
+  return z >= 1e-6f && z <= 1e12f ? fma_(z, kInvFarHi, z * kInvFarLo) : fdiv(z, kDepthFar);
 }
 
 // ---- pinned vector helpers (component order as OpenCL evaluates) ----------

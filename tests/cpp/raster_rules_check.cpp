@@ -4,7 +4,8 @@
 // depth_at and edge_inside at every pixel of random triangles' boxes; tight_box
 // and row_span against edge_inside at the pixels of their bbox4; ssao_tap against ssao_count
 // wherever ssao_exact holds; shadow_bias below kBiasFullCos; and shadow_limits
-// and depth_below against the tests they stand for; and the two-part 1 / 255.
+// and depth_below against the tests they stand for; and the two-part 1 / 255 and
+// 1 / 350000.
 // Usage: raster_rules_check W H <random boxes>; exit code 0 when all hold.
 #include <cmath>
 #include <cstdio>
@@ -151,6 +152,8 @@ int main(int argc, char** argv) {
   }
   for (int c = 0; c < 256; c++)
     shadow += fma_((float)c, kInv255Hi, (float)c * kInv255Lo) != fdiv((float)c, 255.0f);
+  // over_far for every depth of its range
+  for (float z = 1e-6f; z <= 1e12f; z = nextafterf(z, 1e30f)) shadow += over_far(z) != fdiv(z, kDepthFar);
   printf("cosines=%ld shadow=%ld\n", cosines, shadow);
   bad += cosines + shadow;
   printf("taps=%ld inexact=%ld wrong=%ld\n", taps, inexact, wrong);
