@@ -48,20 +48,21 @@ struct __align__(16) RasterRec {
   uint32_t kind;         // kRec*
 };
 
-// Per visible clipped triangle of a view: kernel3's per-triangle constants,
-// computed once by the fill (prep_shade) instead of at every pixel the
-// triangle owns (144 bytes).  Between the setup and the fill, a / e0 / e1
-// hold what the setup knows: the projected vertices (x, y, z) with rconst
-// and the triangle index in the w lanes.
+// Per stored record of a view: kernel3's per-triangle constants, computed once
+// (prep_shade) instead of at every pixel the triangle owns (144 bytes).
+// Between the setup and that, the first 48 bytes hold what the setup knows: the
+// projected vertices (x, y, z) with rconst and the triangle index in the w
+// lanes.  The order is the triangle's (position, normal, texture coordinate of
+// each vertex), so that prep_shade can work in place.
 struct __align__(16) ShadeRec {
   float4 a;      // barycentric frame: p1 = vertex 0 * scale (xyz), d00
-  float4 e0;     // p2 - p1 (xyz), d01
-  float4 e1;     // p3 - p1 (xyz), d11
-  float4 plane;  // get_vtdiff's 1/z plane DA, DB, DC; the frame's denom
   float4 n1;     // vertex normal 0 (xyz), vt0.x
+  float4 plane;  // get_vtdiff's 1/z plane DA, DB, DC; the frame's denom
+  float4 e0;     // p2 - p1 (xyz), d01
   float4 n2;     // vertex normal 1 (xyz), vt0.y
-  float4 n3;     // vertex normal 2 (xyz), vt1.x
   float4 t;      // vt1.y, vt2.x, vt2.y, object id | back-facing << 31 (bits)
+  float4 e1;     // p3 - p1 (xyz), d11
+  float4 n3;     // vertex normal 2 (xyz), vt1.x
   float4 col;    // vertex colours 0..2 (bits; colour 0 == 0: textured), triangle index (bits)
 };
 
