@@ -332,7 +332,7 @@ gbr_status gbr_scene_profile(gbr_scene* scene, int32_t enable);
 enum { GBR_PASS_SHADOW = 0, GBR_PASS_VIEW = 1 };
 
 typedef struct gbr_tuning {
-  int32_t raster_threads;  /* threads of one 16x16 raster tile: 128, 256 or 512 */
+  int32_t raster_threads;  /* threads of one 16x16 raster tile: 128 (64 in view passes of thousands of tiles), 256 or 512 */
   int32_t coarse_tile;     /* coarse bin edge in pixels: 64, 128 or 256 */
   int32_t fine_max_tiles;  /* records touching more 16x16 tiles go to coarse bins: 1..256 */
   float scratch_headroom;  /* record / bin scratch kept, as a multiple of the need: 1.05..4 */

@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // shared-memory atomicMin; pass 1 the minimum packed (key << 32 | record)
 // among tests within +-20 of the final depth.  Both are minima, so neither bin
 // order nor thread order changes the result.  Pass 0 keeps its covered pixels
-// in a list per warp (kHitCap, compacted in place when it fills: an entry 20
+// in a list per warp (hit_cap, compacted in place when it fills: an entry 20
 // or more behind the pixel's depth so far never passes), and pass 1 runs over
 // those lists; only a tile whose lists overflow all the same tests its records
 // again.
@@ -1008,11 +1008,26 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // (terrain).  Rows narrowed to spans instead of all pairs of the bbox: 64
 // sphere views 1.01 -> 0.97 ms, 4K 210 -> 191 us, cube faces with large walls
 // 141 -> 121 us, 1080p terrain 68 -> 67 us.
-constexpr int kHitCap = 256;  // entries of a warp's list: about 100 are used in a tile of 1.2 layers
-// 512-thread CTAs keep no lists (their static shared memory stays under 48 KB)
-// and re-test in the id pass.
+//
+// A view pass of many tiles (kManyWaves of them) takes CTAs of 64 threads for
+// the default 128: a warp's fixed work per tile is paid half as often, two
+// warps wait less for one another than four, and more tiles are in flight
+// behind the first loads of each.  At 128 and at 64 threads: 64 sphere views
+// (253k tiles) 981 and 763 us (instructions 784M and 591M), 4K (32k) 228 and
+// 185, nine ragged views (25k) 200 and 195, 1,000 screen-covering triangles at
+// 1440p (14k) 360 to 460 and 305, 1080p (8k) 80 and 84, 1279x721 (3.7k) 30.5
+// and 33.4: the last wave counts there.
+constexpr uint32_t kManyWaves = 4;
+// Entries of a warp's list: about 100 are used in a tile of 1.2 layers by each
+// of four warps, and twice that by each of two.  512-thread CTAs keep no lists
+// (their static shared memory stays under 48 KB) and re-test in the id pass.
 template <int NT>
-__host__ __device__ constexpr int raster_hits() { return NT <= 256 ? kHitCap * (NT / 32) : 0; }
+__host__ __device__ constexpr int hit_cap() { return NT == 64 ? 352 : 256; }
+template <int NT>
+__host__ __device__ constexpr int raster_hits() { return NT <= 256 ? hit_cap<NT>() * (NT / 32) : 0; }
+// View CTAs per SM, by registers and (64 threads) shared memory.
+template <int NT>
+__host__ __device__ constexpr int raster_ctas() { return NT == 64 ? 15 : 1024 / NT; }
 // A list entry's second word: pixel | record << 8, so records below 2^24
 // (passes with room for more re-test tiles of several chunks).
 constexpr uint32_t kHitRecords = 1u << 24;
@@ -1105,7 +1120,7 @@ struct RasterSmem {
   uint16_t sskip[NT];
   // the covered pixels of pass 0 kept for the id pass: depth, and pixel |
   // record << 8 (the staged slot in one-chunk tiles, else the pass's record);
-  // warp w's list at w * kHitCap
+  // warp w's list at w * hit_cap
   uint2 hits[ID && raster_hits<NT>() ? raster_hits<NT>() : 1];
   uint32_t sdepth[kTilePixels];
   unsigned long long sid[kTilePixels];
@@ -1232,7 +1247,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   const bool packed = with_id && resident && ws.pack_keys;
   uint32_t* sid32 = reinterpret_cast<uint32_t*>(sid);
   // the warp's list of covered pixels and its length
-  uint2* hits = sm.hits + warp * (with_id && raster_hits<NT>() ? kHitCap : 0);
+  uint2* hits = sm.hits + warp * (with_id && raster_hits<NT>() ? hit_cap<NT>() : 0);
   uint32_t nh = 0;
   bool listing = with_id && raster_hits<NT>() > 0 && (resident || ws.rec_cap <= kHitRecords);
   uint32_t wsamples = 0;  // covered tests of pass 0 seen by this warp
@@ -1416,9 +1431,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             const uint32_t n0 = (uint32_t)__popc(b0), n1 = (uint32_t)__popc(b1);
             if (pass == 0) {
               wsamples += n0 + n1;
-              if (listing && nh + n0 + n1 > (uint32_t)kHitCap) {  // warp-uniform
+              if (listing && nh + n0 + n1 > (uint32_t)hit_cap<NT>()) {  // warp-uniform
                 nh = compact_hits(hits, nh, sdepth);
-                listing = nh + n0 + n1 <= (uint32_t)kHitCap;
+                listing = nh + n0 + n1 <= (uint32_t)hit_cap<NT>();
               }
             }
             auto resolve = [&](float px, int pp, uint32_t slot) {
@@ -1472,9 +1487,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
 // prep_blocks (one view that shades): the first blocks of the grid compute the
 // shade constants instead, beside the tiles, which do not read them.
 template <int NT, bool ID, bool CC = false>
-__global__ void __launch_bounds__(NT, (ID ? 1024 : 1280) / NT) k_raster(Workspace ws, const Surface* __restrict__ surfs,
-                                                          uint32_t nsurf, uint32_t tile0, uint32_t prep_blocks,
-                                                          const __grid_constant__ SceneDev sc) {
+__global__ void __launch_bounds__(NT, ID ? raster_ctas<NT>() : 1280 / NT)
+    k_raster(Workspace ws, const Surface* __restrict__ surfs, uint32_t nsurf, uint32_t tile0, uint32_t prep_blocks,
+             const __grid_constant__ SceneDev sc) {
   __shared__ RasterSmem<NT, ID> sm;
   if (ws.ctr->overflow) return;
   if (ID && !CC && blockIdx.x < prep_blocks) {
@@ -2677,28 +2692,35 @@ cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t n
     }
     return cudaGetLastError();
   }
-  const int wid = with_id ? 1 : 0;
+  if (with_id && threads == 128 && ntiles >= kManyWaves * num_sms() * raster_ctas<64>()) threads = 64;
   const uint32_t pb = prep ? std::min<uint32_t>((prep->ntris + threads - 1) / threads, (uint32_t)num_sms() * 4) : 0;
   const SceneDev sc = prep ? *prep : SceneDev{};
   // surfaces of equal size: one grid row per surface, no search for the owner
   const dim3 grid = (tile0 == 0 && tiles_per_surface && nsurf > 1 && nsurf <= 65535 &&
                      tiles_per_surface * nsurf == ntiles) ? dim3(tiles_per_surface, nsurf) : dim3(ntiles + pb);
+#define GBR_RASTER(NT, ...) k_raster<NT, __VA_ARGS__><<<grid, NT, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc)
   if (with_id && ws.tiles) {
     switch (threads) {
-      case 128: k_raster<128, true, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-      case 512: k_raster<512, true, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-      default: k_raster<256, true, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
+      case 64: GBR_RASTER(64, true, true); break;
+      case 128: GBR_RASTER(128, true, true); break;
+      case 512: GBR_RASTER(512, true, true); break;
+      default: GBR_RASTER(256, true, true); break;
     }
-    return cudaGetLastError();
+  } else if (with_id) {
+    switch (threads) {
+      case 64: GBR_RASTER(64, true); break;
+      case 128: GBR_RASTER(128, true); break;
+      case 512: GBR_RASTER(512, true); break;
+      default: GBR_RASTER(256, true); break;
+    }
+  } else {
+    switch (threads) {
+      case 128: GBR_RASTER(128, false); break;
+      case 512: GBR_RASTER(512, false); break;
+      default: GBR_RASTER(256, false); break;
+    }
   }
-  switch (threads * 2 + wid) {
-    case 256: k_raster<128, false><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-    case 257: k_raster<128, true><<<grid, 128, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-    case 1024: k_raster<512, false><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-    case 1025: k_raster<512, true><<<grid, 512, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-    case 513: k_raster<256, true><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-    default: k_raster<256, false><<<grid, 256, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc); break;
-  }
+#undef GBR_RASTER
   return cudaGetLastError();
 }
 

@@ -111,3 +111,27 @@ def test_coarse_records(n):
     st, cap = gs.stats(), 4 * (n + 1024)
     assert st["retries"] == 0 and st["view_records"] == n and (st["view_bin_entries"] + n > cap) == (n == 9000)
     gs.close()
+
+
+@pytest.mark.parametrize("sizes", [[(2001, 1239)], [(1500, 1100), (1201, 907)]])
+@pytest.mark.parametrize("n_big,n_small,gap", [(1, 40, 1.0), (3, 4000, 50.0), (70, 300, 5.0), (140, 0, 0.0)])
+def test_many_tiles(sizes, n_big, n_small, gap):
+    """Passes of more than 9,120 tiles (CTAs of 64 threads) against those of 256: one view, and views of two sizes."""
+    w, h = sizes[0]
+    sc = layers(w, h, n_big, n_small, gap, seed=n_big)
+    gs = GpuScene(sc)
+    cams, views = [sc.cameras[0]] * len(sizes), [S.make_view(a, b, 90.0) for a, b in sizes]
+    outs, samples = {}, {}
+    for threads in (256, 128):
+        gs.set_tuning(S.PASS_VIEW, raster_threads=threads)
+        if len(sizes) == 1:
+            outs[threads] = [gs.render(cams[0], views[0], normals=True).numpy()]
+        else:
+            outs[threads] = [o.numpy() for o in gs.render_batch(cams, views)]
+        samples[threads] = gs.stats()["view_samples"]
+    assert samples[128] == samples[256]
+    for a, b in zip(outs[256], outs[128]):
+        assert (a["depth"] != 0xFFFFFFFF).any()
+        for k in a:
+            assert np.array_equal(a[k], b[k]), k
+    gs.close()
