@@ -1033,12 +1033,24 @@ __host__ __device__ constexpr int raster_ctas() { return NT == 64 ? 15 : 1024 / 
 constexpr uint32_t kHitRecords = 1u << 24;
 constexpr uint32_t kSlotBits = 9;  // staged slots of a one-chunk tile: below 512
 
+// Barrier of a tile's NT threads: the block, or (PART) one of its groups.
+template <int NT, bool PART>
+__device__ __forceinline__ void tile_barrier() {
+  if (!PART)
+    __syncthreads();
+  else if (threadIdx.x < NT)  // (constant numbers: with one in a register a block holds all 16 barriers)
+    asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
+}
+
 // Exclusive block scan with a single barrier: each warp scans its lanes,
 // publishes its total, and after the barrier every thread adds up the totals
 // of the warps before its own (and of all warps, the block total).
-template <int NT>
+// The NT threads are a block, or (PART) one of the block's groups of NT.
+template <int NT, bool PART>
 __device__ __forceinline__ uint32_t block_excl_scan1(uint32_t v, uint32_t* swarp, uint32_t* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x & (NT - 1)) >> 5;
   uint32_t incl = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1046,7 +1058,7 @@ __device__ __forceinline__ uint32_t block_excl_scan1(uint32_t v, uint32_t* swarp
     if (lane >= o) incl += t;
   }
   if (lane == 31) swarp[warp] = incl;
-  __syncthreads();
+  tile_barrier<NT, PART>();
   uint32_t before = 0, all = 0;
 #pragma unroll
   for (int w = 0; w < NT / 32; w++) {
@@ -1133,14 +1145,16 @@ struct RasterSmem {
   uint32_t lists[4];
 };
 
-// NT threads per CTA (128, 256 or 512); ID: resolve the canonical id too
+// NT threads per tile: a CTA of 64, 128, 256 or 512, or (PART) one of a CTA's
+// two halves of 64; ID: resolve the canonical id too
 // (views) or only the depth (cube faces); CC: see chunk below.  surface: the
 // tile's surface when the caller knows it, else -1 (ws.tiles, or the pass's
 // only surface).  Every thread of the block calls it; the caller synchronises
 // before reusing the shared memory.
-template <int NT, bool ID, bool CC = false>
+template <int NT, bool ID, bool CC = false, bool PART = false>
 __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* __restrict__ surfs, uint32_t nsurf,
                                             uint32_t tile, int surface, RasterSmem<NT, ID>& sm) {
+  static_assert(!(ID && PART), "the id pass votes across the block");
   constexpr bool with_id = ID;
   constexpr int NW = NT / 32;
   constexpr uint32_t kCountShift = 18;  // scan word: pixels (< 2^18) | records << 18
@@ -1156,7 +1170,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   uint32_t& ssamples = sm.ssamples;
   Surface& S = sm.S;
   uint32_t* lists = sm.lists;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x & (NT - 1), lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {  // the tile's surface and bins
     const uint32_t fcnt = ws.fine_count[tile], foff = ws.fine_off[tile] - fcnt, ftot = ws.ctr->fine_total;
     uint32_t s, ct;
@@ -1186,7 +1200,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       sid[p] = ~0ull;
     }
   }
-  __syncthreads();
+  tile_barrier<NT, PART>();
   const uint32_t lt = tile - S.tile_base;
   const int tx0 = (lt % S.tiles_x) * kTile, ty0 = (lt / S.tiles_x) * kTile;
   if (with_id && lists[1] + lists[3] == 0) {  // no records: an empty tile
@@ -1276,7 +1290,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
         break;
       }
       if (!(resident && pass == 1)) {
-        if (pass != 0 || c0 != 0) __syncthreads();  // the previous chunk's readers are done
+        if (pass != 0 || c0 != 0) tile_barrier<NT, PART>();  // the previous chunk's readers are done
         uint32_t rows = 0, r = 0, geo = 0, skip = 0;
         int bx0 = 0, bx1 = 0, by0 = 0, by1 = 0;
         float4 q0, q1, q2, q3;
@@ -1331,7 +1345,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
         }
         const uint32_t word = rows ? (rows | (1u << kCountShift)) : 0u;
         uint32_t tot = 0;
-        const uint32_t off = block_excl_scan1<NT>(word, swarp, &tot);
+        const uint32_t off = block_excl_scan1<NT, PART>(word, swarp, &tot);
         if (rows) {
           const uint32_t slot = off >> kCountShift;
           srec[0][slot] = q0;
@@ -1347,7 +1361,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
           soff[tot >> kCountShift] = tot & ((1u << kCountShift) - 1);
           sscan = tot;
         }
-        __syncthreads();
+        tile_barrier<NT, PART>();
       }
       const uint32_t nstaged = sscan >> kCountShift;
       const uint32_t total = soff[nstaged];
@@ -1463,7 +1477,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
     if (with_id && pass == 0)
       cached = __syncthreads_and(listing) != 0;
     else
-      __syncthreads();
+      tile_barrier<NT, PART>();
   }
   if (tid == 0 && ssamples) atomicAdd(&ws.ctr->samples, (unsigned long long)ssamples);
   for (int lp = tid; lp < kTilePixels; lp += NT) {
@@ -1509,15 +1523,34 @@ __global__ void __launch_bounds__(NT, ID ? raster_ctas<NT>() : 1280 / NT)
 // The tiles of ws.list (surfaces of per_surface tiles each) of a depth-only
 // pass, by as many blocks as fit at once: 24,576 tiles of a cubemap of which
 // some 4,000 have records took 30 us as a block each, mostly to start them.
+// A long list (kPartWaves tiles a block of 128) goes to the blocks' halves, a
+// tile each, as in view passes of many tiles: three lights among large walls
+// 123 -> 98 us.  A list of some 6,000 tiles took 32.5 us by blocks and 34.8 by
+// halves, one that the blocks take at once (4K) 13.5 and 17.
+constexpr uint32_t kPartWaves = 6;
+constexpr int kPart = 64;
 template <int NT>
 __global__ void __launch_bounds__(NT, 1280 / NT) k_raster_list(Workspace ws, const Surface* __restrict__ surfs,
                                                                uint32_t nsurf, uint32_t per_surface) {
-  __shared__ RasterSmem<NT, false> sm;
+  constexpr uint32_t kParts = NT == 128 ? NT / kPart : 1;
+  __shared__ union {
+    RasterSmem<NT, false> one;
+    RasterSmem<kPart, false> part[kParts];
+  } sm;
   if (ws.ctr->overflow) return;
   const uint32_t n = ws.ctr->nlist;
+  if (kParts > 1 && n >= kPartWaves * gridDim.x) {
+    const uint32_t part = threadIdx.x / kPart % kParts;
+    for (uint32_t i = kParts * blockIdx.x + part; i < n; i += kParts * gridDim.x) {
+      const uint32_t tile = ws.list[i];
+      raster_tile<kPart, false, false, true>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm.part[part]);
+      tile_barrier<kPart, true>();
+    }
+    return;
+  }
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint32_t tile = ws.list[i];
-    raster_tile<NT, false>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm);
+    raster_tile<NT, false>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm.one);
     __syncthreads();  // the next tile reuses the shared memory
   }
 }

@@ -135,3 +135,33 @@ def test_many_tiles(sizes, n_big, n_small, gap):
         for k in a:
             assert np.array_equal(a[k], b[k]), k
     gs.close()
+
+
+@pytest.mark.parametrize("n_lights", [1, 2])
+def test_many_cube_face_tiles(n_lights):
+    """Lights in a room whose walls cover every tile of every face: lists of 24,576 tiles and more, by halves of a block."""
+    rng = np.random.default_rng(n_lights)
+    tl, size, cells = [], 3000.0, 12  # (a triangle goes to the faces its vertices lie in, so walls of many)
+    for axis in range(3):
+        for side in (-size, size):
+            for cell in range(cells * cells):
+                for tri in ((0, 1, 2), (1, 3, 2)):
+                    t = []
+                    for k in tri:
+                        v = np.full(3, side)
+                        v[(axis + 1) % 3] = size * (2 * (cell % cells + (k & 1)) / cells - 1)
+                        v[(axis + 2) % 3] = size * (2 * (cell // cells + (k >> 1)) / cells - 1)
+                        t.append(tuple(v))
+                    tl.append(t)
+    for _ in range(60):
+        c = rng.uniform(-size, size, 3)
+        tl.append([tuple(c + rng.uniform(-400, 400, 3)) for _ in range(3)])
+    sc = tri_scene(tl, 64, 48, descs=np.stack(TWO_SIDED),
+                   lights=np.stack([S.make_light((40.0 * i, -30.0 * i, 25.0), radius=9000.0, shadow=1)
+                                    for i in range(n_lights)]))
+    gs = GpuScene(sc)
+    gs.shadow_pass()
+    dyn, _ = O.shadow(sc)
+    assert (dyn != 0xFFFFFFFF).mean() > 0.9
+    assert np.array_equal(gs.cubemaps()[:len(dyn)], dyn)
+    gs.close()
