@@ -1,18 +1,23 @@
 // gbr_internal.h — device data layout and kernel launchers of the pipeline.
 //
 // Work flow of one pass (views or cube faces):
-//   setup   1 thread per (triangle, surface group): transform, clip, cull,
+//   begin   clears the counters (views: and tests each object against each
+//           view; cube faces: and clears the faces)
+//   setup   1 thread per (triangle, view or light): transform, clip, cull,
 //           bbox; appends RasterRecs (warp-aggregated atomics) and counts the
 //           16x16 "fine" tiles (or 128x128 "coarse" tiles for large
-//           triangles) each record touches
-//   scan    exclusive scan of the tile counts -> bin offsets
+//           triangles) each record touches; small triangles of cube faces are
+//           rasterised here
+//   offsets every tile's bin gets its place
 //   fill    record indices into per-tile bins
-//   raster  1 CTA per fine tile, 1 thread per pixel: loops over the tile's
-//           fine bin and its coarse tile's bin; resolves the minimum depth in
-//           registers (kernel1), then the canonical id (kernel2).  Every pixel
-//           of a surface is written exactly once, so no clear pass and no
-//           global atomics are needed.
-//   shade   1 thread per view pixel (kernel3)
+//   raster  1 CTA per fine tile: lays the rows of its records (fine bin, then
+//           its coarse tile's) end to end, narrows them to spans and tests
+//           their pixels; resolves the minimum depth in shared memory
+//           (kernel1), then the canonical id (kernel2).  Every pixel of a view
+//           is written exactly once, so no clear pass and no global atomics
+//           are needed there.
+//   shade   kernel3's per-triangle constants (prep_shade: beside the raster),
+//           then 1 thread per view pixel (kernel3)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -184,7 +189,7 @@ struct Workspace {
   uint2* tiles;
   uint32_t* list;       // depth-only passes: the fine tiles that have records (Counters::nlist), or null
   uint32_t ncounts;     // words from ctr on that a pass starts by clearing
-  const uint32_t* vis;  // views: object cull bits (k_object_cull), vis_words per view, or null
+  const uint32_t* vis;  // views: object cull bits (k_begin_views), vis_words per view, or null
   uint32_t vis_words;
   uint32_t pack_keys;   // views: every key (2 * triangle + 1) is below 2^23 - 1 (32-bit id resolve)
   // Views that shade, raster and kernel3 in separate launches: the raster

@@ -642,7 +642,9 @@ __device__ __noinline__ void emit_second(const SceneDev& sc, const Workspace& ws
   setup_add(sums, cnt);
 }
 
-// prearrange (cl2.cl:4271-4409), one thread per (triangle, view).
+// prearrange (cl2.cl:4271-4409), one thread per (triangle, view).  Bound by
+// latency and issue together (51 % active, 45 % of the warps; more CTAs per SM
+// spill): 1M-triangle terrain 36 us, 64 views of 500k triangles 280 us.
 __global__ void __launch_bounds__(256, 5) k_setup_views(const __grid_constant__ SceneDev sc,
                                                      const ViewParams* __restrict__ views,
                                                      const Surface* __restrict__ surfs,
@@ -654,7 +656,7 @@ __global__ void __launch_bounds__(256, 5) k_setup_views(const __grid_constant__ 
   const ViewParams& V = views[blockIdx.y];
   const Surface& S = surfs[V.surface];
   SetupCounts cnt;
-  // the object cull (k_object_cull), when the pass has one, includes the
+  // the object cull (k_begin_views), when the pass has one, includes the
   // reference's own object test.  A pass of one view reads the whole triangle
   // at once (two rounds of loads); a pass of many views, which skips most
   // objects in each, reads the object id alone first.
@@ -694,6 +696,9 @@ __global__ void __launch_bounds__(256, 5) k_setup_views(const __grid_constant__ 
 }
 
 // prearrange_realtime_shadowing (cl2.cl:4419-4636), one thread per (triangle, light job).
+// Bound by the direct rasters: lanes' boxes differ (20 of 32 active) and their
+// atomics wait; 52 % issue active.  1M-triangle terrain 136 -> 76 us;
+// 128 x 7 measured best of blocks of 32 to 256 threads.
 __global__ void __launch_bounds__(128, 7) k_setup_shadow(const __grid_constant__ SceneDev sc,
                                                       const ShadowJob* __restrict__ jobs,
                                                       const Surface* __restrict__ surfs,

@@ -269,19 +269,19 @@ void shadow_layout(gbr_scene* s, bool with_static, int coarse_shift, std::vector
                    std::vector<Surface>& surfs, PassShape& sh);
 // Scratch of a pass sized to the memory's targets (no allocation when it fits).
 gbr_status reserve_pass(WorkMem& w, const PassShape& sh, bool view);
-// Launches of one pass on the pass's scratch: counter clears, setup, scan,
-// fill and raster on geom, then (views) shade and the read-back of the
-// counters into host_ctr on st.  When geom differs from st, join is recorded
+// Launches of one pass on the pass's scratch: begin, setup, offsets, fill and
+// raster on geom, then (views) shade on st and the counters into host_ctr
+// (read back, or written by kernel3 in passes of one view).  When geom differs from st, join is recorded
 // on geom after the raster and st waits for it before shading, so the
 // geometry can run beside whatever st does first (the shadow pass).
 // Allocates nothing, so it can be captured into a graph.  ev, when not null,
 // holds the stage events (profiling): [0..4] around the geometry stages,
 // [5] after shading, [6] before shading.
 //
-// side (views that shade): the shade constants (launch_prep) run on
-// side.stream after the setup, forked by side.fork on geom, and shading
-// waits for side.join, so they overlap the scan, fill and raster; without a
-// side stream they run on geom after the raster.
+// The shade constants (views that shade) run in the raster's launch when the
+// pass has one view.  Otherwise (launch_prep) on side.stream, forked by
+// side.fork on geom after the fill, and shading waits for side.join, so they
+// overlap the raster; without a side stream on geom after the raster.
 gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, const PassShape& sh,
                        Counters* host_ctr, cudaEvent_t* ev, cudaStream_t st, cudaStream_t geom = nullptr,
                        cudaEvent_t join = nullptr, const SideStream* side = nullptr);
@@ -294,8 +294,9 @@ inline bool pass_tile_table(bool view, const PassShape& sh) {
 }
 // Kernel launches of one pass (for the launch statistics): begin (clears and
 // object cull), setup, offsets, fill, raster, and when shading the shade
-// constants (in the raster's launch for one view) and kernel3.  The fused raster -> shade pass is one kernel for
-// two; pipelined groups are two kernels per group.
+// constants (in the raster's launch for one view) and kernel3.  The fused
+// raster -> shade pass is one kernel for two; pipelined groups are two kernels
+// per group.
 inline uint32_t pass_kernels(bool view, bool shade, const PassShape* sh = nullptr) {
   uint32_t k = view && shade ? (sh && sh->nsurf == 1 ? 6u : 7u) : 5u;
   if (sh && sh->nseg) k -= 1;
