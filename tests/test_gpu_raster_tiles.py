@@ -165,3 +165,21 @@ def test_many_cube_face_tiles(n_lights):
     assert (dyn != 0xFFFFFFFF).mean() > 0.9
     assert np.array_equal(gs.cubemaps()[:len(dyn)], dyn)
     gs.close()
+
+
+@pytest.mark.parametrize("offset", [0, 4, 2])
+def test_ids_into_pinned_memory(offset):
+    """Host ids written by the raster itself (pinned, 4-byte aligned) or copied (2 bytes off): the same, and no others."""
+    w, h = 333, 257
+    sc = layers(w, h, 1, 200, 40.0, seed=3)
+    sc.tris = sc.tris[1:]  # (some tiles stay empty)
+    gs = GpuScene(sc)
+    dev = gs.render(sc.cameras[0], sc.views[0]).numpy()
+    raw = torch.empty(4 * w * h + 16, dtype=torch.uint8, pin_memory=True).numpy()
+    raw[:] = 0xA5
+    ids = raw[offset:offset + 4 * w * h].view(np.uint32)
+    for _ in range(2):
+        got = gs.render_host(sc.cameras[0], sc.views[0], ids=ids)
+        assert np.array_equal(ids.reshape(h, w), dev["id"]) and np.array_equal(got["depth"], dev["depth"])
+    assert (raw[:offset] == 0xA5).all() and (raw[offset + 4 * w * h:] == 0xA5).all()
+    gs.close()
