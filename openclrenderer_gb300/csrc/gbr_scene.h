@@ -303,8 +303,8 @@ inline uint32_t pass_kernels(bool view, bool shade, const PassShape* sh = nullpt
   if (sh && sh->ngroups > 1) k += 2 * (sh->ngroups - 1);
   return k;
 }
-// Timed stages of one pass (stage_ms): setup (a depth-only pass's clear
-// included), scan, fill, raster and, for views, shade.
+// Timed stages of one pass (stage_ms): setup (the begin kernel
+// included), scan (the bin offsets), fill, raster and, for views, shade.
 inline uint32_t pass_stages(bool view) { return view ? 5u : 4u; }
 // Record a finished pass's counters in the scene's statistics; on overflow
 // grow the memory's targets by the tuning's headroom and return false.
