@@ -42,11 +42,11 @@ __device__ __forceinline__ uint32_t agg_inc(uint32_t* counter, uint32_t key, boo
 // Colour-only arithmetic of the light loop: every use below feeds the colour
 // continuously (no comparison, rounding or index depends on it), so the
 // approximate division is covered by the 1/255 colour tolerance.  The
-// hardware's approximations, taken as single instructions: __fdividef,
-// rsqrtf and __expf compute the same values but wrap them in three or four
-// more for subnormal operands and results, which here are either exact zeros
-// or far below a colour level.  (1080p kernel3 3,350 -> 3,060 instructions
-// per pixel, 223 -> 210 us.)
+// hardware's approximations, taken as single instructions that flush subnormal
+// operands and results to 0: a flushed result is far below a colour level, and
+// where an operand can be subnormal (csqrt) it is dealt with.  (1080p kernel3
+// 3,350 -> 3,060 instructions per pixel, 223 -> 210 us, against __fdividef,
+// rsqrtf and __expf.)
 __device__ __forceinline__ float ex2_ftz(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -1865,12 +1865,13 @@ __device__ __forceinline__ float c_rational_acos(float x) {
 }
 
 
-// Colour-only square root: 0 for 0, NaN for a negative input.  (An infinite
-// input gives NaN as well; gamma_inv's sum of infinities of both signs is NaN
-// either way.)
+// Colour-only square root: 0 for 0 and for subnormals (whose root is below
+// 1.1e-19; rsqrt_ftz takes them for 0, and x * inf is infinite), NaN for a
+// negative normal input.  (An infinite input gives NaN as well; gamma_inv's sum
+// of infinities of both signs is NaN either way.)
 __device__ __forceinline__ float csqrt(float x) {
   const float s = x * rsqrt_ftz(x);
-  return x == 0.0f ? 0.0f : s;
+  return fabsf(x) < 1.17549435e-38f ? 0.0f : s;
 }
 // gamma_inv (cl2.cl:5778-5782) on the colour path.
 __device__ __forceinline__ float c_gamma_inv(float c) {
