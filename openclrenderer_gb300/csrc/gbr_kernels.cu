@@ -1103,6 +1103,7 @@ __device__ __forceinline__ uint32_t pack_rgba(float r, float g, float b, float a
 __device__ __noinline__ uint32_t compact_hits(uint2* hits, uint32_t n, const uint32_t* sdepth) {
   const int lane = threadIdx.x & 31;
   uint32_t kept = 0;
+  __syncwarp();  // the entries are other lanes' stores, and a vote orders no memory
   for (uint32_t g0 = 0; g0 < n; g0 += 32) {
     const uint32_t g = g0 + lane;
     uint2 e = make_uint2(0, 0);
