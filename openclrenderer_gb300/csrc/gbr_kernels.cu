@@ -1901,17 +1901,17 @@ constexpr float kLightCutoff = 0.1f;
 // margins below cover the approximate colour-path arithmetic of that test
 // (relative errors of a few 1e-7).  -1: always under the cutoff; +inf: no
 // early test (shadow lights, whose cutoff decides the cubemap later shadow
-// lights read); the largest float: only infinite distances (degenerate radii,
-// whose attenuation is then under the cutoff too).  A NaN position makes the
-// reciprocal radius NaN, and with it the attenuation.
+// lights read, and lights whose radius or brightness is not finite); at most
+// the largest float for all others: a squared distance that overflows is past
+// any finite radius.
 constexpr int kLightQuads = 3;
 __device__ __forceinline__ void stage_light(const gbr_light* L, bool linear, float4* dst) {
   f3 c = mk3(L->col[0], L->col[1], L->col[2]);
   if (linear) c = mk3(gamma_fwd(c.x), gamma_fwd(c.y), gamma_fwd(c.z));
   const float radius = L->radius, brightness = L->brightness;
   const float b10 = 10.0f * brightness;
-  float cut2 = L->shadow ? __int_as_float(0x7F800000) : 3.4028235e38f;
-  const float psum = L->pos[0] + L->pos[1] + L->pos[2];
+  const float largest = 3.4028235e38f;
+  float cut2 = __int_as_float(0x7F800000);
   if (!L->shadow && radius > 0.0f && b10 == b10) {
     if (b10 <= 1.0f) {
       cut2 = -1.0f;
@@ -1920,12 +1920,13 @@ __device__ __forceinline__ void stage_light(const gbr_light* L, bool linear, flo
       cut2 = (rs * rs) * 1.00001f;
     }
   }
+  if (!L->shadow && fabsf(radius) <= largest && fabsf(b10) <= largest) cut2 = fmin_(cut2, largest);
   // lights without shadows fold kernel3's cutoff into the brightness:
   // (b / tt^2 - 0.1) / 0.9 = (b / 0.9) / tt^2 - 0.1 / 0.9 (colour only)
   const float bw = L->shadow ? brightness : brightness * (1.0f / (1.0f - kLightCutoff));
   dst[0] = make_float4(L->pos[0], L->pos[1], L->pos[2], cut2);
   dst[1] = make_float4(c.x, c.y, c.z, bw);
-  dst[2] = make_float4(radius, psum == psum ? __fdividef(1.0f, radius) : psum, L->diffuse,
+  dst[2] = make_float4(radius, __fdividef(1.0f, radius), L->diffuse,
                        __uint_as_float((L->shadow ? 1u : 0u) | (L->is_static ? 2u : 0u)));
 }
 
@@ -2192,9 +2193,10 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
       continue;
     }
     // a light without shadows: its occlusion is 1
-    // the approximate square root (0 * inf is NaN, which the maximum turns into
-    // 0; infinite distances are past every cut2)
-    const float distance = fmax_(d2 * rinv, 0.0f);
+    // the approximate square root: 2^63 is the reciprocal root of the smallest
+    // normal float, so the minimum only matters at 0 (and at subnormals), where
+    // rinv is infinite; infinite and NaN squares give NaN
+    const float distance = d2 * fmin_(rinv, 0x1p63f);
     const float tt = fma_(distance, LC.y, 1.0f);
     float illum = fma_(LB.w, crcp(tt * tt), -kLightCutoff / (1.0f - kLightCutoff));
     // at most 0 only between the cutoff and the conservative early test: such a

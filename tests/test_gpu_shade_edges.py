@@ -45,3 +45,16 @@ def test_outline_over_subnormal_colour(specular):
     sc.views = [S.make_view(w, h, 90.0, flags=S.VIEW_OUTLINE)]
     rgba = compare(sc)
     assert (rgba[..., 1] > 3).mean() > 0.5  # the outline, in a channel that the texture leaves at 0
+
+
+@pytest.mark.parametrize("pos,radius", [((0.0, 0.0, -3.0e19), 2.0e19), ((2.0e20, 1.0e20, 0.0), 1.0e20),
+                                        ((0.0, 5.0e18, -5.0e18), 1.0e19), ((0.0, -1.0e25, 0.0), 3.0e30),
+                                        ((0.0, 1.0e19, -1.0e19), -1.0e19), ((3.0e20, 0.0, 0.0), -1.0e19)])
+@pytest.mark.parametrize("shadow", [0, 1])
+def test_lights_farther_than_a_square_can_hold(pos, radius, shadow):
+    """Distances whose squares overflow, or come close, are as dark as the oracle has them."""
+    w, h = 200, 150
+    sc = plane(w, h, 300.0, 900.0, descs=np.stack([S.make_descriptor(tid=0)]),
+               lights=np.stack([S.make_light(pos, radius=radius, brightness=1.0, shadow=shadow),
+                                S.make_light((0.0, 0.0, 10.0), radius=600.0)]))
+    compare(sc)
