@@ -2198,10 +2198,10 @@ __device__ void shade_covered(const SceneDev& sc, const ViewParams& V, const Sur
     // rinv is infinite; infinite and NaN squares give NaN
     const float distance = d2 * fmin_(rinv, 0x1p63f);
     const float tt = fma_(distance, LC.y, 1.0f);
-    float illum = fma_(LB.w, crcp(tt * tt), -kLightCutoff / (1.0f - kLightCutoff));
-    // at most 0 only between the cutoff and the conservative early test: such a
-    // light then adds exactly nothing (a select, not another divergent exit)
-    illum = illum <= 0.0f ? 0.0f : illum;
+    const float illum = fma_(LB.w, crcp(tt * tt), -kLightCutoff / (1.0f - kLightCutoff));
+    // (turned into 0 by a select instead: 1080p frame 395 us against 391, and a
+    // NaN specular term of a dark light cleared the sum of the others)
+    if (illum <= 0.0f) continue;
     ptl = mul3s(ptl, rinv);
     const float light = fmax_(cdot3(ptl, lnormal), 0.0f);
     const float dscale = fma_(amb1, light, ambient) * ((LC.z * g_diffuse) * illum);

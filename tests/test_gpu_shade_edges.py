@@ -58,3 +58,19 @@ def test_lights_farther_than_a_square_can_hold(pos, radius, shadow):
                lights=np.stack([S.make_light(pos, radius=radius, brightness=1.0, shadow=shadow),
                                 S.make_light((0.0, 0.0, 10.0), radius=600.0)]))
     compare(sc)
+
+
+@pytest.mark.parametrize("radius", [0.0, -1000.0])
+def test_dark_lights_opposite_the_eye(radius):
+    """Lights that add nothing, right behind the surface as the eye sees it, leave another light's highlight alone."""
+    w, h = 300, 300
+    rng = np.random.default_rng(2)
+    dark = [S.make_light((*rng.uniform(-3e4, 3e4, 2), 4.0e6), radius=radius) for _ in range(60)]
+    sc = plane(w, h, 900.0, 900.0, lights=np.stack([S.make_light((0.0, 0.0, 10.0), radius=4000.0, brightness=8.0)] + dark))
+    sc.tex_pixels = [np.tile(np.array([0, 0, 0, 255], np.uint8), (64, 64, 1))]
+    sc.views = [S.make_view(w, h, 1.0)]
+    for t in sc.tris:  # screen_tri laid them out for 90 degrees
+        for v in t["vertices"]:
+            v["pos"][:2] *= w / 2.0 / O.fov_const(1.0, w)
+    rgba = compare(sc)
+    assert (rgba[..., :3] > 50).all(-1).mean() > 0.9
