@@ -14,7 +14,7 @@ LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libgbr.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 SOURCES = ["gbr_kernels.cu", "gbr_api.cu", "gbr_batch.cu", "gbr_noalloc.cu", "gbr_server.cu", "gbr_post.cu"]
-HEADERS = ["gbr_math.h", "gbr_shade_math.h", "gbr_internal.h", "gbr_scene.h", "gbr_post.cuh"]
+HEADERS = ["gbr_math.h", "gbr_shade_math.h", "gbr_internal.h", "gbr_scene.h", "gbr_host_range.h", "gbr_post.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-ffp-contract=off", "-I", INCLUDE]

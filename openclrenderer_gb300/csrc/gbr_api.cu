@@ -1,6 +1,7 @@
 // gbr_api.cu — C ABI of the pipeline: scene ownership, texture atlas build,
 // workspace management and the pass drivers (render_tris /
 // generate_realtime_shadowing of the reference engine).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -15,6 +16,7 @@
 #include <vector>
 
 #include "../../include/gbr.h"
+#include "gbr_host_range.h"
 #include "gbr_internal.h"
 #include "gbr_scene.h"
 
@@ -46,11 +48,25 @@ uint8_t* mapped_host_alias(void* p) {
   return nullptr;
 }
 
-// The device address of n words of mapped host memory, null unless both ends are.
-static uint32_t* mapped_host_words(uint32_t* p, size_t n) {
-  uint8_t* a = mapped_host_alias(p);
-  uint8_t* b = a ? mapped_host_alias(p + n - 1) : nullptr;
-  return a && b == a + (n - 1) * 4 ? reinterpret_cast<uint32_t*>(a) : nullptr;
+// The mapped host allocation that holds q, as the driver has it.
+static bool host_span(uint8_t* q, HostSpan* span) {
+  using GetAttribute = CUresult(CUDAAPI*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const GetAttribute get = []() -> GetAttribute {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) == cudaSuccess &&
+        found == cudaDriverEntryPointSuccess)
+      return reinterpret_cast<GetAttribute>(fn);
+    cudaGetLastError();
+    return nullptr;
+  }();
+  span->device = reinterpret_cast<uintptr_t>(mapped_host_alias(q));
+  CUdeviceptr start = 0;
+  if (!span->device || !get || get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, span->device) != CUDA_SUCCESS ||
+      get(&span->size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, span->device) != CUDA_SUCCESS)
+    return false;
+  span->start = (uintptr_t)start;
+  return true;
 }
 
 gbr_status fail(gbr_status s, const char* fmt, ...) {
@@ -1056,7 +1072,7 @@ gbr_status gbr_render_view_host(gbr_scene* s, const gbr_camera* cam, const gbr_v
   // frame, end to end: 0.40 or 0.48 ms as the copies fell, 0.39 to 0.44 so; the
   // depths as well, beside the copy kernel3 reads: 0.43, the raster then waits
   // for the link)
-  uint32_t* id_dev = mapped_host_words(id, P);
+  uint32_t* id_dev = reinterpret_cast<uint32_t*>(mapped_range(id, P * 4, host_span));
   gbr_outputs o{hw.pix_depth.p, id_dev ? id_dev : hw.pix_id.p, rgba_dev ? rgba_dev : hw.pix_rgba.p, nullptr};
   if (!s->copy_stream) {
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));
