@@ -39,15 +39,6 @@ thread_local std::string g_err;
 
 namespace gbr {
 
-uint8_t* mapped_host_alias(void* p) {
-  if (!p || (reinterpret_cast<uintptr_t>(p) & 3) != 0) return nullptr;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
-    return static_cast<uint8_t*>(at.devicePointer);
-  cudaGetLastError();
-  return nullptr;
-}
-
 // The mapped host allocation that holds q, as the driver has it.
 static bool host_span(uint8_t* q, HostSpan* span) {
   using GetAttribute = CUresult(CUDAAPI*)(void*, CUpointer_attribute, CUdeviceptr);
@@ -60,14 +51,22 @@ static bool host_span(uint8_t* q, HostSpan* span) {
     cudaGetLastError();
     return nullptr;
   }();
-  span->device = reinterpret_cast<uintptr_t>(mapped_host_alias(q));
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, q) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (!get || at.type != cudaMemoryTypeHost || !at.devicePointer) return false;
   CUdeviceptr start = 0;
-  if (!span->device || !get || get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, span->device) != CUDA_SUCCESS ||
+  span->device = reinterpret_cast<uintptr_t>(at.devicePointer);
+  if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, span->device) != CUDA_SUCCESS ||
       get(&span->size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, span->device) != CUDA_SUCCESS)
     return false;
   span->start = (uintptr_t)start;
   return true;
 }
+
+uint8_t* mapped_host_alias(void* p, size_t bytes) { return mapped_range(p, bytes, host_span); }
 
 gbr_status fail(gbr_status s, const char* fmt, ...) {
   char buf[512];
@@ -1067,12 +1066,12 @@ gbr_status gbr_render_view_host(gbr_scene* s, const gbr_camera* cam, const gbr_v
   TRY(hw.pix_rgba.reserve(P * 4));
   // RGBA8 into pinned (page-locked, mapped) host memory is written by kernel3
   // itself through the buffer's device address: nothing to copy after shading
-  uint8_t* rgba_dev = mapped_host_alias(rgba);
+  uint8_t* rgba_dev = mapped_host_alias(rgba, P * 4);
   // and so are the ids by the raster, the only kernel that touches them (1080p
   // frame, end to end: 0.40 or 0.48 ms as the copies fell, 0.39 to 0.44 so; the
   // depths as well, beside the copy kernel3 reads: 0.43, the raster then waits
   // for the link)
-  uint32_t* id_dev = reinterpret_cast<uint32_t*>(mapped_range(id, P * 4, host_span));
+  uint32_t* id_dev = reinterpret_cast<uint32_t*>(mapped_host_alias(id, P * 4));
   gbr_outputs o{hw.pix_depth.p, id_dev ? id_dev : hw.pix_id.p, rgba_dev ? rgba_dev : hw.pix_rgba.p, nullptr};
   if (!s->copy_stream) {
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));

@@ -187,7 +187,7 @@ void worker_loop(gbr_server* s, Worker* w) {
       uint8_t* b = pl.p + offs[i];
       cams[i] = batch[i].r.cam;
       views[i] = batch[i].r.view;
-      direct[i] = gbr::mapped_host_alias(batch[i].r.rgba);
+      direct[i] = gbr::mapped_host_alias(batch[i].r.rgba, 4 * P);
       outs[i] = gbr_outputs{reinterpret_cast<uint32_t*>(b), reinterpret_cast<uint32_t*>(b + 4 * P),
                             direct[i] ? direct[i] : b + 8 * P, nullptr};
     }
