@@ -1,4 +1,4 @@
-"""Passes of one view against the oracle: rasters of many tiles."""
+"""Passes of one view against the oracle: scratch that overflows and the re-run, and rasters of many tiles."""
 import numpy as np
 import pytest
 
@@ -23,6 +23,31 @@ def oracle(sc):
 def check(got, ref):
     assert np.array_equal(got["depth"], ref["depth"]) and np.array_equal(got["id"], ref["id"])
     assert np.abs(got["rgba"].astype(int) - ref["rgba"].astype(int)).max() <= 1
+
+
+@pytest.mark.parametrize("host", [False, True])
+def test_overflow(host):
+    """More bin entries than the first scratch holds: the counters reach the host, and the pass is run again whole."""
+    rng = np.random.default_rng(7)
+    w, h, n = 640, 480, 300
+    x, y, z = rng.uniform(0, w - 250, n), rng.uniform(0, h - 250, n), rng.uniform(100, 3000, n)
+    sc = tri_scene([screen_tri([a, a + 240, a], [b, b, b + 240], d, w, h) for a, b, d in zip(x, y, z)], w, h,
+                   descs=TWO_SIDED)
+    ref = oracle(sc)
+    gs = GpuScene(sc)
+    gs.set_tuning(S.PASS_VIEW, fine_max_tiles=256)
+    for again in range(2):
+        if host:
+            pin = [torch.empty((h, w), dtype=torch.int32, pin_memory=True).numpy().view(np.uint32) for _ in range(2)]
+            rgba = torch.empty((h, w, 4), dtype=torch.uint8, pin_memory=True).numpy()
+            check(gs.render_host(sc.cameras[0], sc.views[0], depth=pin[0], ids=pin[1], rgba=rgba), ref)
+        else:
+            check(gs.render(sc.cameras[0], sc.views[0]).numpy(), ref)
+        st = gs.stats()
+        assert st["retries"] >= 1 and st["view_records"] == n and st["view_bin_entries"] > 4 * (n + 1024)
+        retries = st["retries"] if not again else retries
+    assert gs.stats()["retries"] == retries  # the second frame fits
+    gs.close()
 
 
 @pytest.mark.parametrize("n_big,n_small,gap", [(3, 3000, 50.0), (40, 300, 0.01), (70, 0, 5.0)])
