@@ -238,38 +238,6 @@ __device__ __forceinline__ bool rec_in_tri(const float4 q[3], float fx, float fy
   return s > -0.0001f && t > -0.0001f && (s + t) < q[0].w;
 }
 
-// The rows py of [y0, y1) of a record's bbox whose left-column pixel the
-// reference walk skips, as bits py - ty.  The same arithmetic as
-// walk_visits (walk_row_late's 1 / w computed once, (r + 1) * w % chunk
-// stepped row by row), from the first row that can be late at all
-// (walk_first_late_row): a bbox at least its own height below the top of the
-// surface, which is nearly every record, costs one comparison instead of a
-// division, two modulos and a loop over its rows.
-__device__ __forceinline__ uint32_t walk_skip_rows(uint32_t xr, uint32_t yr, int y0, int y1, int ty, int chunk) {
-  const int minx = xr & 0xFFFF, miny = yr & 0xFFFF;
-  const int first = max(y0 - miny, walk_first_late_row(miny));
-  const int last = y1 - miny;  // one past
-  if (first >= last) return 0u;
-  const int w = (int)(xr >> 16) - minx, h = (int)(yr >> 16) - miny;
-  const float iw = fdiv(1.0f, (float)w), fminy = (float)miny;
-  auto late = [&](int r) { return floorf(fma_((float)(r * w), iw, fminy)) != fminy + (float)r; };
-  const int wm = w % chunk;
-  int m = ((first + 1) * w) % chunk;  // (r + 1) * w % chunk
-  bool late_r = late(first);
-  uint32_t bits = 0;
-  for (int r = first; r < last; r++) {
-    const int r1 = r + 1;
-    const bool late_r1 = r1 < h ? late(r1) : false;
-    // walk_visits: not late, or the next row is late and a fragment starts at (r + 1) * w
-    const bool visits = !late_r || (r1 < h && m == 0 && late_r1);
-    if (!visits) bits |= 1u << (miny + r - ty);
-    late_r = late_r1;
-    m += wm;
-    if (m >= chunk) m -= chunk;
-  }
-  return bits;
-}
-
 // One candidate as a record (and shade record for views).
 __device__ __forceinline__ void write_rec(const Cand& c, uint32_t r, uint32_t surface, const Workspace& ws,
                                           bool view) {

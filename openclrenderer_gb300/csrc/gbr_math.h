@@ -498,6 +498,40 @@ GBR_HD bool walk_visits(int j, int r, int w, int h, float miny, int chunk) {
 // late.)
 GBR_HD int walk_first_late_row(int miny) { return miny + 1; }
 
+// The rows py of [y0, y1) of a record's bbox (xr = minx | maxx << 16, yr
+// likewise) whose left-column pixel the reference walk skips, as bits py - ty;
+// the rows are rows of the bbox, and at most 32.  The same arithmetic as
+// walk_visits (walk_row_late's 1 / w computed once, (r + 1) * w % chunk
+// stepped row by row), from the first row that can be late at all
+// (walk_first_late_row): a bbox at least its own height below the top of the
+// surface, which is nearly every record, costs one comparison instead of a
+// division, two modulos and a loop over its rows.
+GBR_HD uint32_t walk_skip_rows(uint32_t xr, uint32_t yr, int y0, int y1, int ty, int chunk) {
+  const int minx = xr & 0xFFFF, miny = yr & 0xFFFF;
+  const int from = walk_first_late_row(miny);
+  const int first = y0 - miny > from ? y0 - miny : from;
+  const int last = y1 - miny;  // one past
+  if (first >= last) return 0u;
+  const int w = (int)(xr >> 16) - minx, h = (int)(yr >> 16) - miny;
+  const float iw = fdiv(1.0f, (float)w), fminy = (float)miny;
+  auto late = [&](int r) { return floorf(fma_((float)(r * w), iw, fminy)) != fminy + (float)r; };
+  const int wm = w % chunk;
+  int m = ((first + 1) * w) % chunk;  // (r + 1) * w % chunk
+  bool late_r = late(first);
+  uint32_t bits = 0;
+  for (int r = first; r < last; r++) {
+    const int r1 = r + 1;
+    const bool late_r1 = r1 < h ? late(r1) : false;
+    // walk_visits: not late, or the next row is late and a fragment starts at (r + 1) * w
+    const bool visits = !late_r || (r1 < h && m == 0 && late_r1);
+    if (!visits) bits |= 1u << (miny + r - ty);
+    late_r = late_r1;
+    m += wm;
+    if (m >= chunk) m -= chunk;
+  }
+  return bits;
+}
+
 // Largest resolution for which walk_visits is proven exact.
 constexpr int kMaxWalkWidth = 3840;
 constexpr int kMaxWalkHeight = 2160;

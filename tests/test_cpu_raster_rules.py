@@ -16,3 +16,13 @@ def test_shortcuts(tmp_path):
                     os.path.join(ROOT, "tests", "cpp", "raster_rules_check.cpp")], check=True)
     r = subprocess.run([str(exe), "800", "600", "200000"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_walk_skip_rows(tmp_path):
+    """The rasterisers' bits of skipped rows are walk_visits' rows."""
+    exe = tmp_path / "wsc"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
+                    os.path.join(ROOT, "openclrenderer_gb300", "csrc"), "-o", str(exe),
+                    os.path.join(ROOT, "tests", "cpp", "walk_skip_check.cpp")], check=True)
+    r = subprocess.run([str(exe), "3", "3000"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
