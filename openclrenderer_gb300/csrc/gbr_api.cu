@@ -292,9 +292,8 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
   ws.ncoarse = sh.ncoarse;
   ws.bins = wm.bins.p;
   ws.bin_cap = (uint32_t)std::min<size_t>(wm.bins.cap, 0xFFFFFFF0u);
-  const bool table = pass_tile_table(view, sh);
-  ws.tiles = table ? wm.tiles.p : nullptr;
-  ws.list = !view && !table ? reinterpret_cast<uint32_t*>(wm.tiles.p) : nullptr;
+  ws.tiles = view && sh.nsurf > 1 ? wm.tiles.p : nullptr;
+  ws.list = view ? nullptr : reinterpret_cast<uint32_t*>(wm.tiles.p);
   // views: the object cull needs the world cache (and with it the radii)
   const bool cull = view && sd.world && s->objr.p && sd.ndescs && sh.nobjects == sd.ndescs && sh.nitems <= 65535;
   ws.vis = cull ? wm.vis.p : nullptr;
@@ -336,15 +335,16 @@ gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, c
     // each group's raster, then its event: kernel3 of the group runs on st
     // after it, beside the next groups' rasters
     for (uint32_t g = 0; g < sh.ngroups; g++) {
-      CU(launch_raster(ws, wm.surf.p, sh.nsurf, sh.group_tile[g + 1] - sh.group_tile[g], true, tu.raster_threads,
-                       geom, 0, sh.group_tile[g]));
+      CU(launch_raster(ws, wm.surf.p, sh.group_tile[g + 1] - sh.group_tile[g], tu.raster_threads, geom,
+                       sh.group_tile[g]));
       if (g + 1 == sh.ngroups) CU(mark(4, geom));
       CU(cudaEventRecord(side->group[g], geom));
     }
   } else {
-    if (!fused)
-      CU(launch_raster(ws, wm.surf.p, sh.nsurf, sh.nfine, view, tu.raster_threads, geom, sh.tiles_per_surface, 0,
-                       inline_prep ? &sd : nullptr));
+    if (!view)
+      CU(launch_raster_faces(ws, wm.surf.p, sh.nfine, tu.raster_threads, geom, sh.tiles_per_surface));
+    else if (!fused)
+      CU(launch_raster(ws, wm.surf.p, sh.nfine, tu.raster_threads, geom, 0, inline_prep ? &sd : nullptr));
     CU(mark(4, geom));
   }
   if (view && s->mark_raster && !fused && !piped) CU(cudaEventRecord(s->raster_done, geom));

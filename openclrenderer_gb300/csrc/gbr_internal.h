@@ -233,13 +233,13 @@ cudaError_t launch_prep(const SceneDev& sc, const Workspace& ws, cudaStream_t st
 // descriptors nums / page sizes of the atlas packing.
 cudaError_t launch_texture_levels(const uint32_t* nums, const uint32_t* sizes, uint32_t mipmap_start,
                                   float4* texlv, cudaStream_t st);
-// tiles_per_surface: the common tile count when every surface has the same
-// size (cube faces), else 0.
-// tile0: the first tile of the launch (ntiles tiles from there).
+// Views.  tile0: the first tile of the launch (ntiles tiles from there).
 // prep (a pass of one view): the launch also does launch_prep's work.
-cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t nsurf,
-                          uint32_t ntiles, bool with_id, int threads, cudaStream_t st,
-                          uint32_t tiles_per_surface = 0, uint32_t tile0 = 0, const SceneDev* prep = nullptr);
+cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t ntiles, int threads, cudaStream_t st,
+                          uint32_t tile0 = 0, const SceneDev* prep = nullptr);
+// Cube faces, of tiles_per_surface tiles each: the tiles of ws.list.
+cudaError_t launch_raster_faces(const Workspace& ws, const Surface* d_surf, uint32_t ntiles, int threads,
+                                cudaStream_t st, uint32_t tiles_per_surface);
 // features: some view has kernel3's optional switches on (gbr_view.flags).
 // Reads the pass's counters: nothing is shaded after an overflow.
 // one_view / one_surf: the view of a one-view pass in host memory, passed with

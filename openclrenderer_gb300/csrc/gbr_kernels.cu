@@ -1120,14 +1120,14 @@ struct RasterSmem {
 };
 
 // NT threads per tile: a CTA of 64, 128, 256 or 512, or (PART) one of a CTA's
-// two halves of 64; ID: resolve the canonical id too
-// (views) or only the depth (cube faces); CC: see chunk below.  surface: the
-// tile's surface when the caller knows it, else -1 (ws.tiles, or the pass's
-// only surface).  Every thread of the block calls it; the caller synchronises
-// before reusing the shared memory.
+// two halves of 64; ID: resolve the canonical id too (views) or only the depth
+// (cube faces, tiles with records); CC: see chunk below.  surface: the tile's
+// surface when the caller knows it, else -1 (ws.tiles, or the pass's only
+// surface).  Every thread of the block calls it; the caller synchronises before
+// reusing the shared memory.
 template <int NT, bool ID, bool CC = false, bool PART = false>
-__device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* __restrict__ surfs, uint32_t nsurf,
-                                            uint32_t tile, int surface, RasterSmem<NT, ID>& sm) {
+__device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* __restrict__ surfs, uint32_t tile,
+                                            int surface, RasterSmem<NT, ID>& sm) {
   static_assert(!(ID && PART), "the id pass votes across the block");
   constexpr bool with_id = ID;
   constexpr int NW = NT / 32;
@@ -1153,7 +1153,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
       s = surface >= 0 ? (uint32_t)surface : tt.x;
       ct = tt.y;
       S = surfs[s];
-    } else {  // the surface is known (grid row, or the pass's only one)
+    } else {  // the surface is known (a cube face, or the pass's only one)
       s = surface >= 0 ? (uint32_t)surface : 0u;
       S = surfs[s];
       const uint32_t lt = tile - S.tile_base;
@@ -1212,8 +1212,7 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   if (with_id && ws.tile_empty && tid == 0) ws.tile_empty[tile] = 0;
   if (!with_id) {
     // depth-only passes: the surface was cleared and holds the small
-    // triangles the setup rasterised; a tile without records keeps it as is
-    if (lists[1] + lists[3] == 0) return;
+    // triangles the setup rasterised (a tile without records is not listed)
     for (int p = tid; p < kTilePixels; p += NT) {
       const int px = tx0 + (p & (kTile - 1)), py = ty0 + p / kTile;
       sdepth[swz32(p)] = (px < S.width && py < S.height) ? S.depth[(size_t)py * S.width + px] : kDepthClear;
@@ -1474,13 +1473,13 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
 
 // prep_blocks (one view that shades): the first blocks of the grid compute the
 // shade constants instead, beside the tiles, which do not read them.
-template <int NT, bool ID, bool CC = false>
-__global__ void __launch_bounds__(NT, ID ? raster_ctas<NT>() : 1280 / NT)
-    k_raster(Workspace ws, const Surface* __restrict__ surfs, uint32_t nsurf, uint32_t tile0, uint32_t prep_blocks,
+template <int NT, bool CC>
+__global__ void __launch_bounds__(NT, raster_ctas<NT>())
+    k_raster(Workspace ws, const Surface* __restrict__ surfs, uint32_t tile0, uint32_t prep_blocks,
              const __grid_constant__ SceneDev sc) {
-  __shared__ RasterSmem<NT, ID> sm;
+  __shared__ RasterSmem<NT, true> sm;
   if (ws.ctr->overflow) return;
-  if (ID && !CC && blockIdx.x < prep_blocks) {
+  if (!CC && blockIdx.x < prep_blocks) {
     // (as many warps as the tile's shared memory has buffers for)
     constexpr uint32_t kWarps = NT / 32 < sizeof(sm) / (16 * kPrepQuads) ? NT / 32 : sizeof(sm) / (16 * kPrepQuads);
     const uint32_t nrec = min(ws.ctr->nrec, ws.rec_cap), warp = threadIdx.x / 32;
@@ -1489,9 +1488,7 @@ __global__ void __launch_bounds__(NT, ID ? raster_ctas<NT>() : 1280 / NT)
         prep_records(sc, ws.srec + r, min(32u, nrec - r), reinterpret_cast<float4*>(&sm) + warp * kPrepQuads);
     return;
   }
-  // surfaces of one size (cube faces) come as grid rows: surface = blockIdx.y
-  const uint32_t tile = gridDim.y > 1 ? surfs[blockIdx.y].tile_base + blockIdx.x : tile0 + blockIdx.x - prep_blocks;
-  raster_tile<NT, ID, CC>(ws, surfs, nsurf, tile, gridDim.y > 1 ? (int)blockIdx.y : -1, sm);
+  raster_tile<NT, true, CC>(ws, surfs, tile0 + blockIdx.x - prep_blocks, -1, sm);
 }
 
 // The tiles of ws.list (surfaces of per_surface tiles each) of a depth-only
@@ -1505,7 +1502,7 @@ constexpr uint32_t kPartWaves = 6;
 constexpr int kPart = 64;
 template <int NT>
 __global__ void __launch_bounds__(NT, 1280 / NT) k_raster_list(Workspace ws, const Surface* __restrict__ surfs,
-                                                               uint32_t nsurf, uint32_t per_surface) {
+                                                               uint32_t per_surface) {
   constexpr uint32_t kParts = NT == 128 ? NT / kPart : 1;
   __shared__ union {
     RasterSmem<NT, false> one;
@@ -1517,25 +1514,19 @@ __global__ void __launch_bounds__(NT, 1280 / NT) k_raster_list(Workspace ws, con
     const uint32_t part = threadIdx.x / kPart % kParts;
     for (uint32_t i = kParts * blockIdx.x + part; i < n; i += kParts * gridDim.x) {
       const uint32_t tile = ws.list[i];
-      raster_tile<kPart, false, false, true>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm.part[part]);
+      raster_tile<kPart, false, false, true>(ws, surfs, tile, (int)(tile / per_surface), sm.part[part]);
       tile_barrier<kPart, true>();
     }
     return;
   }
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint32_t tile = ws.list[i];
-    raster_tile<NT, false>(ws, surfs, nsurf, tile, (int)(tile / per_surface), sm.one);
+    raster_tile<NT, false>(ws, surfs, tile, (int)(tile / per_surface), sm.one);
     __syncthreads();  // the next tile reuses the shared memory
   }
 }
 
 // ---- kernel3 ------------------------------------------------------------------
-struct ShadeCtx {
-  SceneDev sc;
-  const ViewParams* V;
-  const Surface* S;
-};
-
 // Byte -> float: one conversion that selects its byte (kernel3 0.6 % fewer
 // instructions than 2^23 + b, minus 2^23; the conversion pipe is a third busy).
 __device__ __forceinline__ float u8f(uint32_t b) { return (float)(uint8_t)b; }
@@ -2435,7 +2426,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_raster_shade(Workspace ws, co
     const uint32_t v = info & 0x7FFFFFFFu;
     const uint32_t tile = surfs[v].tile_base + (item - __ldg(sched + seg));
     if (!(info >> 31)) {
-      raster_tile<NT, true>(ws, surfs, nsurf, tile, (int)v, sm.r);
+      raster_tile<NT, true>(ws, surfs, tile, (int)v, sm.r);
       __threadfence();  // this thread's depth / id / record-map writes, before the count
       __syncthreads();
       if (threadIdx.x == 0) atomicAdd(&queue[2 + v], 1u);
@@ -2688,35 +2679,28 @@ cudaError_t launch_fill(const Workspace& ws, const Surface* d_surf, cudaStream_t
   return cudaGetLastError();
 }
 
-cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t nsurf, uint32_t ntiles,
-                          bool with_id, int threads, cudaStream_t st, uint32_t tiles_per_surface, uint32_t tile0,
-                          const SceneDev* prep) {
+cudaError_t launch_raster_faces(const Workspace& ws, const Surface* d_surf, uint32_t ntiles, int threads,
+                                cudaStream_t st, uint32_t tiles_per_surface) {
   if (!ntiles) return cudaSuccess;
-  if (prep && (!ws.srec || !with_id || ws.tiles)) return cudaErrorInvalidValue;
-  if (!with_id && ws.list && tiles_per_surface) {
-    const uint32_t blocks = std::min<uint32_t>(ntiles, (uint32_t)num_sms() * (1280 / threads));
-    switch (threads) {
-      case 128: k_raster_list<128><<<blocks, 128, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
-      case 512: k_raster_list<512><<<blocks, 512, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
-      default: k_raster_list<256><<<blocks, 256, 0, st>>>(ws, d_surf, nsurf, tiles_per_surface); break;
-    }
-    return cudaGetLastError();
+  if (!ws.list || !tiles_per_surface) return cudaErrorInvalidValue;
+  const uint32_t blocks = std::min<uint32_t>(ntiles, (uint32_t)num_sms() * (1280 / threads));
+  switch (threads) {
+    case 128: k_raster_list<128><<<blocks, 128, 0, st>>>(ws, d_surf, tiles_per_surface); break;
+    case 512: k_raster_list<512><<<blocks, 512, 0, st>>>(ws, d_surf, tiles_per_surface); break;
+    default: k_raster_list<256><<<blocks, 256, 0, st>>>(ws, d_surf, tiles_per_surface); break;
   }
-  if (with_id && threads == 128 && ntiles >= kManyWaves * num_sms() * raster_ctas<64>()) threads = 64;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t ntiles, int threads, cudaStream_t st,
+                          uint32_t tile0, const SceneDev* prep) {
+  if (!ntiles) return cudaSuccess;
+  if (prep && (!ws.srec || ws.tiles)) return cudaErrorInvalidValue;
+  if (threads == 128 && ntiles >= kManyWaves * num_sms() * raster_ctas<64>()) threads = 64;
   const uint32_t pb = prep ? std::min<uint32_t>((prep->ntris + threads - 1) / threads, (uint32_t)num_sms() * 4) : 0;
   const SceneDev sc = prep ? *prep : SceneDev{};
-  // surfaces of equal size: one grid row per surface, no search for the owner
-  const dim3 grid = (tile0 == 0 && tiles_per_surface && nsurf > 1 && nsurf <= 65535 &&
-                     tiles_per_surface * nsurf == ntiles) ? dim3(tiles_per_surface, nsurf) : dim3(ntiles + pb);
-#define GBR_RASTER(NT, ...) k_raster<NT, __VA_ARGS__><<<grid, NT, 0, st>>>(ws, d_surf, nsurf, tile0, pb, sc)
-  if (with_id && ws.tiles) {
-    switch (threads) {
-      case 64: GBR_RASTER(64, true, true); break;
-      case 128: GBR_RASTER(128, true, true); break;
-      case 512: GBR_RASTER(512, true, true); break;
-      default: GBR_RASTER(256, true, true); break;
-    }
-  } else if (with_id) {
+#define GBR_RASTER(NT, CC) k_raster<NT, CC><<<ntiles + pb, NT, 0, st>>>(ws, d_surf, tile0, pb, sc)
+  if (ws.tiles) {
     switch (threads) {
       case 64: GBR_RASTER(64, true); break;
       case 128: GBR_RASTER(128, true); break;
@@ -2725,6 +2709,7 @@ cudaError_t launch_raster(const Workspace& ws, const Surface* d_surf, uint32_t n
     }
   } else {
     switch (threads) {
+      case 64: GBR_RASTER(64, false); break;
       case 128: GBR_RASTER(128, false); break;
       case 512: GBR_RASTER(512, false); break;
       default: GBR_RASTER(256, false); break;

@@ -257,8 +257,7 @@ extern "C" gbr_status gbr_render_view_noalloc(const gbr_device_scene* sc, const 
   NA_CU(launch_setup_views(d, d_view, 1, d_surf, ws, s), "setup launch failed");
   NA_CU(launch_offsets(ws, d_surf, 1, 0, s), "offsets launch failed");
   NA_CU(launch_fill(ws, d_surf, s), "fill launch failed");
-  NA_CU(launch_raster(ws, d_surf, 1, nfine, true, kRasterThreads, s, 0, 0, shade ? &d : nullptr),
-        "raster launch failed");
+  NA_CU(launch_raster(ws, d_surf, nfine, kRasterThreads, s, 0, shade ? &d : nullptr), "raster launch failed");
   if (shade) NA_CU(launch_shade(d, d_view, 1, d_surf, nfine, ws, s, view->flags != 0, 0, &V, &S), "shade launch failed");
   Counters c{};
   NA_CU(cudaMemcpyAsync(&c, ws.ctr, sizeof c, cudaMemcpyDeviceToHost, s), "counter read-back failed");

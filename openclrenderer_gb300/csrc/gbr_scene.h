@@ -123,7 +123,7 @@ struct PassShape {
   uint32_t nobjects = 0;  // views: descriptors of the scene (object cull bits)
   size_t npix = 0;
   bool shade = true;  // views: some view wants RGBA or normals (else depth / id only)
-  uint32_t tiles_per_surface = 0;  // every surface has this many fine tiles (cube faces), else 0
+  uint32_t tiles_per_surface = 0;  // cube faces: fine tiles of each, else 0
   bool features = false;            // views: some view has gbr_view.flags set
   uint32_t nseg = 0;                // views: segments of the fused raster -> shade pass (GBR_RS_FUSED)
   uint32_t ngroups = 0;             // views: pipelined groups (GBR_RS_PIPELINED), 0 or >= 2
@@ -286,13 +286,6 @@ gbr_status reserve_pass(WorkMem& w, const PassShape& sh, bool view);
 gbr_status launch_pass(gbr_scene* s, WorkMem& wm, const Tuning& tu, bool view, const PassShape& sh,
                        Counters* host_ctr, cudaEvent_t* ev, cudaStream_t st, cudaStream_t geom = nullptr,
                        cudaEvent_t join = nullptr, const SideStream* side = nullptr);
-// Does a pass need the per-tile table (Workspace::tiles)?  Passes of several
-// surfaces whose raster cannot take the surface from its grid row (views;
-// cube faces of more than 65535 surfaces).
-inline bool pass_tile_table(bool view, const PassShape& sh) {
-  return sh.nsurf > 1 && (view || !(sh.tiles_per_surface && sh.nsurf <= 65535 &&
-                                    (uint64_t)sh.tiles_per_surface * sh.nsurf == sh.nfine));
-}
 // Kernel launches of one pass (for the launch statistics): begin (clears and
 // object cull), setup, offsets, fill, raster, and when shading the shade
 // constants (in the raster's launch for one view) and kernel3.  The fused
