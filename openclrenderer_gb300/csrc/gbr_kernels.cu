@@ -992,10 +992,18 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // and 33.4: the last wave counts there.
 constexpr uint32_t kManyWaves = 4;
 // Entries of a warp's list: about 100 are used in a tile of 1.2 layers by each
-// of four warps, and twice that by each of two.  512-thread CTAs keep no lists
-// (their static shared memory stays under 48 KB) and re-test in the id pass.
+// of four warps, and twice that by each of two.  At least what compaction can
+// leave and one window of tests can add: one entry for each of the tile's
+// pixels (more only where layers lie within kernel2's window of one another)
+// and 64.  With room for 256 alone, tiles of dozens of layers over all their
+// pixels gave their lists up and tested everything again: 4,000 overlapping
+// triangles of 30 pixels along a row of tiles at 720p, raster 196 us, 128 with
+// 320 entries, 161 without lists; 1,000 of them 59, 42 and 54.  512-thread CTAs
+// keep no lists (their static shared memory stays under 48 KB) and re-test in
+// the id pass.
 template <int NT>
-__host__ __device__ constexpr int hit_cap() { return NT == 64 ? 352 : 256; }
+__host__ __device__ constexpr int hit_cap() { return NT == 64 ? 352 : 320; }
+static_assert(hit_cap<64>() >= kTilePixels + 64 && hit_cap<128>() >= kTilePixels + 64, "");
 template <int NT>
 __host__ __device__ constexpr int raster_hits() { return NT <= 256 ? hit_cap<NT>() * (NT / 32) : 0; }
 // View CTAs per SM, by registers and (64 threads) shared memory.
