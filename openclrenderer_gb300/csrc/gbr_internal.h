@@ -38,7 +38,8 @@ constexpr int kRasterThreads = 128;  // threads of one raster CTA (default tunin
 constexpr int kMaxLights = 256;              // lights a scene may hold (staged in shared memory)
 
 constexpr uint32_t kRecTight = 1u;   // the box is tight_box's: one column and row less than bbox4
-constexpr uint32_t kRecInside = 2u;  // on_surface: rows can be narrowed to spans
+constexpr uint32_t kRecInside = 2u;  // on_surface: rows can be narrowed to spans exactly
+constexpr uint32_t kRecNear = 4u;    // near_surface, not on it: with span_slack
 
 // Per visible clipped triangle on one surface: everything kernel1/kernel2
 // need per pixel, precomputed once (64 bytes).

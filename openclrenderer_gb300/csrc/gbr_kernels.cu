@@ -111,7 +111,7 @@ __device__ __forceinline__ void make_rec(const Cand& c, uint32_t surface, Raster
   R.xr = (uint32_t)c.mm[0] | ((uint32_t)c.mm[1] << 16);
   R.yr = (uint32_t)c.mm[2] | ((uint32_t)c.mm[3] << 16);
   R.surface = surface;
-  R.kind = (c.box == kBoxTight ? kRecTight : 0u) | (c.inside ? kRecInside : 0u);
+  R.kind = (c.box == kBoxTight ? kRecTight : 0u) | (c.inside ? kRecInside : near_surface(xpv, ypv) ? kRecNear : 0u);
 }
 
 __device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& R) {
@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // rows at a time: it maps rows to records with one ballot of the record starts
 // inside the window (every staged record has a row, so at most 32 start
 // there), narrows each lane's row to the span that the three edges leave
-// (row_span; for records with vertices off the surface the row stays whole),
+// (row_span, with more slack for records with vertices off the surface),
 // and lays the spans' horizontal pixel pairs end to end in turn.  Those are
 // tested 32 at a time, mapped to spans as rows are to records: a pair costs
 // one decode and record load for two exact tests, and small, large and thin
@@ -980,7 +980,10 @@ __global__ void __launch_bounds__(256) k_fill(Workspace ws, const Surface* __res
 // (the depth cull at staging).  Then tight boxes and fewer records: 69 us
 // (terrain).  Rows narrowed to spans instead of all pairs of the bbox: 64
 // sphere views 1.01 -> 0.97 ms, 4K 210 -> 191 us, cube faces with large walls
-// 141 -> 121 us, 1080p terrain 68 -> 67 us.
+// 141 -> 121 us, 1080p terrain 68 -> 67 us.  Records with vertices off the surface
+// as well (whole rows, on top of the pairs, were slower than the pairs alone):
+// cube faces of 3,762, 2,750 and 2,471 large triangles at one depth 1,468 ->
+// 450, 1,349 -> 734 and 1,037 -> 434 us (1,031, 1,123 and 892 by pairs).
 //
 // A view pass of many tiles (kManyWaves of them) takes CTAs of 64 threads for
 // the default 128: a warp's fixed work per tile is paid half as often, two
@@ -1106,7 +1109,7 @@ struct RasterSmem {
   float4 srec[3][NT];  // the staged records' first three float4, one array each (conflict-free stores)
   uint32_t sidx[NT];
   uint32_t soff[NT + 1];
-  uint32_t sgeo[NT];   // lx0 | ly0 << 4 | bw << 8 | kRecTight << 13 | kRecInside << 13
+  uint32_t sgeo[NT];   // lx0 | ly0 << 4 | bw << 8 | kind << 13
   float2 sinv[NT];     // reciprocal x slopes of t and of bound - s - t (that of s: srec[1].w)
   uint2 spans[NT / 32][kSpanRing];  // per warp: spans of rows that can be covered
   // bit ly: the walk skips the record's left-column pixel in tile row ly (0
@@ -1375,12 +1378,16 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             int xa = (int)(geo & 0xF), xb = xa + (int)((geo >> 8) & 0x1F) - 1;
             // the walk rule: only a row's first pixel can be the bbox's left column
             xa += (int)((sskip[row_rec] >> ly) & 1u);
-            if (geo & (kRecInside << 13)) {
+            if (geo & ((kRecInside | kRecNear) << 13)) {
               const float4 q1 = srec[1][row_rec], q2 = srec[2][row_rec];
               const float2 inv = sm.sinv[row_rec];
               const float ftx = (float)tx0, fy = (float)(ty0 + ly);
-              row_span((q1.x + q1.z * fy) + q1.y * ftx, (q2.x + q2.z * fy) + q2.y * ftx, srec[0][row_rec].w, q1.w,
-                       inv.x, inv.y, (geo & (kRecTight << 13)) != 0, &xa, &xb);
+              const float bound = srec[0][row_rec].w;
+              float slack = 0.5f, slack_u = (geo & (kRecTight << 13)) ? 0.5f : 4.0f;  // row_span's
+              if (geo & (kRecNear << 13))
+                slack = slack_u = span_slack(q1.x, q1.y, q1.z, q2.x, q2.y, q2.z, bound, ftx + (float)kTile, fy);
+              row_span_slack((q1.x + q1.z * fy) + q1.y * ftx, (q2.x + q2.z * fy) + q2.y * ftx, bound, q1.w, inv.x,
+                             inv.y, slack, slack_u, &xa, &xb);
             }
             if (xb >= xa) {
               pairs = (uint32_t)(xb - xa + 2) >> 1;

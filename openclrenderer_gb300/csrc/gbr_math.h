@@ -410,9 +410,10 @@ GBR_HD float span_slope(float a) {
 // (apart from bound's tolerance), exact or, for s + t of a large triangle, off
 // by less than 4: half a unit (4 units) to the safe side, and 0.01 pixel for
 // the reciprocals.
-GBR_HD void row_span(float s, float t, float bound, float is, float it, float iu, bool small, int* xa, int* xb) {
-  const float rs = (-0.5f - s) * is, rt = (-0.5f - t) * it;
-  const float ru = ((small ? -0.5f : -4.0f) - ((bound - s) - t)) * iu;
+GBR_HD void row_span_slack(float s, float t, float bound, float is, float it, float iu, float slack, float slack_u,
+                           int* xa, int* xb) {
+  const float rs = (-slack - s) * is, rt = (-slack - t) * it;
+  const float ru = (-slack_u - ((bound - s) - t)) * iu;
   const float inf = 3.4028235e38f;
   const float lo = fmax_(fmax_(is > 0.0f ? rs : -inf, it > 0.0f ? rt : -inf), iu > 0.0f ? ru : -inf);
   const float hi = fmin_(fmin_(is > 0.0f ? inf : rs, it > 0.0f ? inf : rt), iu > 0.0f ? inf : ru);
@@ -423,6 +424,24 @@ GBR_HD void row_span(float s, float t, float bound, float is, float it, float iu
 #endif
   *xa = a > *xa ? a : *xa;
   *xb = b < *xb ? b : *xb;
+}
+
+GBR_HD void row_span(float s, float t, float bound, float is, float it, float iu, bool small, int* xa, int* xb) {
+  row_span_slack(s, t, bound, is, it, iu, 0.5f, small ? 0.5f : 4.0f, xa, xb);
+}
+// The slack of row_span_slack for a record with vertices off the surface, whose
+// edge functions (s0, sa, sb and t0, ta, tb, bound; sign folded in) are rounded:
+// each evaluation of s and t is off by at most 3 * 2^-24 of the magnitudes that
+// enter it, at the pixel and at the row's start, and the sums with bound by as
+// much again: 13 * 2^-24 of all of them covers the worst, bound - s - t.  x and
+// y: no pixel of the row lies beyond them.
+GBR_HD float span_slack(float s0, float sa, float sb, float t0, float ta, float tb, float bound, float x, float y) {
+  const float m = fma_(fabsf(sa) + fabsf(ta), x, fma_(fabsf(sb) + fabsf(tb), y, (fabsf(s0) + fabsf(t0)) + fabsf(bound)));
+  return fma_(m, 8e-7f, 0.5f);
+}
+// Vertices near enough for that to be of use (and none NaN or infinite).
+GBR_HD bool near_surface(f3 x, f3 y) {
+  return ((fabsf(x.x) + fabsf(x.y)) + (fabsf(x.z) + fabsf(y.x))) + (fabsf(y.y) + fabsf(y.z)) <= 1048576.0f;
 }
 
 // Quantised depth of a covered pixel (cl2.cl:5113-5115).

@@ -26,3 +26,13 @@ def test_walk_skip_rows(tmp_path):
                     os.path.join(ROOT, "tests", "cpp", "walk_skip_check.cpp")], check=True)
     r = subprocess.run([str(exe), "3", "3000"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_span_slack(tmp_path):
+    """Spans of triangles with vertices off the surface leave no covered pixel out."""
+    exe = tmp_path / "ssc"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
+                    os.path.join(ROOT, "openclrenderer_gb300", "csrc"), "-o", str(exe),
+                    os.path.join(ROOT, "tests", "cpp", "span_slack_check.cpp")], check=True)
+    r = subprocess.run([str(exe), "5", "200000"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
