@@ -1007,8 +1007,9 @@ constexpr uint32_t kManyWaves = 4;
 template <int NT>
 __host__ __device__ constexpr int hit_cap() { return NT == 64 ? 352 : 320; }
 static_assert(hit_cap<64>() >= kTilePixels + 64 && hit_cap<128>() >= kTilePixels + 64, "");
-template <int NT>
-__host__ __device__ constexpr int raster_hits() { return NT <= 256 ? hit_cap<NT>() * (NT / 32) : 0; }
+// The fused pass keeps 256: with 320 its blocks leave kernel3 less of the L1 (16
+// sphere views 948 -> 1,000 us).
+constexpr int kFusedHits = 256;
 // View CTAs per SM, by registers and (64 threads) shared memory.
 template <int NT>
 __host__ __device__ constexpr int raster_ctas() { return NT == 64 ? 15 : 1024 / NT; }
@@ -1103,9 +1104,10 @@ __device__ __noinline__ uint32_t compact_hits(uint2* hits, uint32_t n, const uin
 // Spans a warp holds at once: fewer than 32 that wait, and those of 32 rows.
 constexpr uint32_t kSpanRing = 64;
 
-// Shared memory of one tile's raster (NT threads; ID: views).
-template <int NT, bool ID>
+// Shared memory of one tile's raster (NT threads; ID: views; lists of CAP).
+template <int NT, bool ID, int CAP = hit_cap<NT>()>
 struct RasterSmem {
+  static constexpr int kHits = ID && NT <= 256 ? CAP : 0;  // entries of a warp's list, 0: none
   float4 srec[3][NT];  // the staged records' first three float4, one array each (conflict-free stores)
   uint32_t sidx[NT];
   uint32_t soff[NT + 1];
@@ -1117,8 +1119,8 @@ struct RasterSmem {
   uint16_t sskip[NT];
   // the covered pixels of pass 0 kept for the id pass: depth, and pixel |
   // record << 8 (the staged slot in one-chunk tiles, else the pass's record);
-  // warp w's list at w * hit_cap
-  uint2 hits[ID && raster_hits<NT>() ? raster_hits<NT>() : 1];
+  // warp w's list at w * kHits
+  uint2 hits[kHits ? kHits * (NT / 32) : 1];
   uint32_t sdepth[kTilePixels];
   unsigned long long sid[kTilePixels];
   uint32_t swarp[NT / 32];
@@ -1136,9 +1138,10 @@ struct RasterSmem {
 // surface when the caller knows it, else -1 (ws.tiles, or the pass's only
 // surface).  Every thread of the block calls it; the caller synchronises before
 // reusing the shared memory.
-template <int NT, bool ID, bool CC = false, bool PART = false>
+template <int NT, bool ID, bool CC = false, bool PART = false, int CAP = hit_cap<NT>()>
 __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* __restrict__ surfs, uint32_t tile,
-                                            int surface, RasterSmem<NT, ID>& sm) {
+                                            int surface, RasterSmem<NT, ID, CAP>& sm) {
+  constexpr uint32_t kHits = RasterSmem<NT, ID, CAP>::kHits;
   static_assert(!(ID && PART), "the id pass votes across the block");
   constexpr bool with_id = ID;
   constexpr int NW = NT / 32;
@@ -1245,9 +1248,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
   const bool packed = with_id && resident && ws.pack_keys;
   uint32_t* sid32 = reinterpret_cast<uint32_t*>(sid);
   // the warp's list of covered pixels and its length
-  uint2* hits = sm.hits + warp * (with_id && raster_hits<NT>() ? hit_cap<NT>() : 0);
+  uint2* hits = sm.hits + warp * kHits;
   uint32_t nh = 0;
-  bool listing = with_id && raster_hits<NT>() > 0 && (resident || ws.rec_cap <= kHitRecords);
+  bool listing = kHits > 0 && (resident || ws.rec_cap <= kHitRecords);
   uint32_t wsamples = 0;  // covered tests of pass 0 seen by this warp
   bool cached = false;
   for (int pass = 0; pass < passes; pass++) {
@@ -1433,9 +1436,9 @@ __device__ __forceinline__ void raster_tile(const Workspace& ws, const Surface* 
             const uint32_t n0 = (uint32_t)__popc(b0), n1 = (uint32_t)__popc(b1);
             if (pass == 0) {
               wsamples += n0 + n1;
-              if (listing && nh + n0 + n1 > (uint32_t)hit_cap<NT>()) {  // warp-uniform
+              if (listing && nh + n0 + n1 > kHits) {  // warp-uniform
                 nh = compact_hits(hits, nh, sdepth);
-                listing = nh + n0 + n1 <= (uint32_t)hit_cap<NT>();
+                listing = nh + n0 + n1 <= kHits;
               }
             }
             auto resolve = [&](float px, int pp, uint32_t slot) {
@@ -2416,7 +2419,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_raster_shade(Workspace ws, co
                                                                 const uint32_t* __restrict__ sched, uint32_t nseg,
                                                                 uint32_t* __restrict__ queue) {
   union Smem {
-    RasterSmem<NT, true> r;
+    RasterSmem<NT, true, kFusedHits> r;
     ShadeSmem s;
   };
   __shared__ Smem sm;
@@ -2441,7 +2444,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_raster_shade(Workspace ws, co
     const uint32_t v = info & 0x7FFFFFFFu;
     const uint32_t tile = surfs[v].tile_base + (item - __ldg(sched + seg));
     if (!(info >> 31)) {
-      raster_tile<NT, true>(ws, surfs, tile, (int)v, sm.r);
+      raster_tile<NT, true, false, false, kFusedHits>(ws, surfs, tile, (int)v, sm.r);
       __threadfence();  // this thread's depth / id / record-map writes, before the count
       __syncthreads();
       if (threadIdx.x == 0) atomicAdd(&queue[2 + v], 1u);
