@@ -241,9 +241,10 @@ gbr_status gbr_render_view(gbr_scene* scene, const gbr_camera* cam, const gbr_vi
 gbr_status gbr_render_view_blend(gbr_scene* scene, const gbr_camera* cam, const gbr_view* view,
                                  const gbr_outputs* out, const gbr_outputs* blend, void* stream);
 
-/* gbr_render_view with HOST output buffers, filled before returning.  A
- * pinned, mapped, 4-byte aligned rgba buffer is written by kernel3 itself;
- * other buffers are copied back. */
+/* gbr_render_view with HOST output buffers, filled before returning.  Id and
+ * rgba buffers that are 4-byte aligned and pinned and mapped throughout are
+ * written by the raster and by kernel3 themselves while the call runs; other
+ * buffers, and the depths, are copied back. */
 gbr_status gbr_render_view_host(gbr_scene* scene, const gbr_camera* cam, const gbr_view* view,
                                 uint32_t* depth, uint32_t* id, uint8_t* rgba, void* stream);
 

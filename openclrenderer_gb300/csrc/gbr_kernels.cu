@@ -2293,18 +2293,6 @@ __device__ __forceinline__ void shade_tile(const SceneDev& sc, const ViewParams*
   }
 }
 
-// 1080p terrain: 2,690 instructions per pixel (3,350 before the
-// approximations as single instructions, the SSAO counts without compares,
-// packed texel blends, integer texel coordinates and the view in the constant
-// bank), 183 us (223); 64 sphere views 2.13 ms (2.62).  It is bound by instruction issue (77 %
-// active).  The lights' shared memory is sized by the scene: with room for
-// kMaxLights the L1 lost 3 points of its hit rate (1.4 % of the batch's time).
-// Tiles of 128 or 64 pixels per block were slower (203 / 212 us): their
-// blocks share less in the L1 and start more often.
-//
-// A pass whose setup or binning overflowed its scratch leaves the depth and
-// record map unwritten (the raster returns at once); shading returns too, and
-// the host re-runs the pass with grown scratch.
 // kernel3 over the tiles of a pass, one 256-thread CTA per 16x16 tile.
 // tile_empty (or null): tiles whose output the raster wrote, which return at
 // once; tiles (null for one view): each tile's surface (Workspace).  Each
@@ -2313,6 +2301,19 @@ __device__ __forceinline__ void shade_tile(const SceneDev& sc, const ViewParams*
 // ONE: a pass of one view whose parameters come with the launch (one_view,
 // one_surf: constant-bank operands instead of loads that hold registers);
 // otherwise they are read from views / surfs.
+//
+// A pass whose setup or binning overflowed its scratch leaves the depth and
+// record map unwritten (the raster returns at once); shading returns too, and
+// the host re-runs the pass with grown scratch.
+//
+// Bound by instruction issue (79 % active; 73 % in batches).  1080p terrain:
+// 2,690 instructions per pixel (3,350 before the approximations as single
+// instructions, the SSAO counts without compares, packed texel blends, integer
+// texel coordinates and the view in the constant bank), 182 us (223); 64 sphere
+// views 1.79 ms (2.24).  The lights' shared memory is sized by the scene: with
+// room for kMaxLights the L1 lost 3 points of its hit rate (1.4 % of the batch's
+// time).  Tiles of 128 or 64 pixels per block were slower (203 / 212 us): their
+// blocks share less in the L1 and start more often.
 template <bool FEAT, bool ONE>
 __global__ void __launch_bounds__(kTilePixels, 4) k_shade(SceneDev sc,
                                                const __grid_constant__ ViewParams one_view,
@@ -2744,8 +2745,9 @@ cudaError_t launch_shade(const SceneDev& sc, const ViewParams* d_views, uint32_t
   if (!sc.objq || !sc.texlv || !ws.srec || (nviews > 1 && !ws.tiles)) return cudaErrorInvalidValue;
   const bool one = nviews == 1 && one_view && one_surf;
   auto go = [&](auto kernel) {
-    kernel<<<ntiles, kTilePixels, sizeof(float4) * kLightQuads * sc.nlights, st>>>(sc, one ? *one_view : ViewParams{}, one ? *one_surf : Surface{}, d_views, d_surf,
-                                   ws.srec, ws.ctr, ws.rec_cap, tile0, ws.tile_empty, ws.tiles, host_ctr);
+    kernel<<<ntiles, kTilePixels, sizeof(float4) * kLightQuads * sc.nlights, st>>>(
+        sc, one ? *one_view : ViewParams{}, one ? *one_surf : Surface{}, d_views, d_surf, ws.srec, ws.ctr, ws.rec_cap,
+        tile0, ws.tile_empty, ws.tiles, host_ctr);
   };
   if (features)
     one ? go(k_shade<true, true>) : go(k_shade<true, false>);

@@ -301,13 +301,6 @@ cudaError_t launch_pseudo_aa(const uint32_t* depth, const uint32_t* ids, const u
 }
 
 // ---- do_motion_blur (cl2.cl:6714-6860) ---------------------------------------
-// The pixel's surface point, in its object's frame, is carried through the
-// object's pose of the previous frame (history slot 1 on even frame ids, 2 on
-// odd) and projected with this frame's and the previous frame's camera; the
-// blend of the two screen motions (camera_contribution), times strength and
-// capped at 50 px, is averaged over that many bilinear taps centred on the
-// pixel.  Objects with a pixel on screen are marked in seen[] for the history
-// update.
 // Bytes LO and HI of t over 255, as RN(x * hi + RN(x * lo)) with 1 / 255 = hi +
 // lo: equal to u8_over_255 for every byte (two packed operations, not three).
 template <int LO, int HI>
@@ -328,10 +321,10 @@ __device__ __forceinline__ void add_texel(uint32_t t, float w, bool first, f4& o
 
 // read_linear_rgba8 with two channels per packed instruction: the bytes as
 // 2^23 + b less 2^23, their quotients by 255, and the weighted texels, which
-// are then added in the same order.  (Added one channel at a
-// time: the assembler contracts a packed product and a packed sum into one
-// rounding, --fmad=false or not.)  (A shared table of the 256 quotients took 16 lookups a tap,
-// with bank conflicts, and bound the pass.)
+// are then added in the same order, one channel at a time: with a packed sum
+// behind the packed product the results were those of one rounding, whatever
+// --fmad says.  (A shared table of the 256 quotients took 16 lookups a tap, with
+// bank conflicts, and bound the pass.)
 __device__ __forceinline__ f4 read_linear_packed(const uint8_t* __restrict__ img, int W, int H, float cx, float cy) {
   const float u = cx - 0.5f, v = cy - 0.5f;
   const float fi = floorf(u), fj = floorf(v);
@@ -371,6 +364,13 @@ __device__ __forceinline__ f4 read_linear_inner(const uint8_t* __restrict__ img,
   return o;
 }
 
+// The pixel's surface point, in its object's frame, is carried through the
+// object's pose of the previous frame (history slot 1 on even frame ids, 2 on
+// odd) and projected with this frame's and the previous frame's camera; the
+// blend of the two screen motions (camera_contribution), times strength and
+// capped at 50 px, is averaged over that many bilinear taps centred on the
+// pixel.  Objects with a pixel on screen are marked in seen[] for the history
+// update.
 struct MotionCam {
   f3 cpos, cc, cs, opos, oc, os;
   float fov, strength, cam_w;
